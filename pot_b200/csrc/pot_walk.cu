@@ -1,12 +1,11 @@
 // Barnes-Hut walks fused with the Boris push, grain absorption and the
 // boundary test; edge potential (chi_b); grain update.
 //
-// Plain form (POT_FORM_PLAIN): one thread per target, FP64, leaf size 1, the
-// reference's stack discipline (children pushed in member order, popped
-// last-first, pot.c:1755-1772), opening test and force expressions
-// (pot.c:1719-1803) with unfused products so every accept/open decision is
-// the reference's.  The reference accumulates in x87 long double; here the
-// accumulation is FP64 with fused multiply-adds.
+// Plain form (POT_FORM_PLAIN): FP64, leaf size 1.  Every target makes its own
+// accept/open decisions with the reference's unfused opening test
+// (pot.c:1719-1772), so its terms are exactly the reference's; the terms
+// (pot.c:1737-1749, 1789-1798) are evaluated and summed in FP64 with fused
+// multiply-adds, where the reference accumulates in x87 long double.
 //
 // Fast form (POT_FORM_FAST): see pot_walk_fast.cu.
 #include "pot_push.cuh"
@@ -15,146 +14,298 @@ namespace pot {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
-// E (V/m) at (x, y, z) for the particle in Morton slot `self`:
-// field_particle_feels_at, pot.c:1696-1808 (monopole cells).
-// E[] holds the starting field on entry: zero, or a spheroidal grain's own
-// field (pot-spheroid.c:1815-1819).
-__device__ int field_plain(uint32_t self, double x, double y, double z, const TreeDev& T,
-                           const double4* __restrict__ src64, const Params& P, double E[3],
-                           uint32_t& n_inter)
+// One 32-byte load of data that the kernel does not write.
+__device__ __forceinline__ double4 ld_nc(const double4* p)
 {
-	int32_t stack[WALK_STACK];
-	int len = 1;
-	stack[0] = 0;
-	double ex = E[0], ey = E[1], ez = E[2];
-	while (len) {
-		const int32_t code = stack[--len];
-		if (code >= 0) {
-			const double4 c = T.cq[code];
-			const double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
-			const double dist2 = dsq3(dx, dy, dz);
-			if (T.w2[code] < dmul(P.oap2, dist2)) {
-				if (T.dip) {
-					if (T.aq[code] != 0) {
-						// DIPOLES, pot.c:1739-1745: the cell's dipole term too
-						const double dist = sqrt(dist2);
-						const double es = ddiv(QE, dmul(dmul(P.k4, dist2), dist));
-						const double4 pd = T.dip[code];
-						const double rp = ddiv(dadd(dadd(dmul(dx, pd.x), dmul(dy, pd.y)), dmul(dz, pd.z)), dist2);
-						ex = fma(es, dadd(dsub(dmul(c.w, dx), pd.x), dmul(dmul(3.0, dx), rp)), ex);
-						ey = fma(es, dadd(dsub(dmul(c.w, dy), pd.y), dmul(dmul(3.0, dy), rp)), ey);
-						ez = fma(es, dadd(dsub(dmul(c.w, dz), pd.z), dmul(dmul(3.0, dz), rp)), ez);
-						n_inter++;
-					}
-				} else if (c.w != 0.0) {
-					const double dist = sqrt(dist2);
-					const double es = dmul(ddiv(QE, dmul(dmul(P.k4, dist2), dist)), c.w);
-					ex = fma(es, dx, ex);
-					ey = fma(es, dy, ey);
-					ez = fma(es, dz, ez);
-					n_inter++;
-				}
-			} else {
-				if (len + 8 > WALK_STACK) {
-					E[0] = E[1] = E[2] = 0.0;
-					return POT_E_WALK;
-				}
-				const int32_t* ch = &T.child[8u * (uint32_t)code];
-#pragma unroll
-				for (int s = 0; s < 8; s++) {
-					const int32_t cc = ch[slot_digit(s)];
-					if (cc != CH_EMPTY) stack[len++] = cc;
-				}
-			}
-		} else {
-			const uint32_t e = leaf_payload(code);
-			uint32_t j0 = e, j1 = e + 1;
-			if (e >= P.n_tree) {  // overflow bucket (see OVF_CAP)
-				const uint2 r = T.ovf[e - P.n_tree];
-				j0 = r.x;
-				j1 = r.x + r.y;
-			}
-			for (uint32_t slot = j0; slot < j1; slot++) {
-				if (slot == self) continue;
-				const double4 p = src64[slot];
-				const double dx = dsub(x, p.x), dy = dsub(y, p.y), dz = dsub(z, p.z);
-				double dist2 = dsq3(dx, dy, dz);
-				if (dist2 == 0.0) {
-					E[0] = E[1] = E[2] = 0.0;
-					return POT_E_COINCIDENT;
-				}
-				dist2 = dadd(dist2, P.soft2);
-				const double dist = sqrt(dist2);
-				const double es = ddiv(dmul(QE, p.w), dmul(dmul(P.k4, dist2), dist));
-				ex = fma(es, dx, ex);
-				ey = fma(es, dy, ey);
-				ez = fma(es, dz, ez);
-				n_inter++;
-			}
-		}
-	}
-	E[0] = ex;
-	E[1] = ey;
-	E[2] = ez;
-	return POT_OK;
+	double4 r;
+	asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+	return r;
 }
 
-// phi_particle_feels (pot.c:1934-2018): potential at (x, y, z) for the
-// particle in slot `self`, which is excluded; cells unsoftened, pairs
-// softened, the reference's visit order and expressions.
-__device__ double phi_plain(uint32_t self, double x, double y, double z, const TreeDev& T,
-                            const double4* __restrict__ src64, const Params& P, int& rc)
+// A target's sum: the field, or the potential in x.
+struct PlainAcc {
+	double x, y, z;
+};
+
+// 1 / sqrt(x) to FP64 rounding, for normal positive x and without branches:
+// the hardware's approximation y0 keeps 20 fraction bits, so y0^2 is exact
+// and e = 1 - x y0^2 has one rounding of its own; then x^(-p/2) is
+// y0^p (1 - e)^(-p/2), the binomial series in e (|e| < 2^-17) to third order.
+struct Rsqrt {
+	double y0, y02, e;
+	__device__ __forceinline__ explicit Rsqrt(double x)
+	{
+		asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+		y02 = y0 * y0;
+		e = fma(-x, y02, 1.0);
+	}
+	// s x^(-1/2), s / x and s x^(-3/2)
+	__device__ __forceinline__ double p1(double s) const
+	{
+		const double w = s * y0;
+		return fma(w, e * fma(e, fma(e, 0.3125, 0.375), 0.5), w);
+	}
+	__device__ __forceinline__ double p2(double s) const
+	{
+		const double w = s * y02;
+		return fma(w, e * fma(e, 1.0 + e, 1.0), w);
+	}
+	__device__ __forceinline__ double p3(double s) const
+	{
+		const double w = s * (y02 * y0);
+		return fma(w, e * fma(e, fma(e, 2.1875, 1.875), 1.5), w);
+	}
+};
+
+// One term of the sum at offset (dx, dy, dz), squared distance d2 (of a
+// particle, softened; of a cell, not): kq is QE q / (4 pi eps0).  A term
+// whose bit is not set adds zero.
+template <bool PHI, bool DIP>
+__device__ __forceinline__ void plain_term(PlainAcc& E, bool on, bool dip, const double4& pd, double kq, double dx,
+                                           double dy, double dz, double d2)
 {
-	int32_t stack[WALK_STACK];
-	int len = 1;
-	stack[0] = 0;
-	double phi = 0.0;
-	while (len) {
-		const int32_t code = stack[--len];
-		if (code >= 0) {
-			const double4 c = T.cq[code];
-			const double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
-			const double dist2 = dsq3(dx, dy, dz);
-			if (T.w2[code] < dmul(P.oap2, dist2)) {
-				if (T.dip) {
-					if (T.aq[code] != 0) {  // DIPOLES, pot.c:1966-1974
-						const double dist = sqrt(dist2);
-						const double4 pd = T.dip[code];
-						const double rp = dadd(dadd(dmul(dx, pd.x), dmul(dy, pd.y)), dmul(dz, pd.z));
-						phi += ddiv(dmul(QE, dadd(ddiv(c.w, dist), ddiv(rp, dmul(dist, dist2)))), P.k4);
-					}
-				} else if (c.w != 0.0) {
-					phi += ddiv(dmul(QE, c.w), dmul(P.k4, sqrt(dist2)));
-				}
-			} else {
-				if (len + 8 > WALK_STACK) {
-					rc = POT_E_WALK;
-					return 0.0;
-				}
-				const int32_t* ch = &T.child[8u * (uint32_t)code];
+	const Rsqrt r(d2);
+	if (PHI) {
+		double v = r.p1(kq);  // pot.c:1960-1973
+		if (DIP && dip) v += r.p3(fma(dx, pd.x, fma(dy, pd.y, dz * pd.z)));
+		E.x += on ? v : 0.0;
+	} else {
+		double es = r.p3(kq);  // pot.c:1737-1749, 1789-1798
+		if (DIP && dip) {  // DIPOLES, pot.c:1739-1745: (q + 3 (p.r) / r^2) r / r^3 - p / r^3
+			es = r.p3(kq + 3.0 * r.p2(fma(dx, pd.x, fma(dy, pd.y, dz * pd.z))));
+			const double n3 = on ? r.p3(-1.0) : 0.0;
+			E.x = fma(n3, pd.x, E.x);
+			E.y = fma(n3, pd.y, E.y);
+			E.z = fma(n3, pd.z, E.z);
+		}
+		es = on ? es : 0.0;
+		E.x = fma(es, dx, E.x);
+		E.y = fma(es, dy, E.y);
+		E.z = fma(es, dz, E.z);
+	}
+}
+
+// The walk: a warp walks the tree once for G targets, keeping every target's
+// own decisions.  A stack entry is a node and the mask of the targets that
+// have opened all of its ancestors.  Each lane takes one node a round and
+// makes the reference's unfused test (pot.c:1719-1803) for each of the G
+// targets: a cell some of them accept goes to a list with their mask, and
+// its children are pushed with the mask of those that open it; a particle
+// goes to the list with its mask less the target that is that particle.
+// Whole 32-entry lists are then evaluated with the lanes split into G targets
+// by 32 / G entries, each lane skipping the entries its target's bit is not
+// set in.  So every target's terms are the reference's; only the order of
+// its FP64 sum differs.
+//
+// What bounds it: instruction issue (a walk of one thread per target, the
+// form before, ran 17 of 32 lanes on average through three divergent paths
+// and waited on its stack in local memory).  Sharing a node's load, stack
+// entry and list entry between G neighbours, and evaluating branch-free
+// lists, took a step's walk from 958 to 54 us on the 8,193-particle plasma,
+// from 2,570 to 291 us at 60,001 particles (theta 0.4) and from 9.18 to
+// 2.57 ms at 1,000,001.  The sums' error against a long double walk fell
+// with it (RMS 7.0e-16 to 3.9e-16 on the 8,193-particle plasma).
+//
+// Stack: a round that pops t nodes leaves at most 7 t more than it found, so
+// t is cut (down to 1, a depth-first descent, which needs at most 7 entries
+// for each of the 21 levels) when the stack nears its capacity: no tree can
+// overflow it.
+constexpr int PW_WARPS = 4;  // warps per block
+constexpr int PW_CAP = 640;
+constexpr int PW_RESERVE = 7 * (MAX_LEVELS + 1);
+constexpr uint32_t PW_PART = 1u << 31;  // list word: a particle (softened); the low bits the targets' mask
+template <int G, bool DIP> struct PwSmem {
+	int2 stack[PW_CAP];       // node code, targets' mask
+	double4 src[64];          // the list: position and charge
+	double4 dip[DIP ? 64 : 1];
+	uint32_t word[64];
+	double2 txy[G];           // the targets
+	double tz[G];
+	uint32_t self[G];
+};
+
+// The list's first 32 entries (unused ones have no bit set) against the lane's
+// target, G entries a lane.
+template <int G, bool PHI, bool DIP>
+__device__ __forceinline__ void plain_eval(PlainAcc& E, uint32_t t, uint32_t sub, double x, double y, double z,
+                                           const PwSmem<G, DIP>& sm, const Params& P, uint32_t& n_inter, int& rc)
+{
+#pragma unroll(G < 4 ? G : 4)
+	for (int k = 0; k < G; k++) {
+		const int i = k * (32 / G) + (int)sub;
+		const uint32_t w = sm.word[i];
+		const double4 c = sm.src[i];
+		const bool on = ((w >> t) & 1u) != 0u, part = (w & PW_PART) != 0u;
+		const double dx = x - c.x, dy = y - c.y, dz = z - c.z;
+		double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+		if (!PHI && on && part && d2 == 0.0) rc = POT_E_COINCIDENT;
+		if (part) d2 += P.soft2;
+		plain_term<PHI, DIP>(E, on, !part, sm.dip[DIP ? i : 0], c.w, dx, dy, dz, d2);
+		n_inter += on ? 1u : 0u;
+	}
+}
+
+// Evaluate the list's first 32 of n >= 32 entries; those beyond move to the
+// front.
+template <int G, bool PHI, bool DIP>
+__device__ __forceinline__ void plain_flush(PlainAcc& E, int& n, uint32_t t, uint32_t sub, double x, double y, double z,
+                                            PwSmem<G, DIP>& sm, const Params& P, uint32_t& n_inter, int& rc)
+{
+	const uint32_t lane = lane_id();
+	plain_eval<G, PHI, DIP>(E, t, sub, x, y, z, sm, P, n_inter, rc);
+	n -= 32;
+	__syncwarp();
+	if ((int)lane < n) {
+		sm.src[lane] = sm.src[32 + lane];
+		sm.word[lane] = sm.word[32 + lane];
+		if (DIP) sm.dip[DIP ? lane : 0] = sm.dip[DIP ? 32 + lane : 0];
+	}
+	__syncwarp();
+}
+
+// Sums of the warp's nt <= G targets: lane l holds target l % G's point and
+// slot (0xFFFFFFFF for none) and its share of the lists; the lanes l < G
+// return the targets' sums.  n_inter counts the lane's terms.
+template <int G, bool PHI, bool DIP>
+__device__ PlainAcc plain_walk(uint32_t nt, double x, double y, double z, uint32_t me, const TreeDev& T,
+                               const double4* __restrict__ src64, const Params& P, PwSmem<G, DIP>& sm,
+                               uint32_t& n_inter, int& rc)
+{
+	const uint32_t lane = lane_id(), t = lane % G, sub = lane / G;
+	const uint32_t lt = (1u << lane) - 1u;
+	PlainAcc E { 0.0, 0.0, 0.0 };
+	if (lane < G) {
+		sm.txy[lane] = make_double2(x, y);
+		sm.tz[lane] = z;
+		sm.self[lane] = me;
+	}
+	sm.src[lane] = make_double4(0.0, 0.0, 0.0, 0.0);  // unused entries are evaluated too
+	const double ke = QE / P.k4;
+	int len = 0, n = 0;
+	// the round's node: the root on lane 0
+	int32_t code = lane == 0 ? 0 : CH_EMPTY;
+	uint32_t mask = (1u << nt) - 1u;
+	double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+	double w2 = 0.0;
+	if (code == 0) {
+		c = ld_nc(&T.cq[0]);
+		w2 = __ldg(&T.w2[0]);
+	}
+	__syncwarp();
+	while (__any_sync(0xffffffffu, code != CH_EMPTY)) {
+		const bool cell = code >= 0;
+		const uint32_t e = leaf_payload(code);
+		const bool over = code < CH_EMPTY && e >= P.n_tree;  // overflow bucket (see OVF_CAP)
+		uint32_t acc = 0, opn = 0;
+		if (cell) {
 #pragma unroll
-				for (int s = 0; s < 8; s++) {
-					const int32_t cc = ch[slot_digit(s)];
-					if (cc != CH_EMPTY) stack[len++] = cc;
-				}
+			for (int k = 0; k < G; k++) {
+				const double2 q = sm.txy[k];
+				const double d2 = dsq3(dsub(q.x, c.x), dsub(q.y, c.y), dsub(sm.tz[k], c.z));
+				if (w2 < dmul(P.oap2, d2)) acc |= 1u << k;
 			}
-		} else {
-			const uint32_t e = leaf_payload(code);
-			uint32_t j0 = e, j1 = e + 1;
-			if (P.leaf_size > 1 || e >= P.n_tree) {
-				const uint2 r = P.leaf_size > 1 ? T.lrange[e] : T.ovf[e - P.n_tree];
-				j0 = r.x;
-				j1 = r.x + r.y;
-			}
-			for (uint32_t slot = j0; slot < j1; slot++) {
-				if (slot == self) continue;
-				const double4 p = src64[slot];
-				const double d2 = dsq3(dsub(x, p.x), dsub(y, p.y), dsub(z, p.z));
-				phi += ddiv(dmul(QE, p.w), dmul(P.k4, sqrt(dadd(d2, P.soft2))));
+			opn = mask & ~acc;
+			acc &= mask;
+			if (DIP ? T.aq[code] == 0 : c.w == 0.0) acc = 0;
+		} else if (code != CH_EMPTY && !over) {
+			acc = mask;
+#pragma unroll
+			for (int k = 0; k < G; k++)
+				if (sm.self[k] == e) acc &= ~(1u << k);
+		}
+		// the children of the opened nodes, appended with a warp scan
+		int4 c0 = make_int4(CH_EMPTY, CH_EMPTY, CH_EMPTY, CH_EMPTY), c1 = c0;
+		int nch = 0;
+		if (opn) {
+			const int4* cp = reinterpret_cast<const int4*>(&T.child[8u * (uint32_t)code]);
+			c0 = __ldg(cp);
+			c1 = __ldg(cp + 1);
+			nch = (c0.x != CH_EMPTY) + (c0.y != CH_EMPTY) + (c0.z != CH_EMPTY) + (c0.w != CH_EMPTY) +
+			      (c1.x != CH_EMPTY) + (c1.y != CH_EMPTY) + (c1.z != CH_EMPTY) + (c1.w != CH_EMPTY);
+		}
+		// the list
+		const uint32_t am = __ballot_sync(0xffffffffu, acc != 0u);
+		if (acc) {
+			const int i = n + __popc(am & lt);
+			sm.src[i] = make_double4(c.x, c.y, c.z, ke * c.w);
+			sm.word[i] = acc | (cell ? 0u : PW_PART);
+			if (DIP && cell) {
+				const double4 d = T.dip[code];
+				sm.dip[i] = make_double4(ke * d.x, ke * d.y, ke * d.z, 0.0);
 			}
 		}
+		n += __popc(am);
+		int incl = nch;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const int v = __shfl_up_sync(0xffffffffu, incl, o);
+			if ((int)lane >= o) incl += v;
+		}
+		int w = len + incl - nch;
+		len += __shfl_sync(0xffffffffu, incl, 31);
+		if (opn) {
+			const int32_t cc[8] = { c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w };
+#pragma unroll
+			for (int d = 0; d < 8; d++)
+				if (cc[d] != CH_EMPTY) sm.stack[w++] = make_int2(cc[d], (int)opn);
+		}
+		__syncwarp();
+		uint32_t om = __ballot_sync(0xffffffffu, over);
+		while (om) {  // every particle of an overflow bucket, a list at a time
+			const int b = __ffs(om) - 1;
+			om &= om - 1u;
+			const uint2 r = T.ovf[__shfl_sync(0xffffffffu, e, b) - P.n_tree];
+			const uint32_t bm = __shfl_sync(0xffffffffu, mask, b);
+			for (uint32_t j0 = r.x; j0 < r.x + r.y; j0 += 32) {
+				const uint32_t j = j0 + lane;
+				if (j < r.x + r.y) {
+					uint32_t m = bm;
+					for (int k = 0; k < G; k++)
+						if (sm.self[k] == j) m &= ~(1u << k);
+					const double4 p = src64[j];
+					sm.src[n + (int)lane] = make_double4(p.x, p.y, p.z, ke * p.w);
+					sm.word[n + (int)lane] = m | PW_PART;
+				}
+				n += (int)min(32u, r.x + r.y - j0);
+				__syncwarp();
+				if (n >= 32) plain_flush<G, PHI, DIP>(E, n, t, sub, x, y, z, sm, P, n_inter, rc);
+			}
+		}
+		// the next round's nodes, whose loads are in flight while the list is
+		// evaluated
+		int take = min(len, 32);
+		if (len + 7 * take > PW_CAP - PW_RESERVE) take = max(1, min(take, (PW_CAP - PW_RESERVE - len) / 7));
+		int2 next = make_int2(CH_EMPTY, 0);
+		if ((int)lane < take) next = sm.stack[len - 1 - (int)lane];
+		len -= take;
+		double4 cn = c;
+		if (next.x >= 0) {
+			cn = ld_nc(&T.cq[next.x]);
+			w2 = __ldg(&T.w2[next.x]);
+		} else if (next.x != CH_EMPTY && leaf_payload(next.x) < P.n_tree) {
+			cn = ld_nc(&src64[leaf_payload(next.x)]);
+		}
+		if (n >= 32) plain_flush<G, PHI, DIP>(E, n, t, sub, x, y, z, sm, P, n_inter, rc);
+		__syncwarp();
+		code = next.x;
+		mask = (uint32_t)next.y;
+		c = cn;
 	}
-	return phi;
+	if (n > 0) {
+		if ((int)lane >= n) sm.word[lane] = 0u;
+		__syncwarp();
+		plain_eval<G, PHI, DIP>(E, t, sub, x, y, z, sm, P, n_inter, rc);
+		__syncwarp();
+	}
+#pragma unroll
+	for (int o = G; o < 32; o <<= 1) {
+		E.x += __shfl_xor_sync(0xffffffffu, E.x, o);
+		if (!PHI) {
+			E.y += __shfl_xor_sync(0xffffffffu, E.y, o);
+			E.z += __shfl_xor_sync(0xffffffffu, E.z, o);
+		}
+	}
+	return E;
 }
 
 // Deterministic block sum of three doubles (fixed shuffle and warp order).
@@ -178,19 +329,29 @@ __device__ void block_sum3(double v[3], double* __restrict__ out)
 
 // compute_epe of move_particles (pot.c:2771-2804), plain form: every
 // particle's potential at its step-start position; per-block partial sums
-// of q e phi per species (slots assigned to blocks statically).
-__global__ void __launch_bounds__(128) k_epe_plain(const double4* __restrict__ pos, TreeDev T,
-                                                   const double4* __restrict__ src64, double* __restrict__ partial,
-                                                   Params P, RunRec* rec)
+// of q e phi per species (slots assigned to warps statically).
+template <int G, bool DIP>
+__global__ void __launch_bounds__(PW_WARPS * 32) k_epe_plain(const double4* __restrict__ pos, TreeDev T,
+                                                             const double4* __restrict__ src64,
+                                                             double* __restrict__ partial, Params P, RunRec* rec)
 {
+	__shared__ PwSmem<G, DIP> smem[PW_WARPS];
+	PwSmem<G, DIP>& sm = smem[threadIdx.x >> 5];
 	double acc[3] = { 0.0, 0.0, 0.0 };
-	if (rec->status == POT_OK) {
+	// warp-uniform: another warp may set the status meanwhile
+	if (__shfl_sync(0xffffffffu, lane_id() == 0 ? rec->status : 0, 0) == POT_OK) {
 		const uint32_t gs = rec->grain_slot;
-		for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < P.n; s += gridDim.x * blockDim.x) {
-			const double4 p = src64[s];
+		const uint32_t warps = gridDim.x * PW_WARPS;
+		for (uint32_t b = blockIdx.x * PW_WARPS + (threadIdx.x >> 5); b * G < P.n; b += warps) {
+			const uint32_t s = b * G + lane_id() % G, nt = min((uint32_t)G, P.n - b * G);
+			const bool has = s < P.n;
+			double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
+			if (has) p = src64[s];
 			int rc = POT_OK;
-			double phi = phi_plain(s, p.x, p.y, p.z, T, src64, P, rc);
-			if (rc != POT_OK) set_status(rec, rc);
+			uint32_t ni = 0;
+			const PlainAcc r = plain_walk<G, true, DIP>(nt, p.x, p.y, p.z, s, T, src64, P, sm, ni, rc);
+			if (!has || lane_id() >= G) continue;
+			double phi = r.x;
 			if (s == gs) {
 				rec->phi_grain = phi;
 				continue;
@@ -238,14 +399,19 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, unsigned l
 // those sources (leaf particles moved, cells as built) and finishes the step
 // (pot.c:2533-2639), then absorption and the boundary against the
 // start-of-step position in src64.
-template <int STG>
-__global__ void __launch_bounds__(128) k_push_plain(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T,
-                                                    const double4* __restrict__ src64,
-                                                    const uint32_t* __restrict__ due_list,
-                                                    uint32_t* __restrict__ rein_list, Params P, RunRec* rec,
-                                                    StageBufs sb)
+// Each warp takes G targets (neighbours in Morton order) from the run's work
+// counter, finds their fields (plain_walk) and pushes them.
+template <int STG, int G, bool DIP>
+__global__ void __launch_bounds__(PW_WARPS * 32) k_push_plain(double4* __restrict__ pos, double4* __restrict__ vel,
+                                                              TreeDev T, const double4* __restrict__ src64,
+                                                              const uint32_t* __restrict__ due_list,
+                                                              uint32_t* __restrict__ rein_list, Params P, RunRec* rec,
+                                                              StageBufs sb)
 {
-	if (rec->status != POT_OK) return;
+	__shared__ PwSmem<G, DIP> smem[PW_WARPS];
+	PwSmem<G, DIP>& sm = smem[threadIdx.x >> 5];
+	// warp-uniform: another warp may set the status meanwhile
+	if (__shfl_sync(0xffffffffu, lane_id() == 0 ? rec->status : 0, 0) != POT_OK) return;
 	const uint32_t n_due = rec->n_due;
 	const unsigned long long t = rec->t_steps;
 	const bool grain_due = rec->grain_due != 0;
@@ -260,25 +426,41 @@ __global__ void __launch_bounds__(128) k_push_plain(double4* __restrict__ pos, d
 	unsigned long long n_inter = 0, n_push = 0;
 	for (;;) {
 		uint32_t base = 0;
-		if (lane_id() == 0) base = atomicAdd(&rec->work_ctr, 32u);
+		if (lane_id() == 0) base = atomicAdd(&rec->work_ctr, (uint32_t)G);
 		base = __shfl_sync(0xffffffffu, base, 0);
 		if (base >= n_due) break;
-		const uint32_t i = base + lane_id();
-		if (i >= n_due) continue;
-		const uint32_t s = due_list[i];
+		const uint32_t i = base + lane_id() % G, nt = min((uint32_t)G, n_due - base);
+		const bool has = i < n_due;
+		uint32_t s = 0xFFFFFFFFu;
+		double3 h = make_double3(0.0, 0.0, 0.0);
+		if (has) {
+			s = due_list[i];
+			const double4 p = pos[s];
+			h = make_double3(p.x, p.y, p.z);
+			if (STG == 0) {
+				const double4 v = vel[s];
+				const double half = 0.5 * (P.dt * (double)P.tss[(int)p.w]);
+				h = make_double3(fma(half, v.x, p.x), fma(half, v.y, p.y), fma(half, v.z, p.z));
+			}
+		}
+		uint32_t ni = 0;
+		int rc = POT_OK;
+		const PlainAcc r = plain_walk<G, false, DIP>(nt, h.x, h.y, h.z, s, T, src, P, sm, ni, rc);
+		if (rc != POT_OK) set_status(rec, rc);
+		n_inter += ni;
+		if (!has || lane_id() >= G) continue;
 		const double4 p = pos[s];
 		double4 v = vel[s];
 		const int sp = (int)p.w;
 		const double dt = P.dt * (double)P.tss[sp];
-		const double half = 0.5 * dt;
-		const double3 h = STG == 0 ? make_double3(fma(half, v.x, p.x), fma(half, v.y, p.y), fma(half, v.z, p.z))
-		                           : make_double3(p.x, p.y, p.z);
-		double E[3] = { 0.0, 0.0, 0.0 };
-		if (P.shape && sp != SP_DUST) spheroid_field(P, qg, dsub(h.x, gx), dsub(h.y, gy), dsub(h.z, gz), E);
-		uint32_t ni = 0;
-		const int rc = field_plain(s, h.x, h.y, h.z, T, src, P, E, ni);
-		if (rc != POT_OK) set_status(rec, rc);
-		n_inter += ni;
+		double E[3] = { r.x, r.y, r.z };
+		if (P.shape && sp != SP_DUST) {
+			// a spheroidal grain's own field first (pot-spheroid.c:1815-1819)
+			spheroid_field(P, qg, dsub(h.x, gx), dsub(h.y, gy), dsub(h.z, gz), E);
+			E[0] += r.x;
+			E[1] += r.y;
+			E[2] += r.z;
+		}
 		const double charge = sp == SP_DUST ? qg : (sp == SP_ION ? 1.0 : -1.0);
 		const double qom = (QE * charge) / mass_of(sp, P);
 		if (STG == 1) {
@@ -598,23 +780,38 @@ __global__ void k_phi_query(TreeDev T, const double4* __restrict__ src64, const 
 	}
 }
 
-__global__ void k_field_query_plain(TreeDev T, const double4* __restrict__ src64, const double* __restrict__ xyz,
-                                    const uint32_t* __restrict__ self_slot, uint32_t nq, double* __restrict__ E,
-                                    Params P, RunRec* rec)
+template <int G, bool DIP>
+__global__ void __launch_bounds__(PW_WARPS * 32) k_field_query_plain(TreeDev T, const double4* __restrict__ src64,
+                                                                     const double* __restrict__ xyz,
+                                                                     const uint32_t* __restrict__ self_slot,
+                                                                     uint32_t nq, double* __restrict__ E, Params P,
+                                                                     RunRec* rec)
 {
-	const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-	if (q >= nq) return;
-	double e[3] = { 0.0, 0.0, 0.0 };
-	if (P.shape && self_slot[q] != rec->grain_slot) {
-		spheroid_field(P, (double)rec->grain_q, dsub(xyz[3 * q], rec->grain_pos[0]), dsub(xyz[3 * q + 1], rec->grain_pos[1]),
-		               dsub(xyz[3 * q + 2], rec->grain_pos[2]), e);
+	__shared__ PwSmem<G, DIP> smem[PW_WARPS];
+	PwSmem<G, DIP>& sm = smem[threadIdx.x >> 5];
+	const uint32_t base = (blockIdx.x * PW_WARPS + (threadIdx.x >> 5)) * G;
+	if (base >= nq) return;
+	const uint32_t q = base + lane_id() % G, nt = min((uint32_t)G, nq - base);
+	const bool has = q < nq;
+	double3 h = make_double3(0.0, 0.0, 0.0);
+	uint32_t self = 0xFFFFFFFFu;
+	if (has) {
+		h = make_double3(xyz[3 * (size_t)q], xyz[3 * (size_t)q + 1], xyz[3 * (size_t)q + 2]);
+		self = self_slot[q];
 	}
 	uint32_t ni = 0;
-	const int rc = field_plain(self_slot[q], xyz[3 * q], xyz[3 * q + 1], xyz[3 * q + 2], T, src64, P, e, ni);
+	int rc = POT_OK;
+	const PlainAcc r = plain_walk<G, false, DIP>(nt, h.x, h.y, h.z, self, T, src64, P, sm, ni, rc);
 	if (rc != POT_OK) set_status(rec, rc);
-	E[3 * q] = e[0];
-	E[3 * q + 1] = e[1];
-	E[3 * q + 2] = e[2];
+	if (!has || lane_id() >= G) return;
+	double e[3] = { 0.0, 0.0, 0.0 };
+	if (P.shape && self != rec->grain_slot) {
+		spheroid_field(P, (double)rec->grain_q, dsub(h.x, rec->grain_pos[0]), dsub(h.y, rec->grain_pos[1]),
+		               dsub(h.z, rec->grain_pos[2]), e);
+	}
+	E[3 * (size_t)q] = e[0] + r.x;
+	E[3 * (size_t)q + 1] = e[1] + r.y;
+	E[3 * (size_t)q + 2] = e[2] + r.z;
 }
 
 // ---------------------------------------------------------------------------
@@ -640,6 +837,38 @@ static int sm_count()
 	return n;
 }
 
+// Targets per warp of the plain walk for n targets.  More targets share each
+// node's load, test round and stack entry, fewer make more warps: with 4,096
+// targets (8,193 particles) the walk takes 55, 63, 88 and 138 us with 2, 4, 8
+// and 16 targets a warp, with 15,000 132, 115, 129 and 209, with 30,000 399,
+// 294, 288 and 380, with 500,000 4,990, 3,248, 2,647 and 2,570.
+static int plain_group(uint32_t n) { return n < 8192u ? 2 : (n < 32768u ? 4 : 8); }
+
+template <int STG, int G, bool DIP>
+static void push_plain(double4* pos, double4* vel, const TreeDev& T, const double4* src64, const uint32_t* due_list,
+                       uint32_t* rein_list, const Params& P, RunRec* rec, const StageBufs& sb, cudaStream_t s)
+{
+	static int per = 0;
+	if (!per) {
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_push_plain<STG, G, DIP>, PW_WARPS * 32, 0);
+		if (per <= 0) per = 1;
+	}
+	k_push_plain<STG, G, DIP><<<sm_count() * per, PW_WARPS * 32, 0, s>>>(pos, vel, T, src64, due_list, rein_list, P,
+	                                                                    rec, sb);
+}
+
+template <int STG>
+static void push_plain_stage(double4* pos, double4* vel, const TreeDev& T, const double4* src64,
+                             const uint32_t* due_list, uint32_t* rein_list, const Params& P, RunRec* rec,
+                             const StageBufs& sb, cudaStream_t s)
+{
+	const int G = plain_group(P.n / 2);  // at least the electrons are due
+	if (T.dip) push_plain<STG, 8, true>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+	else if (G == 4) push_plain<STG, 4, false>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+	else if (G == 2) push_plain<STG, 2, false>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+	else push_plain<STG, 8, false>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+}
+
 void launch_chi_b(const TreeDev& T, const double4* src64, const Params& P, RunRec* rec, int force,
                   cudaStream_t s, Timer& tm)
 {
@@ -657,14 +886,9 @@ void launch_push(double4* pos, double4* vel, const TreeDev& T, const double4* sr
 		return;
 	}
 	ScopedKernel k(tm, sb.stage == 0 ? "walk_push_plain" : (sb.stage == 1 ? "walk_half1_plain" : "walk_half2_plain"));
-	const int nb = sm_count() * 8;
-	if (sb.stage == 0) {
-		k_push_plain<0><<<nb, 128, 0, s>>>(pos, vel, T, src64, due_list, rein_list, P, rec, sb);
-	} else if (sb.stage == 1) {
-		k_push_plain<1><<<nb, 128, 0, s>>>(pos, vel, T, src64, due_list, rein_list, P, rec, sb);
-	} else {
-		k_push_plain<2><<<nb, 128, 0, s>>>(pos, vel, T, src64, due_list, rein_list, P, rec, sb);
-	}
+	if (sb.stage == 0) push_plain_stage<0>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+	else if (sb.stage == 1) push_plain_stage<1>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
+	else push_plain_stage<2>(pos, vel, T, src64, due_list, rein_list, P, rec, sb, s);
 }
 
 void launch_absorb_late(double4* pos, double4* vel, const double4* src64, const uint32_t* due_list,
@@ -691,7 +915,11 @@ void launch_epe(const double4* pos, const TreeDev& T, const double4* src64, cons
 		return;
 	}
 	ScopedKernel k(tm, "epe_plain", 2);
-	k_epe_plain<<<EPE_BLOCKS, 128, 0, s>>>(pos, T, src64, partial, P, rec);
+	const int G = plain_group(P.n), th = PW_WARPS * 32;
+	if (T.dip) k_epe_plain<8, true><<<EPE_BLOCKS, th, 0, s>>>(pos, T, src64, partial, P, rec);
+	else if (G == 2) k_epe_plain<2, false><<<EPE_BLOCKS, th, 0, s>>>(pos, T, src64, partial, P, rec);
+	else if (G == 4) k_epe_plain<4, false><<<EPE_BLOCKS, th, 0, s>>>(pos, T, src64, partial, P, rec);
+	else k_epe_plain<8, false><<<EPE_BLOCKS, th, 0, s>>>(pos, T, src64, partial, P, rec);
 	k_epe_final<<<1, 1024, 0, s>>>(partial, nullptr, EPE_BLOCKS, rec);
 }
 
@@ -704,7 +932,13 @@ void launch_field_query(const TreeDev& T, const double4* src64, const float4* sr
 		return;
 	}
 	ScopedKernel k(tm, "field_query");
-	k_field_query_plain<<<(nq + 127) / 128, 128, 0, s>>>(T, src64, xyz, self_slot, nq, E, P, rec);
+	const int G = T.dip ? 8 : plain_group(nq);
+	const uint32_t per = PW_WARPS * (uint32_t)G, nb = (nq + per - 1) / per;
+	const int th = PW_WARPS * 32;
+	if (T.dip) k_field_query_plain<8, true><<<nb, th, 0, s>>>(T, src64, xyz, self_slot, nq, E, P, rec);
+	else if (G == 2) k_field_query_plain<2, false><<<nb, th, 0, s>>>(T, src64, xyz, self_slot, nq, E, P, rec);
+	else if (G == 4) k_field_query_plain<4, false><<<nb, th, 0, s>>>(T, src64, xyz, self_slot, nq, E, P, rec);
+	else k_field_query_plain<8, false><<<nb, th, 0, s>>>(T, src64, xyz, self_slot, nq, E, P, rec);
 }
 
 void launch_phi_query(const TreeDev& T, const double4* src64, const double* xyz, uint32_t nq, double* phi,
