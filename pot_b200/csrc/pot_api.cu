@@ -485,16 +485,6 @@ static int fill_params(pot_gpu_ctx* c)
 	return POT_OK;
 }
 
-static void tree_ptrs_fast(pot_gpu_ctx* c, bool fast)
-{
-	if (!fast) {
-		c->T.f = nullptr;
-		c->T.r2 = nullptr;
-		c->T.lf = nullptr;
-		c->T.lr2 = nullptr;
-	}
-}
-
 static int sync_status(pot_gpu_ctx* c)
 {
 	cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -786,28 +776,16 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	}
 	AL(T.ovf, OVF_CAP);
 	if (fast) {
-		AL(T.f, cap);
-		AL(T.r2, cap);
+		AL(T.nrec, 8ull * cap + 1);
 		AL(T.mom_pre, 5 * mom_prefix_entries(n));
 		AL(T.mom_blk, 5 * mom_block_entries(n));
 		if (cfg->flags & POT_CFG_DIPOLES) {
 			AL(T.mom_pre_d, 5 * mom_prefix_entries(n));
 			AL(T.mom_blk_d, 5 * mom_block_entries(n));
-			AL(T.fd, cap);
-			if (L > 1) AL(T.lfd, 8ull * cap);
+			AL(T.drec, 8ull * cap + 1);
 		}
-		if (L > 1) {
-			AL(T.lf, 8ull * cap);
-			AL(T.lr2, 8ull * cap);
-			AL(T.lrange, 8ull * cap);
-		}
+		if (L > 1) AL(T.lrange, 8ull * cap);
 	}
-	if (!fast || L == 1) {
-		T.lf = nullptr;
-		T.lr2 = nullptr;
-		if (!T.lrange) T.lrange = nullptr;
-	}
-	tree_ptrs_fast(c, fast);
 #undef AL
 	if (dry) {
 		*bytes = c->bytes;

@@ -262,7 +262,7 @@ static void member_blocks(const MemberView& v, uint32_t out[PS_COUNT])
 	out[PS_FILL] = div_up(nt - L, 256);
 	out[PS_FINISH] = div_up(nt, 256);
 	out[PS_MOM] = div_up(nt, PACK_MOM_TILE);
-	out[PS_MOMPRE] = div_up(nt / 4 + 1, 256);
+	out[PS_MOMPRE] = mom_cell_blocks(nt, L);
 	out[PS_GROUPS] = std::min<uint32_t>(592u, std::max<uint32_t>(1u, div_up(nt, 2048)));
 	out[PS_ONE] = 1;
 	out[PS_SMALL] = std::max<uint32_t>(4u, std::min<uint32_t>(148u, n / 8192u));

@@ -430,7 +430,7 @@ __device__ __forceinline__ void finish_nodes_body(G grd, const uint64_t* __restr
 					code = CH_EMPTY;
 				} else {
 					code = (int32_t)kc;
-					T.parent[kc] = (int32_t)k;
+					T.parent[kc] = (int32_t)(8u * k + (uint32_t)c);
 					nint++;
 				}
 			}
@@ -506,7 +506,6 @@ __global__ void k_moments(TreeDev T, const double4* __restrict__ src64, Params P
 		uint32_t aq = 0;
 		double cx = 0.0, cy = 0.0, cz = 0.0;
 		double px = 0.0, py = 0.0, pz = 0.0;
-		const float w_child = 0.5f * (float)(sqrt(T.w2[k]) * P.inv_rad);
 		for (int s = 0; s < 8; s++) {
 			const int d = slot_digit(s);
 			const int32_t code = T.child[8u * k + (uint32_t)d];
@@ -551,11 +550,6 @@ __global__ void k_moments(TreeDev T, const double4* __restrict__ src64, Params P
 						add_moment(cq, caq, ccx, ccy, ccz, pq, paq, sp.x, sp.y, sp.z);
 					}
 				}
-				if (T.lf && L > 1) {
-					T.lf[e] = make_float4((float)((ccx - P.rad) * P.inv_rad), (float)((ccy - P.rad) * P.inv_rad),
-					                      (float)((ccz - P.rad) * P.inv_rad), (float)cq);
-					T.lr2[e] = w_child * w_child / P.oap2_f;
-				}
 			}
 			if (caq) {
 				if (dip) {
@@ -569,13 +563,8 @@ __global__ void k_moments(TreeDev T, const double4* __restrict__ src64, Params P
 		T.aq[k] = aq;
 		T.cq[k] = make_double4(cx, cy, cz, (double)q);
 		if (dip) T.dip[k] = make_double4(px, py, pz, 0.0);
-		if (T.f) {
-			T.f[k] = make_float4((float)((cx - P.rad) * P.inv_rad), (float)((cy - P.rad) * P.inv_rad),
-			                     (float)((cz - P.rad) * P.inv_rad), (float)q);
-			T.r2[k] = (float)(T.w2[k] * P.inv_rad * P.inv_rad / P.oap2);
-		}
 		if (k == 0) break;
-		const int32_t p = T.parent[k];
+		const int32_t p = T.parent[k] >> 3;
 		if (p < 0 || (uint32_t)p >= k) {  // parents precede children in pre-order
 			set_status(rec, POT_E_CAPACITY);
 			break;
@@ -586,99 +575,6 @@ __global__ void k_moments(TreeDev T, const double4* __restrict__ src64, Params P
 		__threadfence();
 		k = (uint32_t)p;
 	}
-	}
-}
-
-// Fast form: the same bottom-up pass with plain sums, sum |q| x / sum |q|
-// divided once per cell, and bucket leaves summed directly.
-__global__ void k_moments_fast(TreeDev T, const double4* __restrict__ src64, Params P, RunRec* rec)
-{
-	const uint32_t M = rec->n_nodes;
-	if (M > T.cap) return;
-	const uint32_t L = P.leaf_size;
-	for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < M; k0 += gridDim.x * blockDim.x) {
-		if (T.nint[k0] != 0) continue;
-		uint32_t k = k0;
-		for (;;) {
-			int q = 0;
-			uint32_t aq = 0;
-			double sx = 0.0, sy = 0.0, sz = 0.0;
-			const float w_child = 0.5f * (float)(sqrt(T.w2[k]) * P.inv_rad);
-			const int4* cp = reinterpret_cast<const int4*>(&T.child[8u * k]);
-			const int4 c0 = cp[0], c1 = cp[1];
-			const int32_t cc[8] = { c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w };
-#pragma unroll
-			for (int d = 0; d < 8; d++) {
-				const int32_t code = cc[d];
-				if (code == CH_EMPTY) continue;
-				if (code >= 0) {
-					const int cq = __ldcg(&T.q[code]);
-					const uint32_t caq = __ldcg(&T.aq[code]);
-					const double2* p2 = reinterpret_cast<const double2*>(&T.cq[code]);
-					const double2 a01 = __ldcg(p2), a23 = __ldcg(p2 + 1);
-					q += cq;
-					aq += caq;
-					sx = fma((double)caq, a01.x, sx);
-					sy = fma((double)caq, a01.y, sy);
-					sz = fma((double)caq, a23.x, sz);
-					continue;
-				}
-				const uint32_t e = leaf_payload(code);
-				uint32_t j0 = e, j1 = e + 1;
-				if (L > 1) {
-					const uint2 r = T.lrange[e];
-					j0 = r.x;
-					j1 = r.x + r.y;
-				} else if (e >= P.n_tree) {
-					const uint2 r = T.ovf[e - P.n_tree];
-					j0 = r.x;
-					j1 = r.x + r.y;
-				}
-				int lq = 0;
-				uint32_t laq = 0;
-				double lx = 0.0, ly = 0.0, lz = 0.0;
-				for (uint32_t j = j0; j < j1; j++) {
-					const double4 sp = src64[j];
-					const int pq = (int)sp.w;
-					const double pa = (double)abs(pq);
-					lq += pq;
-					laq += (uint32_t)abs(pq);
-					lx = fma(pa, sp.x, lx);
-					ly = fma(pa, sp.y, ly);
-					lz = fma(pa, sp.z, lz);
-				}
-				if (L > 1 && T.lf) {
-					const double inv = laq ? 1.0 / (double)laq : 0.0;
-					T.lf[e] = make_float4((float)((lx * inv - P.rad) * P.inv_rad), (float)((ly * inv - P.rad) * P.inv_rad),
-					                      (float)((lz * inv - P.rad) * P.inv_rad), (float)lq);
-					T.lr2[e] = w_child * w_child / P.oap2_f;
-				}
-				q += lq;
-				aq += laq;
-				sx += lx;
-				sy += ly;
-				sz += lz;
-			}
-			const double inv = aq ? 1.0 / (double)aq : 0.0;
-			const double cx = sx * inv, cy = sy * inv, cz = sz * inv;
-			T.q[k] = q;
-			T.aq[k] = aq;
-			T.cq[k] = make_double4(cx, cy, cz, (double)q);
-			T.f[k] = make_float4((float)((cx - P.rad) * P.inv_rad), (float)((cy - P.rad) * P.inv_rad),
-			                     (float)((cz - P.rad) * P.inv_rad), (float)q);
-			T.r2[k] = (float)(T.w2[k] * P.inv_rad * P.inv_rad / P.oap2);
-			if (k == 0) break;
-			const int32_t p = T.parent[k];
-			if (p < 0 || (uint32_t)p >= k) {
-				set_status(rec, POT_E_CAPACITY);
-				break;
-			}
-			__threadfence();
-			const uint32_t arrived = atomicAdd(&T.ctr[p], 1u) + 1u;
-			if (arrived != T.nint[p]) break;
-			__threadfence();
-			k = (uint32_t)p;
-		}
 	}
 }
 
@@ -873,47 +769,65 @@ __device__ __forceinline__ double3 dipole_of(const Mom5& pd, double q, double cx
 	return make_double3(pd.q - q * cx, pd.a - q * cy, pd.x - q * cz);
 }
 
+__device__ __forceinline__ void put_rec(NodeRec* rec, float x, float y, float z, float q, float r2, uint32_t base,
+                                        uint32_t info)
+{
+	uint4* o = reinterpret_cast<uint4*>(rec);
+	o[0] = make_uint4(__float_as_uint(x), __float_as_uint(y), __float_as_uint(z), __float_as_uint(q));
+	o[1] = make_uint4(__float_as_uint(r2), base, info, 0u);
+}
+
+// Eight lanes a cell: each writes its child's record if that is a leaf, the
+// first the cell's own moments and record.
 template <class G>
 __device__ __forceinline__ void moments_prefix_body(G grd, const TreeDev& T, const Mom5* __restrict__ pre,
                                                     const Mom5* __restrict__ pre_d, const Params& P, RunRec* rec)
 {
 	const uint32_t M = rec->n_nodes;
 	if (M > T.cap) return;
-	const uint32_t L = P.leaf_size;
-	for (uint32_t k = grd.id() * blockDim.x + threadIdx.x; k < M; k += grd.n() * blockDim.x) {
-		const Mom5 m = mom_range(pre, T.first[k], T.last[k] + 1);
+	const uint32_t L = P.leaf_size, d = threadIdx.x & 7u;
+	const uint32_t n = (8u * M + 31u) & ~31u;  // whole warps
+	for (uint32_t i = grd.id() * blockDim.x + threadIdx.x; i < n; i += grd.n() * blockDim.x) {
+		const uint32_t k = i >> 3;
+		const int32_t code = k < M ? T.child[i] : CH_EMPTY;
+		const uint32_t mask = (__ballot_sync(0xffffffffu, code != CH_EMPTY) >> (threadIdx.x & 24u)) & 0xFFu;
+		if (code < CH_EMPTY) {
+			const uint32_t e = leaf_payload(code);
+			if (L > 1) {
+				const float w_child = 0.5f * (float)(sqrt(T.w2[k]) * P.inv_rad);
+				const uint2 r = T.lrange[e];
+				const Mom5 lm = mom_range(pre, r.x, r.x + r.y);
+				const double li = lm.a > 0.0 ? 1.0 / lm.a : 0.0;
+				put_rec(&T.nrec[i], (float)(lm.x * li * P.inv_rad), (float)(lm.y * li * P.inv_rad),
+				        (float)(lm.z * li * P.inv_rad), (float)llrint(lm.q), w_child * w_child / P.oap2_f, r.x,
+				        NR_LEAF | r.y);
+				if (pre_d) {
+					const double3 dl = dipole_of(mom_range(pre_d, r.x, r.x + r.y), (double)llrint(lm.q), lm.x * li,
+					                             lm.y * li, lm.z * li);
+					T.drec[i] = make_float4((float)(dl.x * P.inv_rad), (float)(dl.y * P.inv_rad),
+					                        (float)(dl.z * P.inv_rad), 0.f);
+				}
+			} else {
+				const uint2 r = e < P.n_tree ? make_uint2(e, 1u) : T.ovf[e - P.n_tree];
+				put_rec(&T.nrec[i], 0.f, 0.f, 0.f, 0.f, 0.f, r.x, NR_LEAF | NR_UNTESTED | r.y);
+			}
+		}
+		if (d != 0 || k >= M) continue;
+		const uint32_t a = T.first[k], b = T.last[k] + 1;
+		const Mom5 m = mom_range(pre, a, b);
 		const double inv = m.a > 0.0 ? 1.0 / m.a : 0.0;
 		const double cx = m.x * inv, cy = m.y * inv, cz = m.z * inv;  // relative to the centre
 		const int q = (int)llrint(m.q);
 		T.q[k] = q;
 		T.aq[k] = (uint32_t)llrint(m.a);
 		T.cq[k] = make_double4(cx + P.rad, cy + P.rad, cz + P.rad, (double)q);
-		T.f[k] = make_float4((float)(cx * P.inv_rad), (float)(cy * P.inv_rad), (float)(cz * P.inv_rad), (float)q);
-		T.r2[k] = (float)(T.w2[k] * P.inv_rad * P.inv_rad / P.oap2);
+		const uint32_t o = k == 0 ? 8u * T.cap : (uint32_t)T.parent[k];
+		put_rec(&T.nrec[o], (float)(cx * P.inv_rad), (float)(cy * P.inv_rad), (float)(cz * P.inv_rad), (float)q,
+		        (float)(T.w2[k] * P.inv_rad * P.inv_rad / P.oap2), 8u * k, mask);
 		if (pre_d) {
-			const double3 d = dipole_of(mom_range(pre_d, T.first[k], T.last[k] + 1), (double)q, cx, cy, cz);
-			T.dip[k] = make_double4(d.x, d.y, d.z, 0.0);
-			T.fd[k] = make_float4((float)(d.x * P.inv_rad), (float)(d.y * P.inv_rad), (float)(d.z * P.inv_rad), 0.f);
-		}
-		if (L > 1) {
-			const float w_child = 0.5f * (float)(sqrt(T.w2[k]) * P.inv_rad);
-			for (int d = 0; d < 8; d++) {
-				const int32_t code = T.child[8u * k + (uint32_t)d];
-				if (code >= CH_EMPTY) continue;
-				const uint32_t e = leaf_payload(code);
-				const uint2 r = T.lrange[e];
-				const Mom5 lm = mom_range(pre, r.x, r.x + r.y);
-				const double li = lm.a > 0.0 ? 1.0 / lm.a : 0.0;
-				T.lf[e] = make_float4((float)(lm.x * li * P.inv_rad), (float)(lm.y * li * P.inv_rad),
-				                      (float)(lm.z * li * P.inv_rad), (float)llrint(lm.q));
-				T.lr2[e] = w_child * w_child / P.oap2_f;
-				if (pre_d) {
-					const double3 d = dipole_of(mom_range(pre_d, r.x, r.x + r.y), (double)llrint(lm.q), lm.x * li,
-					                            lm.y * li, lm.z * li);
-					T.lfd[e] = make_float4((float)(d.x * P.inv_rad), (float)(d.y * P.inv_rad),
-					                       (float)(d.z * P.inv_rad), 0.f);
-				}
-			}
+			const double3 dc = dipole_of(mom_range(pre_d, a, b), (double)q, cx, cy, cz);
+			T.dip[k] = make_double4(dc.x, dc.y, dc.z, 0.0);
+			T.drec[o] = make_float4((float)(dc.x * P.inv_rad), (float)(dc.y * P.inv_rad), (float)(dc.z * P.inv_rad), 0.f);
 		}
 	}
 }
@@ -923,6 +837,10 @@ __global__ void k_moments_prefix(TreeDev T, const Mom5* __restrict__ pre, const 
 {
 	moments_prefix_body(GridSelf {}, T, pre, pre_d, P, rec);
 }
+
+// Blocks of the cells' moments kernel: eight lanes a cell, of which there are
+// about n / 2 with leaf size 1 and n / (2 L) or fewer with larger leaves.
+uint32_t mom_cell_blocks(size_t n, uint32_t leaf) { return (uint32_t)((std::max(n / 4, 4 * n / leaf) + 256) / 256); }
 
 size_t mom_prefix_entries(size_t n) { return n + 1; }
 size_t mom_block_entries(size_t n) { return (n + MOM_TILE - 1) / MOM_TILE + 1; }
@@ -974,7 +892,7 @@ void launch_build(const uint64_t* keys, TreeDev& T, const double4* src64, const 
 		k_finish_nodes<<<blocks_for(n, 256), 256, 0, s>>>(keys, n, L, T.lvl8, T.base, T, P, rec);
 	}
 	{
-		const bool prefix = P.form == POT_FORM_FAST && T.mom_pre;
+		const bool prefix = P.form == POT_FORM_FAST;
 		const bool dip = prefix && T.mom_pre_d;
 		ScopedKernel k(tm, "tree_moments", prefix ? (dip ? 7 : 4) : 1);
 		if (prefix) {
@@ -992,9 +910,7 @@ void launch_build(const uint64_t* keys, TreeDev& T, const double4* src64, const 
 				k_mom_top<<<1, MOM_THREADS, 0, s>>>(bs_d, nb);
 				k_mom_down<1><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs_d, pre_d);
 			}
-			k_moments_prefix<<<blocks_for(n / 4 + 1, 256), 256, 0, s>>>(T, pre, pre_d, P, rec);
-		} else if (P.form == POT_FORM_FAST) {
-			k_moments_fast<<<blocks_for(n, 256), 256, 0, s>>>(T, src64, P, rec);
+			k_moments_prefix<<<mom_cell_blocks(n, L), 256, 0, s>>>(T, pre, pre_d, P, rec);
 		} else {
 			k_moments<<<blocks_for(n, 256), 256, 0, s>>>(T, src64, P, rec);
 		}

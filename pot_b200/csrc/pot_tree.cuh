@@ -5,6 +5,21 @@
 
 namespace pot {
 
+// A tree node as the FP32 walk reads it, in units of the domain radius from
+// the domain centre.  A cell: centre of charge and charge, critical radius
+// squared (accepted when d^2 > r2), the index of its first child's record and
+// the mask of its children by octal digit.  A leaf: the same moments, its
+// first slot and, with NR_LEAF, its particle count; a leaf of a leaf-size-1
+// tree has no moments (NR_UNTESTED: always opened).
+constexpr uint32_t NR_LEAF = 1u << 31, NR_UNTESTED = 1u << 30, NR_COUNT = NR_UNTESTED - 1u;
+struct __align__(32) NodeRec {
+	float x, y, z, q;
+	float r2;
+	uint32_t base;
+	uint32_t info;
+	uint32_t pad;
+};
+
 // Internal nodes in pre-order, structure of arrays; `cap` entries each
 // (the leaf table of bucket leaves has 8 * cap entries).
 struct TreeDev {
@@ -16,7 +31,7 @@ struct TreeDev {
 	uint32_t* last;    // last particle
 	uint8_t* level;    // depth (root 0)
 	int32_t* child;    // [8 * cap] child codes by octal digit
-	int32_t* parent;
+	int32_t* parent;   // 8 parent + octal digit, -1 for the root
 	uint8_t* nint;     // internal children
 	uint32_t* ctr;     // arrivals in the upward pass
 	int32_t* q;        // net charge (Tree.q)
@@ -24,22 +39,20 @@ struct TreeDev {
 	double4* cq;       // centre of |q| and q
 	double* w2;        // (x2 - x1)^2
 	double4* dip;      // DIPOLES: dipole moment about cq (FP64, both forms); null otherwise
-	// FP32 walk (fast form only; null otherwise)
-	float4* f;         // centre relative to the domain centre, q
-	float* r2;         // w2 / OAP^2: accepted when d^2 > r2
-	float4* lf;        // [8 * cap] bucket-leaf moments
-	float* lr2;        // [8 * cap] bucket-leaf critical radius^2
+	// FP32 walk (fast form only; null otherwise): one 32-byte record per child,
+	// record 8 k + d for child d of cell k (the root's is record 8 cap), so that
+	// a walk reads everything it needs of a node with one load
+	NodeRec* nrec;     // [8 * cap + 1]
 	uint2* lrange;     // [8 * cap] bucket-leaf (first slot, count)
 	uint2* ovf;        // [OVF_CAP] leaf-size-1 overflow buckets (first slot, count)
 	// fast form: exclusive prefix sums of (q, |q|, |q| x, |q| y, |q| z), 5 doubles each
 	double* mom_pre;   // [n + 1]
 	double* mom_blk;   // [blocks + 1]
 	// fast form with DIPOLES: prefix sums of (q x, q y, q z) in the same layout,
-	// and the cells' and bucket leaves' dipoles in FP32 units of q R
+	// and the nodes' dipoles in FP32 units of q R
 	double* mom_pre_d;
 	double* mom_blk_d;
-	float4* fd;        // [cap]
-	float4* lfd;       // [8 * cap]
+	float4* drec;      // [8 * cap + 1], indexed as nrec
 };
 
 // One member run of a packed batch as the batched kernels see it: the
@@ -86,7 +99,7 @@ struct MemberView {
 //   PS_FILL    blocks_for(n_tree - L, 256)
 //   PS_FINISH  blocks_for(n_tree, 256)
 //   PS_MOM     moment tiles over n_tree: prefix sums
-//   PS_MOMPRE  blocks_for(n_tree / 4 + 1, 256): cell moments from the sums
+//   PS_MOMPRE  mom_cell_blocks(n_tree, leaf size): cell moments from the sums
 //   PS_GROUPS  target groups
 //   PS_ONE     one block per member: digit offsets, scan tops, chi_b, grain
 //   PS_SMALL   4-148 blocks per member (one per 8,192 particles): late
@@ -127,6 +140,7 @@ void pack_grain_end(const PackDev& B, int k, cudaStream_t s);
 constexpr uint32_t PACK_MOM_TILE = 256 * 16;  // moment prefix-sum tile (tree.cu MOM_TILE)
 uint32_t pack_scan_blocks(uint32_t n);        // scan tiles over n items
 
+uint32_t mom_cell_blocks(size_t n, uint32_t leaf);
 size_t mom_prefix_entries(size_t n);
 size_t mom_block_entries(size_t n);
 void launch_keys(const double4* pos, uint64_t* keys, uint32_t* vals, const Params& P, RunRec* rec,

@@ -36,6 +36,7 @@ constexpr int FW_CELLS = 104;      // staged monopoles (flush at >= 64; at most 
 constexpr int FW_CELL_FLUSH = 64;
 constexpr int FW_LEAVES = 64;      // staged leaf ranges (flush at >= 32)
 constexpr int FW_LEAF_FLUSH = 32;
+constexpr uint32_t NONE = 0xFFFFFFFFu;
 static_assert(GROUP_MAX == 32 * FW_TPL_MAX, "one group per warp, at most FW_TPL_MAX targets per lane");
 // Blocks per SM the push kernels are compiled for.  With two targets per
 // lane the walk holds both targets' sums and operands: at four blocks (128
@@ -53,10 +54,10 @@ constexpr int fw_push_blocks(int tpl) { return tpl == 2 ? 4 : 5; }
 // holds each staged cell's dipole moment, packed in pairs like the positions.
 template <int TPL, bool DIP = false>
 struct FastSmem {
-	int32_t stack[FW_STACK];
+	uint32_t stack[FW_STACK];  // node records awaiting a test
 	float4 cells[FW_CELLS * TPL * (DIP ? 2 : 1)];
 	uint2 leaves[FW_LEAVES];
-	uint32_t loff[FW_LEAVES];  // exclusive prefix of the staged leaves' particle counts
+	uint32_t lsrc[FW_LEAVES];  // staged leaves' first slots less their start in the list
 	float4 pbuf[32 * TPL];     // one 32-particle chunk of opened leaves
 };
 
@@ -185,6 +186,21 @@ __device__ __forceinline__ void pair_pack(float4* buf, int p)
 	const float4 a = buf[2 * p], b = buf[2 * p + 1];
 	buf[2 * p] = make_float4(-a.x, -b.x, -a.y, -b.y);
 	buf[2 * p + 1] = make_float4(-a.z, -b.z, a.w, b.w);
+}
+
+// One chunk of 32 gathered particles, one a lane, in evaluation layout.  With
+// one target per lane neighbouring lanes exchange halves, so that each writes
+// one float4 of their pair (pair_pack's layout).
+__device__ __forceinline__ void stage_chunk(float4* buf, uint32_t lane, float4 c, Acc<1>*)
+{
+	const bool odd = (lane & 1u) != 0u;
+	const float r0 = __shfl_xor_sync(0xffffffffu, odd ? c.x : c.z, 1);
+	const float r1 = __shfl_xor_sync(0xffffffffu, odd ? c.y : c.w, 1);
+	buf[lane] = odd ? make_float4(-r0, -c.z, r1, c.w) : make_float4(-c.x, -r0, -c.y, -r1);
+}
+__device__ __forceinline__ void stage_chunk(float4* buf, uint32_t lane, float4 c, Acc<2>* tag)
+{
+	stage_src(buf, (int)lane, c, tag);
 }
 
 // the dipoles of two staged cells, (px, py, pz, 0) in slots 2p and 2p + 1,
@@ -377,6 +393,19 @@ struct FarExp {
 	}
 };
 
+// One 32-byte load of a node's record.
+__device__ __forceinline__ void load_rec(const NodeRec* r, float4& c, float& r2, uint32_t& base, uint32_t& info)
+{
+	uint32_t v[8];
+	asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+	    : "l"(r));
+	c = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+	r2 = __uint_as_float(v[4]);
+	base = v[5];
+	info = v[6];
+}
+
 // Group walk.  Returns the fields in units of q / R^2 (multiply by
 // QE / (4 pi eps0 R^2) for V/m) and the number of entries evaluated per
 // target.
@@ -438,7 +467,6 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 	}
 	const float eps2 = fmaxf(P.soft2_f, 1e-20f);
 	const float3 bc = make_float3(0.5f * (bmin.x + bmax.x), 0.5f * (bmin.y + bmax.y), 0.5f * (bmin.z + bmax.z));
-	const bool single_leaves = P.leaf_size == 1;
 	// far cells (fields of monopoles only): expanded about bc instead of staged
 	constexpr bool USE_FAR = !POT && !DIP;
 	float far2 = 3.0e38f;
@@ -480,58 +508,27 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 	const int cell_unroll = (TPL == 1 && split > 1) ? 4 : 8;
 	int len = 1, ncell = 0, nleaf = 0;
 	uint32_t n_cells_ev = 0, n_parts_ev = 0, n_far = 0;
-	if (lane == 0) sm.stack[0] = 0;
+	if (lane == 0) sm.stack[0] = 8u * T.cap;  // the root's record
 	__syncwarp();
 	for (;;) {
 		const bool done = (len == 0);
 		if (!done) {
 			const int take = len < 32 ? len : 32;
-			const int32_t code = (int)lane < take ? sm.stack[len - 1 - (int)lane] : CH_EMPTY;
+			const uint32_t node = (int)lane < take ? sm.stack[len - 1 - (int)lane] : NONE;
 			__syncwarp();
 			len -= take;
 			bool acc = false, leafr = false;
 			float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
 			float4 dipole = make_float4(0.f, 0.f, 0.f, 0.f);
 			uint2 range = make_uint2(0u, 0u);
-			int nch = 0;
-			int32_t cc[8];
-#pragma unroll
-			for (int d = 0; d < 8; d++) cc[d] = CH_EMPTY;
-			// Cells and bucket leaves load their moments from their own arrays
-			// but share one opening test and one far expansion: a round whose
-			// lanes hold both kinds runs that code once, not once per kind.  A
-			// leaf's particle range travels in c0.x, c0.y.
-			const bool is_cell = code >= 0;
-			bool tested = false, opened = false;
-			float r2 = 0.f;
-			int4 c0 = make_int4(0, 0, 0, 0), c1 = c0;
-			if (is_cell) {
-				// the child codes are loaded with the cell's moments, before the
-				// test, so an opened cell costs one round trip to L2, not two
-				const int4* cp = reinterpret_cast<const int4*>(&T.child[8u * (uint32_t)code]);
-				cell = T.f[code];
-				r2 = T.r2[code];
-				c0 = cp[0];
-				c1 = cp[1];
-				if (DIP) dipole = T.fd[code];
-				tested = true;
-			} else if (code != CH_EMPTY) {
-				const uint32_t e = leaf_payload(code);
-				if (single_leaves) {
-					leafr = true;
-					range = e < P.n_tree ? make_uint2(e, 1u) : T.ovf[e - P.n_tree];
-				} else {
-					cell = T.lf[e];
-					r2 = T.lr2[e];
-					const uint2 lr = T.lrange[e];  // with the moments, as for cells
-					c0.x = (int)lr.x;
-					c0.y = (int)lr.y;
-					if (DIP) dipole = T.lfd[e];
-					tested = true;
-				}
-			}
-			if (tested) {
-				if (group_accepts(bmin, bmax, bc, cell, r2, P.oap2_f)) {
+			uint32_t kids = 0u, base = 0u;  // an opened cell's children: mask, first record
+			if (node != NONE) {
+				uint32_t info;
+				float r2;
+				load_rec(&T.nrec[node], cell, r2, base, info);
+				if (DIP) dipole = T.drec[node];
+				const bool leaf = (info & NR_LEAF) != 0u;
+				if (!(info & NR_UNTESTED) && group_accepts(bmin, bmax, bc, cell, r2, P.oap2_f)) {
 					acc = cell.w != 0.f || (DIP && (dipole.x != 0.f || dipole.y != 0.f || dipole.z != 0.f));
 					if (USE_FAR && acc) {
 						const float fx = bc.x - cell.x, fy = bc.y - cell.y, fz = bc.z - cell.z;
@@ -541,19 +538,14 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 							n_far++;
 						}
 					}
-				} else if (is_cell) {
-					opened = true;
-					nch = (c0.x != CH_EMPTY) + (c0.y != CH_EMPTY) + (c0.z != CH_EMPTY) + (c0.w != CH_EMPTY) +
-					      (c1.x != CH_EMPTY) + (c1.y != CH_EMPTY) + (c1.z != CH_EMPTY) + (c1.w != CH_EMPTY);
-				} else {
+				} else if (leaf) {
 					leafr = true;
-					range = make_uint2((uint32_t)c0.x, (uint32_t)c0.y);
+					range = make_uint2(base, info & NR_COUNT);
+				} else {
+					kids = info;
 				}
 			}
-			if (opened) {
-				cc[0] = c0.x; cc[1] = c0.y; cc[2] = c0.z; cc[3] = c0.w;
-				cc[4] = c1.x; cc[5] = c1.y; cc[6] = c1.z; cc[7] = c1.w;
-			}
+			const int nch = __popc(kids);
 			leafr = leafr && range.y > 0u;  // the leaf flush relies on no staged leaf being empty
 			// one warp scan for the three appends: accepted cells in bits 0-9,
 			// leaf ranges in bits 10-19, children in bits 20-31 (totals <= 32,
@@ -584,8 +576,8 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 			}
 			int w = len + po;
 #pragma unroll
-			for (int d = 0; d < 8; d++)
-				if (cc[d] != CH_EMPTY) sm.stack[w++] = cc[d];
+			for (uint32_t d = 0; d < 8; d++)
+				if (kids & (1u << d)) sm.stack[w++] = base + d;
 			len += tch;
 			maxlen = max(maxlen, len);
 			__syncwarp();
@@ -645,21 +637,24 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 		// flush staged leaves: their particles are gathered 32 at a time into
 		// shared memory (dense, by a prefix sum over the leaf sizes)
 		if (nleaf >= FW_LEAF_FLUSH || (done && nleaf > 0)) {
-			const uint32_t c0 = (int)lane < nleaf ? sm.leaves[lane].y : 0u;
-			const uint32_t c1 = (int)lane + 32 < nleaf ? sm.leaves[lane + 32].y : 0u;
+			const uint2 l0 = (int)lane < nleaf ? sm.leaves[lane] : make_uint2(0u, 0u);
+			const uint2 l1 = (int)lane + 32 < nleaf ? sm.leaves[lane + 32] : make_uint2(0u, 0u);
 			int t0, t1;
-			const int e0 = warp_excl((int)c0, t0);
-			const int e1 = warp_excl((int)c1, t1);
-			sm.loff[lane] = (uint32_t)e0;
-			sm.loff[lane + 32] = (uint32_t)(t0 + e1);
+			const int e0 = warp_excl((int)l0.y, t0);
+			const int e1 = warp_excl((int)l1.y, t1);
 			const uint32_t total = (uint32_t)(t0 + t1);
-			// start offsets of this lane's two staged leaves, ~0 for none
+			// start offsets of this lane's two staged leaves, ~0 for none, and each
+			// leaf's first slot less its start: the particle at position g of the
+			// list is in slot g + lsrc[leaf]
 			const uint32_t st0 = (int)lane < nleaf ? (uint32_t)e0 : 0xFFFFFFFFu;
 			const uint32_t st1 = (int)lane + 32 < nleaf ? (uint32_t)(t0 + e1) : 0xFFFFFFFFu;
+			sm.lsrc[lane] = l0.x - (uint32_t)e0;
+			sm.lsrc[lane + 32] = l1.x - (uint32_t)(t0 + e1);
 			const uint32_t le_mask = (2u << lane) - 1u;  // lanes 0..lane (all for lane 31)
-			int before = 0;  // staged leaves that start before this chunk
+			int before = 0;  // staged leaves that start before the chunk gathered next
 			__syncwarp();
-			for (uint32_t base = 0; base < total; base += 32) {
+			// the lane's particle of the chunk at `base`
+			const auto gather = [&](uint32_t base) {
 				const uint32_t g = base + lane;
 				// the staged leaves that start inside this chunk, one bit per
 				// start offset (no leaf is empty, so no two share a start)
@@ -669,17 +664,18 @@ __device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const
 				const uint32_t starts = __reduce_or_sync(0xffffffffu, bits);
 				// padding: zero charge far outside the domain
 				float4 p = make_float4(64.f, 64.f, 64.f, 0.f);
-				if (g < total) {
-					const int a = before + __popc(starts & le_mask) - 1;  // the last leaf starting at or before g
-					p = __ldg(&src32[sm.leaves[a].x + (g - sm.loff[a])]);
-				}
+				// the last leaf starting at or before g
+				if (g < total) p = __ldg(&src32[g + sm.lsrc[before + __popc(starts & le_mask) - 1]]);
 				before += __popc(starts);
-				stage_src(sm.pbuf, (int)lane, p, tag);
+				return p;
+			};
+			float4 p = gather(0);
+			for (uint32_t base = 0; base < total; base += 32) {
+				stage_chunk(sm.pbuf, lane, p, tag);
 				__syncwarp();
-				if (TPL == 1) {
-					if (lane < 16) pair_pack(sm.pbuf, (int)lane);
-					__syncwarp();
-				}
+				// the next chunk's particles are on the way while this one's are
+				// evaluated
+				if (base + 32 < total) p = gather(base + 32);
 				constexpr int nev = 32 / PER_EV;
 				const uint32_t in_chunk = total - base < 32u ? total - base : 32u;
 				if (split == 1 && in_chunk == 32u) {
@@ -1367,7 +1363,7 @@ void launch_epe_fast(const double4* pos, const TreeDev& T, const float4* src32, 
 	if (two) {
 		k_epe_fast<2><<<sm_count_fast() * 6, FW_WARPS * 32, 0, s>>>(pos, T, src32, src64, groups_all, partial, P,
 		                                                            rec);
-	} else if (T.fd) {
+	} else if (T.drec) {
 		k_epe_fast<1, true><<<sm_count_fast() * 6, FW_WARPS * 32, 0, s>>>(pos, T, src32, src64, groups_all, partial,
 		                                                                  P, rec);
 	} else {
@@ -1385,7 +1381,7 @@ static void push_fast_stage(double4* pos, double4* vel, const TreeDev& T, const 
 	if (P.group_max > 32) {
 		k_push_fast<2, STG><<<nb, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P, rec,
 		                                                 src64, sb);
-	} else if (T.fd) {  // DIPOLES
+	} else if (T.drec) {  // DIPOLES
 		k_push_fast<1, STG, true><<<nb, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P,
 		                                                       rec, src64, sb);
 	} else {
@@ -1419,7 +1415,7 @@ void launch_field_query_fast(const TreeDev& T, const float4* src32, const double
 	if (gsize == 64) {
 		k_field_query_fast<2><<<nb, FW_WARPS * 32, 0, s>>>(T, src32, xyz, self_slot, nq, E, P, rec);
 	} else {
-		if (T.fd)
+		if (T.drec)
 			k_field_query_fast<1, true><<<nb, FW_WARPS * 32, 0, s>>>(T, src32, xyz, self_slot, nq, E, P, rec);
 		else
 			k_field_query_fast<1><<<nb, FW_WARPS * 32, 0, s>>>(T, src32, xyz, self_slot, nq, E, P, rec);
