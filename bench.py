@@ -493,16 +493,15 @@ def kernel_table(kt, N, pushes, hbm_peak):
     """Per-kernel time per launch, algorithmic bytes per launch and the
     fraction of the measured HBM bandwidth they represent.  Algorithmic
     bytes count each array a kernel must read or write once: keys (FP64
-    position in, 64-bit key and 32-bit slot out), the sort's histogram (keys
-    in) and each onesweep pass (key and slot in and out), the reorder
-    (gather of position, velocity and identity; write of the same plus FP64
-    and FP32 sources and a due flag), the compaction (due flags in, list
-    and prefix out), the fast moments (FP32 sources in, per-particle FP64
-    prefix sums out and read back per cell) and the walk (FP64 state of each
-    pushed particle in and out).  Kernels bound by latency or L2 (tree
-    build, groups, reinjection, grain update) get none."""
-    per_particle = {"keys": 32 + 12, "sort_hist": 8, "sort_pass": 24, "reorder": 72 + 117, "compact": 1 + 8,
-                    "tree_moments": 16 + 40 + 40}
+    position in, 64-bit key and 32-bit slot out) and each onesweep pass (key
+    and slot in and out), the reorder (gather of position, velocity and
+    identity; write of the same plus FP64 and FP32 sources and a due flag),
+    the due list (flags in, list and prefix out), the fast form's moment sums
+    (FP64 sources in, per-particle FP64 prefix sums out) and the walk (FP64
+    state of each pushed particle in and out).  Kernels bound by latency or
+    L2 (tree build, cell moments, groups, the step's end) get none."""
+    per_particle = {"keys": 32 + 12, "sort_pass": 24, "reorder": 72 + 117, "due_list": 1 + 8,
+                    "moment_sums": 32 + 40}
     out = {}
     for name, (ms, n) in sorted(kt.items(), key=lambda kv: -kv[1][0]):
         per = ms / max(n, 1)

@@ -33,10 +33,8 @@ struct pot_gpu_ctx {
 	uint64_t* keys[2] = { nullptr, nullptr };
 	uint32_t* vals[2] = { nullptr, nullptr };
 	int kb = 0;  // which key buffer holds the sorted keys
-	uint32_t* counts = nullptr;
-	uint32_t* block_sums = nullptr;
+	uint32_t* words = nullptr;       // the step's cleared words (StepWords)
 	uint8_t* due = nullptr;
-	uint32_t* due_tiles = nullptr;   // due flags per scan tile (counted by the reorder)
 	uint32_t* due_list = nullptr;
 	uint32_t* due_prefix = nullptr;  // n + 1
 	uint2* groups = nullptr;
@@ -69,6 +67,7 @@ struct pot_gpu_ctx {
 	cudaGraphExec_t step_exec[2][2] = { { nullptr, nullptr }, { nullptr, nullptr } };
 	uint64_t step_launches[2][2] = { { 0, 0 }, { 0, 0 } };
 	bool graphs_off = false;  // a capture failed once: enqueue kernel by kernel
+	StepStreams streams;      // side streams of a captured step
 	// the drop-in call's copy stream, chunk events and pinned records
 	cudaStream_t xfer = nullptr;
 	cudaEvent_t xev[2 * 4 + 1] = {};
@@ -513,7 +512,8 @@ static int fetch(std::vector<T>& v, const T* d, size_t n)
 }
 
 extern "C" {
-static void enqueue_step(pot_gpu_ctx* c, uint32_t flags);
+static void enqueue_step(pot_gpu_ctx* c, uint32_t flags, const StepStreams& S);
+static StepStreams step_streams(pot_gpu_ctx* c, bool fork);
 }
 
 // ---- internal interface of the batch runtime (pot_batch.cu) --------------
@@ -530,7 +530,10 @@ int ctx_enqueue(pot_gpu_ctx* c, uint32_t nsteps)
 {
 	const int rc = ctx_ready(c);
 	if (rc != POT_OK) return rc;
-	for (uint32_t k = 0; k < nsteps; k++) enqueue_step(c, 0);
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	const bool fork = cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive;
+	const StepStreams S = step_streams(c, fork);
+	for (uint32_t k = 0; k < nsteps; k++) enqueue_step(c, 0, S);
 	c->tree_valid = true;
 	return POT_OK;
 }
@@ -587,17 +590,14 @@ bool ctx_member_view(pot_gpu_ctx* c, MemberView* v)
 	}
 	v->src64 = c->src64;
 	v->src32 = c->src32;
-	v->counts = c->counts;
-	v->block_sums = c->block_sums;
+	v->words = c->words;
 	v->due = c->due;
-	v->due_tiles = c->due_tiles;
 	v->due_list = c->due_list;
 	v->due_prefix = c->due_prefix;
 	v->groups = c->groups;
 	v->rein_list = c->rein_list;
 	v->cur = (uint32_t)c->cur;
 	v->kb = (uint32_t)(radix_passes((int)c->P.key_bits) & 1);
-	v->tiles = radix_tiles(c->n);
 	return true;
 }
 }  // namespace pot
@@ -631,6 +631,7 @@ void pot_gpu_destroy(pot_gpu_ctx* c)
 	for (auto& row : c->step_exec)
 		for (auto& g : row)
 			if (g) cudaGraphExecDestroy(g);
+	c->streams.destroy();
 	if (c->xfer) cudaStreamSynchronize(c->xfer);
 	for (auto& e : c->xev)
 		if (e) cudaEventDestroy(e);
@@ -717,7 +718,6 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	const bool fast = o.form == POT_FORM_FAST;
 	const uint32_t L = o.leaf_size;
 	const uint32_t cap = (L == 1 ? 4u * n : (4u * n) / L + 8u * n / 64u) + 4096u;
-	const size_t nsum = std::max(scan_blocks(radix_counts_words(n)), scan_blocks(n)) + 16;
 #define AL(ptr, count)                         \
 	do {                                       \
 		if ((rc = dalloc(c, &(ptr), (count)))) { \
@@ -734,10 +734,8 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	}
 	AL(c->src64, n);
 	if (fast) AL(c->src32, n);
-	AL(c->counts, radix_counts_words(n));
-	AL(c->block_sums, nsum);
+	AL(c->words, StepWords::words(n, OS_MAX_PASSES));
 	AL(c->due, n);
-	AL(c->due_tiles, scan_blocks(n) + 1);
 	AL(c->due_list, n);
 	AL(c->due_prefix, (size_t)n + 1);
 	if (fast) AL(c->groups, n);
@@ -755,7 +753,6 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	TreeDev& T = c->T;
 	T.cap = cap;
 	AL(T.lvl8, n);
-	AL(T.cnt, n);
 	AL(T.base, n);
 	AL(T.first, cap);
 	AL(T.last, cap);
@@ -876,34 +873,45 @@ int pot_gpu_init_particles(pot_gpu_ctx* c)
 	return POT_OK;
 }
 
-// Keys, sort, reorder (+ due flags) and tree for the current state.
-static void enqueue_tree(pot_gpu_ctx* c, int begin_step)
+// Keys, sort, reorder (+ due flags) and tree for the current state, on the
+// branches of S.  The target groups and chi_b of a step (begin_step) go
+// beside the moments and the walk; the caller joins the two side branches.
+static void enqueue_tree(pot_gpu_ctx* c, int begin_step, const StepStreams& S)
 {
 	Params& P = c->P;
-	cudaStream_t s = c->stream;
-	uint32_t* hist = radix_sort_begin(c->counts, c->n, (int)P.key_bits, s);
-	launch_keys(c->pos[c->cur], c->keys[0], c->vals[0], P, c->rec, begin_step, hist, s, c->timer);
-	const int kb = radix_sort_pairs(c->keys, c->vals, c->n, c->counts, c->block_sums, (int)P.key_bits, s, c->timer,
-	                                &c->rec->status);
+	cudaStream_t s = S.main;
+	step_words_clear(c->words, c->n, (int)P.key_bits, s);
+	launch_keys(c->pos[c->cur], c->keys[0], c->vals[0], P, c->rec, begin_step, c->words, s, c->timer);
+	const int kb = radix_sort_pairs(c->keys, c->vals, c->n, c->words, (int)P.key_bits, s, c->timer, &c->rec->status);
 	c->kb = kb;
+	S.order(0, s, S.tree());
+	launch_cells(c->keys[kb], c->T, P, c->rec, c->words, S.tree(), c->timer);
 	const int nx = c->cur ^ 1;
-	cudaMemsetAsync(c->due_tiles, 0, sizeof(uint32_t) * scan_blocks(c->n), s);
-	launch_reorder(c->vals[kb], c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->pos[nx], c->vel[nx], c->pid[nx],
-	               c->src64, c->src32, c->due, P, c->rec, c->due_tiles, s, c->timer);
+	launch_reorder(c->keys[kb], c->vals[kb], c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->pos[nx], c->vel[nx],
+	               c->pid[nx], c->src64, c->src32, c->due, c->words, P, c->rec, s, c->timer);
 	c->cur = nx;
-	launch_build(c->keys[kb], c->T, c->src64, P, c->rec, c->block_sums, s, c->timer);
+	if (begin_step) {
+		S.order(1, s, S.list());
+		launch_due_list(c->due, c->words, c->due_list, c->due_prefix, P, c->rec, S.list(), c->timer);
+		if (P.form == POT_FORM_FAST) {
+			S.order(2, S.tree(), S.list());
+			launch_groups(c->T, c->due_prefix, c->groups, c->gcell, c->gblk, P, c->rec, S.list(), c->timer);
+		}
+	}
+	launch_mom_sums(c->T, c->src64, P, s, c->timer);
+	S.order(3, S.tree(), s);
+	launch_moments(c->T, c->src64, P, c->rec, s, c->timer);
 }
 
-static void enqueue_step(pot_gpu_ctx* c, uint32_t flags)
+static void enqueue_step(pot_gpu_ctx* c, uint32_t flags, const StepStreams& S)
 {
 	const int epe = (flags & POT_STEP_EPE) ? 1 : 0;
 	Params& P = c->P;
-	cudaStream_t s = c->stream;
-	enqueue_tree(c, 1);
-	compact_flags(c->due, c->n, c->due_list, c->due_tiles, &c->rec->n_due, s, c->timer, c->due_prefix, true);
-	if (P.form == POT_FORM_FAST)
-		launch_groups(c->T, c->due_prefix, c->groups, c->gcell, c->gblk, P, c->rec, s, c->timer);
-	launch_chi_b(c->T, c->src64, P, c->rec, 0, s, c->timer);
+	cudaStream_t s = S.main;
+	enqueue_tree(c, 1, S);
+	S.order(4, s, S.tree());
+	launch_chi_b(c->T, c->src64, P, c->rec, 0, S.tree(), c->timer);
+	S.order(5, S.list(), s);
 	if (P.integrator == POT_INT_BORIS) {
 		launch_push(c->pos[c->cur], c->vel[c->cur], c->T, c->src64, c->src32, c->due_list, c->groups, c->rein_list,
 		            P, c->rec, StageBufs { 0, nullptr, nullptr, nullptr }, s, c->timer);
@@ -920,7 +928,6 @@ static void enqueue_step(pot_gpu_ctx* c, uint32_t flags)
 		launch_push(c->pos[c->cur], c->vel[c->cur], c->T, c->src64, c->src32, c->due_list, c->groups, c->rein_list,
 		            P, c->rec, sb, s, c->timer);
 	}
-	launch_absorb_late(c->pos[c->cur], c->vel[c->cur], c->src64, c->due_list, c->rein_list, P, c->rec, s, c->timer);
 	if (epe) {
 		// with two field evaluations the energies are those of the
 		// intermediate state, whose sources the second evaluation used
@@ -928,10 +935,20 @@ static void enqueue_step(pot_gpu_ctx* c, uint32_t flags)
 		launch_epe(c->pos[c->cur], c->T, two ? c->src64b : c->src64, two ? c->src32b : c->src32, c->groups_all,
 		           c->epe_partial, P, c->rec, s, c->timer);
 	}
-	launch_reinject(c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->rein_list, c->src64, P, c->rec, s, c->timer);
-	launch_grain_end(c->pos[c->cur], c->vel[c->cur], c->hist, P, c->rec, epe, s, c->timer);
+	S.order(0, S.tree(), s);  // chi_b
+	launch_finish_step(c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->due_list, c->rein_list, c->src64, c->hist, P,
+	                   c->rec, epe, s, c->timer);
 }
 
+// The context's streams for one enqueued step; forked when the step is being
+// captured into a graph of the library's own (or a batch's).
+static StepStreams step_streams(pot_gpu_ctx* c, bool fork)
+{
+	c->streams.main = c->stream;
+	StepStreams S = c->streams;
+	S.forked = fork && S.side[0];
+	return S;
+}
 
 // One step: replay of the step's CUDA graph for the current parity (the
 // step's ~25 launches become one), captured the first time; kernel by kernel
@@ -942,7 +959,7 @@ static int step_once(pot_gpu_ctx* c, uint32_t flags)
 	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
 	if (c->graphs_off || c->timer.enabled || cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess ||
 	    cs != cudaStreamCaptureStatusNone) {
-		enqueue_step(c, flags);
+		enqueue_step(c, flags, step_streams(c, false));
 		return POT_OK;
 	}
 	const int e = (flags & POT_STEP_EPE) ? 1 : 0;
@@ -950,12 +967,13 @@ static int step_once(pot_gpu_ctx* c, uint32_t flags)
 	if (!c->step_exec[p][e]) {
 		const uint64_t l0 = c->timer.launches;
 		cudaGraph_t g = nullptr;
+		c->streams.create();  // without side streams the step is one chain
 		if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
 			c->graphs_off = true;
-			enqueue_step(c, flags);
+			enqueue_step(c, flags, step_streams(c, false));
 			return POT_OK;
 		}
-		enqueue_step(c, flags);  // records the launches; flips c->cur
+		enqueue_step(c, flags, step_streams(c, true));  // records the launches; flips c->cur
 		const cudaError_t ec = cudaStreamEndCapture(c->stream, &g);
 		const uint64_t per_step = c->timer.launches - l0;
 		c->cur = p;
@@ -968,7 +986,7 @@ static int step_once(pot_gpu_ctx* c, uint32_t flags)
 		if (!c->step_exec[p][e]) {
 			cudaGetLastError();
 			c->graphs_off = true;
-			enqueue_step(c, flags);
+			enqueue_step(c, flags, step_streams(c, false));
 			return POT_OK;
 		}
 		c->step_launches[p][e] = per_step;
@@ -1265,7 +1283,7 @@ int pot_gpu_build_tree(pot_gpu_ctx* c, uint64_t* n_nodes)
 	if (!c) return POT_E_ARG;
 	if (!c->uploaded) return POT_E_STATE;
 	CK(cudaSetDevice(c->device));
-	enqueue_tree(c, 0);
+	enqueue_tree(c, 0, step_streams(c, false));
 	CK(cudaGetLastError());
 	const int st = sync_status(c);
 	if (n_nodes) {

@@ -76,7 +76,7 @@ struct PackClass {
 	std::vector<int> slots;
 	void* mem = nullptr;
 	PackDev B {};
-	cudaStream_t st = nullptr;
+	StepStreams streams;  // main: the class's own stream
 	cudaEvent_t join = nullptr;
 };
 
@@ -105,7 +105,9 @@ static void free_packs(pot_batch* b)
 	for (auto& pc : b->packs) {
 		if (pc.mem) cudaFree(pc.mem);
 		if (pc.join) cudaEventDestroy(pc.join);
-		if (pc.st) cudaStreamDestroy(pc.st);
+		cudaStream_t st = pc.streams.main;
+		pc.streams.destroy();
+		if (st) cudaStreamDestroy(st);
 	}
 	b->packs.clear();
 }
@@ -254,12 +256,10 @@ static void member_blocks(const MemberView& v, uint32_t out[PS_COUNT])
 {
 	const uint32_t n = v.P.n, nt = v.P.n_tree, L = v.P.leaf_size;
 	out[PS_KEYS] = keys_blocks(n);
-	out[PS_N256] = div_up(n, 256);
-	out[PS_TILES] = v.tiles;
-	out[PS_CMP] = pack_scan_blocks(n);
-	out[PS_PAIRS] = div_up(nt - 1, 256);
-	out[PS_NODES] = pack_scan_blocks(nt - L);
-	out[PS_FILL] = div_up(nt - L, 256);
+	out[PS_N256] = div_up(n, REORDER_THREADS);
+	out[PS_DUE] = StepWords::due_tiles(n);
+	out[PS_TILES] = StepWords::radix_tiles(n);
+	out[PS_CELLS] = StepWords::cell_tiles(nt - L);
 	out[PS_FINISH] = div_up(nt, 256);
 	out[PS_MOM] = div_up(nt, PACK_MOM_TILE);
 	out[PS_MOMPRE] = mom_cell_blocks(nt, L);
@@ -320,7 +320,8 @@ static int plan_packs(pot_batch* b, std::vector<int>& chains)
 		}
 		pc.B.gpre = w + (size_t)PS_COUNT * (M + 1);
 		pc.B.ctr = w + (size_t)PS_COUNT * (M + 1) + (M + 1);
-		BCK(cudaStreamCreateWithFlags(&pc.st, cudaStreamNonBlocking));
+		BCK(cudaStreamCreateWithFlags(&pc.streams.main, cudaStreamNonBlocking));
+		pc.streams.forked = pc.streams.create();
 		BCK(cudaEventCreateWithFlags(&pc.join, cudaEventDisableTiming));
 	}
 	return POT_OK;
@@ -331,20 +332,28 @@ static int plan_packs(pot_batch* b, std::vector<int>& chains)
 static void enqueue_pack(const PackClass& pc, uint32_t spl)
 {
 	const PackDev& B = pc.B;
-	cudaStream_t s = pc.st;
+	const StepStreams& S = pc.streams;
+	cudaStream_t s = S.main;
 	for (uint32_t k = 0; k < spl; k++) {
 		pack_sort_begin(B, s);
 		pack_keys(B, (int)k, s);
 		pack_sort(B, s);
+		S.order(0, s, S.tree());
+		pack_cells(B, S.tree());
 		pack_reorder(B, (int)k, s);
-		pack_build(B, s);
-		pack_compact(B, s);
-		pack_groups(B, s);
-		pack_chi_b(B, s);
+		S.order(1, s, S.list());
+		pack_due_list(B, S.list());
+		S.order(2, S.tree(), S.list());
+		pack_groups(B, S.list());
+		pack_mom_sums(B, s);
+		S.order(3, S.tree(), s);
+		pack_moments(B, s);
+		S.order(4, s, S.tree());
+		pack_chi_b(B, S.tree());
+		S.order(5, S.list(), s);
 		pack_push(B, (int)k, pc.group_max > 32 ? 2u : 1u, s);
-		pack_absorb_late(B, (int)k, s);
-		pack_reinject(B, (int)k, s);
-		pack_grain_end(B, (int)k, s);
+		S.order(0, S.tree(), s);  // chi_b
+		pack_finish_step(B, (int)k, s);
 	}
 }
 
@@ -379,13 +388,13 @@ static int capture(pot_batch* b)
 	int first_err = ce == cudaSuccess ? POT_OK : POT_E_CUDA;
 	for (auto& pc : b->packs) {
 		if (first_err != POT_OK) break;
-		if (cudaStreamWaitEvent(pc.st, b->fork, 0) != cudaSuccess) {
+		if (cudaStreamWaitEvent(pc.streams.main, b->fork, 0) != cudaSuccess) {
 			first_err = POT_E_CUDA;
 			break;
 		}
 		enqueue_pack(pc, b->spl);
 		if (cudaGetLastError() != cudaSuccess) first_err = POT_E_CUDA;
-		if (cudaEventRecord(pc.join, pc.st) != cudaSuccess || cudaStreamWaitEvent(b->origin, pc.join, 0) != cudaSuccess) {
+		if (cudaEventRecord(pc.join, pc.streams.main) != cudaSuccess || cudaStreamWaitEvent(b->origin, pc.join, 0) != cudaSuccess) {
 			if (first_err == POT_OK) first_err = POT_E_CUDA;
 		}
 		for (int k : pc.slots) {

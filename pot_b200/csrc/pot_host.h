@@ -52,39 +52,58 @@ struct ScopedKernel {
 };
 
 // ---- sort.cu ------------------------------------------------------------
-constexpr int SCAN_THREADS = 1024;
-constexpr int SCAN_ITEMS = 4;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_BINS = 256;
 constexpr int OS_MAX_PASSES = 8;  // radix passes at most (64-bit keys, 8 bits each)
+constexpr int OS_TILE = 2048;     // keys per tile of a radix pass
+constexpr int TILE_THREADS = 256;  // of the cell numbering and the due list
+constexpr int CELL_TILE = 2048;   // key pairs per tile of the cell numbering
+constexpr int DUE_TILE = 4096;    // slots per tile of the due list (whole blocks of the reorder)
+constexpr int REORDER_THREADS = 256;
 
-size_t scan_blocks(size_t n);
-// out[i] = sum in[0..i); *total = sum of all (device pointer, may be null).
-void scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t* block_sums,
-                    unsigned int* total, cudaStream_t s, Timer& tm);
-// list[k] = i for the k-th i with flags[i] != 0; *count = number of such i;
-// prefix (optional, n + 1 entries) = exclusive prefix sum of the flags.
-// tiles_counted: block_sums already holds each scan tile's count of set
-// flags (the producer counted them), so the first stage is skipped.
-void compact_flags(const uint8_t* flags, size_t n, uint32_t* list, uint32_t* block_sums,
-                   unsigned int* count, cudaStream_t s, Timer& tm, uint32_t* prefix = nullptr,
-                   bool tiles_counted = false);
-size_t radix_counts_words(size_t n);
-// LSD radix sort of (keys, vals) on bits [low_bit, 64) in 8-bit passes;
-// result in keys[0]/vals[0] when the number of passes is even, keys[1]/vals[1]
-// otherwise (returns the index).
-// tiles and 8-bit passes of radix_sort_pairs for n keys sorted from low_bit
-uint32_t radix_tiles(size_t n);
+// Words of a step that start at zero: the radix sort's digit counts, the keys
+// kernel's block counter, a tile ticket counter per radix pass, the due
+// slots of each DUE_TILE and the passes' look-back status words, 256 a tile.
+// The words of the passes in use come last, so that one memset clears a
+// step's.  The cell counts of each CELL_TILE need no clearing.
+struct StepWords {
+	uint32_t* hist;      // [OS_MAX_PASSES * 256]
+	unsigned int* pass_ctr;  // [OS_MAX_PASSES]
+	unsigned int* keys_ctr;
+	uint32_t* cell;      // [cell_tiles(n)]
+	uint32_t* due;       // [due_tiles(n)]
+	uint32_t* status;    // [passes * radix_tiles(n) * 256]
+	__host__ __device__ static uint32_t radix_tiles(uint32_t n) { return (n + OS_TILE - 1) / OS_TILE; }
+	__host__ __device__ static uint32_t cell_tiles(uint32_t n) { return (n + CELL_TILE - 1) / CELL_TILE; }
+	__host__ __device__ static uint32_t due_tiles(uint32_t n) { return (n + DUE_TILE - 1) / DUE_TILE; }
+	// words before the status rows, which start on a 256-byte boundary
+	__host__ __device__ static uint32_t head(uint32_t n)
+	{
+		return (uint32_t)(OS_MAX_PASSES * RS_BINS + 16 + cell_tiles(n) + due_tiles(n) + 63) & ~63u;
+	}
+	__host__ __device__ StepWords(uint32_t* w, uint32_t n)
+	{
+		hist = w;
+		pass_ctr = w + OS_MAX_PASSES * RS_BINS;
+		keys_ctr = pass_ctr + OS_MAX_PASSES;
+		cell = w + OS_MAX_PASSES * RS_BINS + 16;
+		due = cell + cell_tiles(n);
+		status = w + head(n);
+	}
+	__host__ __device__ static size_t words(uint32_t n, int passes)
+	{
+		return head(n) + (size_t)passes * radix_tiles(n) * RS_BINS;
+	}
+};
+
+// 8-bit passes of the sort from low_bit
 int radix_passes(int low_bit);
-// Clear the sort's status words, digit counts and tile counters before the
-// keys are written; returns the digit-count array (OS_MAX_PASSES x 256) that
-// the keys kernel fills as it writes the keys.
-uint32_t* radix_sort_begin(uint32_t* counts, size_t n, int low_bit, cudaStream_t s);
-// After radix_sort_begin and the keys kernel's digit counts:
-int radix_sort_pairs(uint64_t* keys[2], uint32_t* vals[2], size_t n, uint32_t* counts, uint32_t* block_sums,
-                     int low_bit, cudaStream_t s, Timer& tm, int* err);
+// Clear the step's words; the keys kernel then counts the digits into hist.
+void step_words_clear(uint32_t* words, uint32_t n, int low_bit, cudaStream_t s);
+// After step_words_clear and the keys kernel's digit counts: LSD radix sort
+// of (keys, vals) on bits [low_bit, 64) in 8-bit passes; result in
+// keys[0]/vals[0] when the number of passes is even, keys[1]/vals[1]
+// otherwise (returns the index).
+int radix_sort_pairs(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t* words, int low_bit, cudaStream_t s,
+                     Timer& tm, int* err);
 
 }  // namespace pot

@@ -462,7 +462,7 @@ __device__ __forceinline__ bool outside_sphere(const double4& p, const Params& P
 // wall's, against the start-of-step position in src64), 2 = left the domain.
 template <class G>
 __device__ __forceinline__ void reinject_body(G grd, double4* __restrict__ pos, double4* __restrict__ vel,
-                                              const uint32_t* __restrict__ pid, const uint32_t* __restrict__ list,
+                                              const uint32_t* __restrict__ pid, const uint32_t* list,
                                               const double4* __restrict__ src64, const Params& P, RunRec* rec)
 {
 	if (rec->status != POT_OK) return;
@@ -506,10 +506,164 @@ __device__ __forceinline__ void reinject_body(G grd, double4* __restrict__ pos, 
 	}
 }
 
-__global__ void k_reinject(double4* __restrict__ pos, double4* __restrict__ vel, const uint32_t* __restrict__ pid,
-                           const uint32_t* __restrict__ list, const double4* __restrict__ src64, Params P, RunRec* rec)
+// Steps where the grain itself moves (t a multiple of tss[DUST]): the
+// reference tests absorption against the grain's new position
+// (new_parts[0], pot.c:2641-2652), so the tests run after all pushes.
+template <class G>
+__device__ __forceinline__ void absorb_late_body(G grd, double4* __restrict__ pos, double4* __restrict__ vel,
+                                                 const double4* __restrict__ src64,
+                                                 const uint32_t* __restrict__ due_list,
+                                                 uint32_t* __restrict__ rein_list, const Params& P, RunRec* rec)
 {
-	reinject_body(GridSelf {}, pos, vel, pid, list, src64, P, rec);
+	if (rec->status != POT_OK || !rec->grain_due) return;
+	const uint32_t n_due = rec->n_due;
+	const bool absorb_on = !(P.flags & FLAG_NO_GRAIN) && rec->t_steps >= P.t_settle;
+	const double4 g = pos[rec->grain_slot];
+	for (uint32_t i = grd.id() * blockDim.x + threadIdx.x; i < n_due; i += grd.n() * blockDim.x) {
+		const uint32_t s = due_list[i];
+		const double4 p = pos[s];
+		double4 v = vel[s];
+		const double4 p_old = src64[s];
+		const int sp = (int)p.w;
+		double3 xn = make_double3(p.x, p.y, p.z);
+		const uint32_t reason = after_push(sp, p_old, xn, v, P, rec, absorb_on, g.x, g.y, g.z);
+		if (P.bounce > 0.0 && !reason) {  // a bounce moved it
+			pos[s] = make_double4(xn.x, xn.y, xn.z, p.w);
+			vel[s] = v;
+		}
+		if (reason) rein_list[atomicAdd(&rec->n_rein, 1u)] = s | (reason << 30);
+	}
+}
+
+// Poisson variate by inversion (prng.c:50-70): walk the CDF from k = 0 until
+// the uniform draw is used up.  The reference loops until the term
+// underflows; the cap (the oracle's too) only ends a loop that cannot end
+// (a rate of NaN or infinity), returning 0 as the reference's exit does.
+constexpr uint32_t POISSON_CAP = 1u << 20;
+__device__ uint32_t poisson_inv(double lambda, double uni, bool& capped)
+{
+	const double e = exp(-lambda);
+	uint32_t k = 0;
+	double ratio = 1.0;
+	while (ratio != 0.0) {
+		uni = dsub(uni, dmul(ratio, e));
+		if (uni < 0.0) break;
+		k++;
+		ratio = dmul(ratio, ddiv(lambda, (double)k));
+		if (k >= POISSON_CAP) {
+			capped = true;
+			return 0;
+		}
+	}
+	return ratio != 0.0 ? k : 0;
+}
+
+// Grain update of pot.c:2825-2848 and the step's statistics.
+template <class G>
+__device__ __forceinline__ void grain_end_body(G grd, double4* __restrict__ pos, double4* __restrict__ vel,
+                                               StepHist* hist, const Params& P, RunRec* rec, int epe)
+{
+	if (threadIdx.x != 0 || grd.id() != 0) return;
+	const double dm = (double)rec->nabs_ion * P.m_ion + (double)rec->nabs_e * MASS_E;
+	const double m = rec->grain_m + dm;
+	double dp[3];
+	for (int k = 0; k < 3; k++) {
+		dp[k] = MASS_E * ((double)rec->sumv_e[k] / VFIX) + P.m_ion * ((double)rec->sumv_ion[k] / VFIX);
+	}
+	const uint32_t gs = rec->grain_slot;
+	double gv[3] = { rec->grain_vel[0], rec->grain_vel[1], rec->grain_vel[2] };
+	if (gs < P.n) {
+		const double4 v = vel[gs];
+		gv[0] = v.x; gv[1] = v.y; gv[2] = v.z;
+	}
+	for (int k = 0; k < 3; k++) gv[k] += dp[k] / m;
+	if (gs < P.n) {
+		vel[gs] = make_double4(gv[0], gv[1], gv[2], 0.0);
+		if (rec->grain_due) {
+			const double4 p = pos[gs];
+			rec->grain_pos[0] = p.x; rec->grain_pos[1] = p.y; rec->grain_pos[2] = p.z;
+		}
+	}
+	for (int k = 0; k < 3; k++) rec->grain_vel[k] = gv[k];
+	rec->grain_m = m;
+	rec->grain_q += rec->dq;
+	if ((P.flags & FLAG_POIS) && rec->t_steps >= P.t_settle) {
+		// POIS_POS_COLLECTION, pot.c:2837-2854: the OML ion flux at the cached
+		// ion temperature and the grain's charge after this step's absorptions
+		const double kb_ti = KB * rec->ion_temp;
+		double phi_normed = dmul(dmul(QE, QE), (double)rec->grain_q);
+		phi_normed = ddiv(phi_normed, dmul(dmul(dmul(4.0 * PI_REF, EPSILON0), P.a), kb_ti));
+		const double lambda = dmul(dmul(P.pos_rate_const, sqrt(kb_ti)), dsub(1.0, phi_normed));
+		Stream st;
+		st.init(P.seed, 0u, (uint32_t)rec->t_steps, 0x30000u);
+		bool capped = false;
+		const uint32_t k = poisson_inv(lambda, st.rnd(1.0), capped);
+		if (capped) rec->warn |= WARN_POISSON;
+		rec->n_collected = k;
+		rec->grain_q += k;
+	}
+	rec->q_sum += rec->grain_q;
+	rec->tot_absor_e += rec->de;
+	if (epe) {
+		// the grain's energy with its updated charge, pot.c:2859-2864
+		rec->epe[SP_DUST] = rec->grain_q ? (double)rec->grain_q * QE * rec->phi_grain : 0.0;
+	}
+	StepHist h;
+	h.t_steps = rec->t_steps;
+	h.grain_q = rec->grain_q;
+	h.dq = rec->dq;
+	h.de = rec->de;
+	h.n_absorbed = rec->nabs_ion + rec->nabs_e;
+	h.n_reinjected = rec->n_rein;
+	h.n_pushed = rec->n_pushed;
+	h.interactions = rec->interactions;
+	h.far_cells = rec->far_cells;
+	h.n_nodes = rec->n_nodes;
+	h.chi_b = rec->chi_b;
+	h.status = rec->status;
+	h.pad = (int)rec->warn;
+	for (int k = 0; k < 3; k++) h.epe[k] = epe ? rec->epe[k] : 0.0;
+	hist[rec->t_steps % HIST] = h;
+}
+
+// The end of a step, one launch: the late absorption of a step on which the
+// grain moves, the reinjections, then -- by the block that finishes last --
+// the grain update and the step's statistics.  On a step on which the grain
+// moves (rare: every tss[DUST] steps) the list of reinjections is complete
+// only when every block has tested its particles, so the last block makes
+// them all.
+template <class G>
+__device__ __forceinline__ void finish_step_body(G grd, double4* __restrict__ pos, double4* __restrict__ vel,
+                                                 const uint32_t* __restrict__ pid,
+                                                 const uint32_t* __restrict__ due_list, uint32_t* rein_list,
+                                                 const double4* __restrict__ src64, StepHist* hist, const Params& P,
+                                                 RunRec* rec, int epe)
+{
+	__shared__ bool s_last;
+	const bool late = rec->grain_due != 0;
+	if (late) absorb_late_body(grd, pos, vel, src64, due_list, rein_list, P, rec);
+	else reinject_body(grd, pos, vel, pid, rein_list, src64, P, rec);
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0) s_last = atomicAdd(&rec->done_ctr, 1u) + 1u == grd.n();
+	__syncthreads();
+	if (!s_last) return;
+	__threadfence();
+	if (late) {
+		reinject_body(GridSeg { 0, 1 }, pos, vel, pid, rein_list, src64, P, rec);
+		__threadfence();
+		__syncthreads();
+	}
+	grain_end_body(GridSeg { 0, 1 }, pos, vel, hist, P, rec, epe);
+}
+
+__global__ void __launch_bounds__(128) k_finish_step(double4* __restrict__ pos, double4* __restrict__ vel,
+                                                     const uint32_t* __restrict__ pid,
+                                                     const uint32_t* __restrict__ due_list, uint32_t* rein_list,
+                                                     const double4* __restrict__ src64, StepHist* hist, Params P,
+                                                     RunRec* rec, int epe)
+{
+	finish_step_body(GridSelf {}, pos, vel, pid, due_list, rein_list, src64, hist, P, rec, epe);
 }
 
 // init_particles for one rank (pot.c:887-935), reference order: slot i holds
@@ -539,11 +693,12 @@ __global__ void k_init(double4* __restrict__ pos, double4* __restrict__ vel, uin
 	vel[i] = v;
 }
 
-void launch_reinject(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* rein_list,
-                     const double4* src64, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm)
+void launch_finish_step(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* due_list, uint32_t* rein_list,
+                        const double4* src64, StepHist* hist, const Params& P, RunRec* rec, int epe, cudaStream_t s,
+                        Timer& tm)
 {
-	ScopedKernel k(tm, "reinject");
-	k_reinject<<<148, 128, 0, s>>>(pos, vel, pid, rein_list, src64, P, rec);
+	ScopedKernel k(tm, "finish_step");
+	k_finish_step<<<148, 128, 0, s>>>(pos, vel, pid, due_list, rein_list, src64, hist, P, rec, epe);
 }
 
 void launch_init(double4* pos, double4* vel, uint32_t* pid, const Params& P, RunRec* rec, cudaStream_t s,
@@ -556,21 +711,22 @@ void launch_init(double4* pos, double4* vel, uint32_t* pid, const Params& P, Run
 }  // namespace pot
 
 // ---------------------------------------------------------------------------
-// packed batch: the reinjection of every member in one launch
+// packed batch: the end of every member's step in one launch
 // ---------------------------------------------------------------------------
 namespace pot {
 
-__global__ void kp_reinject(PackDev B, int k)
+__global__ void __launch_bounds__(128) kp_finish_step(PackDev B, int k)
 {
 	const SegBlock sb = seg_block(B.pre[PS_SMALL], B.M);
 	const MemberView& v = B.mv[sb.m];
 	const uint32_t b = pack_out(v, k);
-	reinject_body(GridSeg { sb.id, sb.n }, v.pos[b], v.vel[b], v.pid[b], v.rein_list, v.src64, v.P, v.rec);
+	finish_step_body(GridSeg { sb.id, sb.n }, v.pos[b], v.vel[b], v.pid[b], v.due_list, v.rein_list, v.src64, v.hist,
+	                 v.P, v.rec, 0);
 }
 
-void pack_reinject(const PackDev& B, int k, cudaStream_t s)
+void pack_finish_step(const PackDev& B, int k, cudaStream_t s)
 {
-	kp_reinject<<<B.blocks[PS_SMALL], 128, 0, s>>>(B, k);
+	kp_finish_step<<<B.blocks[PS_SMALL], 128, 0, s>>>(B, k);
 }
 
 }  // namespace pot

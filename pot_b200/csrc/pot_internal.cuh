@@ -106,7 +106,7 @@ struct RunRec {
 	unsigned int n_collected;  // Poisson ion collection: charges added this step
 	unsigned int n_wall;       // OUT_BOUNCE: particles outside moving inwards this step
 	unsigned int n_bounced;    // OUT_BOUNCE: particles bounced this step
-	unsigned int pad_v;
+	unsigned int done_ctr;     // blocks of the step's last kernel that are done
 	double ion_temp;           // cached ion temperature of the Poisson collection (Proc.Ti)
 };
 

@@ -72,19 +72,23 @@ __device__ __forceinline__ uint64_t scaled_key(double x, double y, double z, dou
 	return (spread3(ix) << 2) | (spread3(iy) << 1) | spread3(iz);
 }
 
-// Keys of every particle (grid-stride) and, when hist is given, the digit
-// counts of each of the radix sort's npass 8-bit passes from low_bit,
-// hist[p * 256 + d], counted in shared memory and added once per block: the
-// sort then needs no read of the keys of its own for them.
+// Keys of every particle (grid-stride) and the digit counts of each of the
+// radix sort's npass 8-bit passes from low_bit, counted in shared memory and
+// added once per block to hist[p * 256 + d]: the sort then needs no read of
+// the keys of its own for them.
 template <class G>
 __device__ __forceinline__ void keys_body(G grd, const double4* __restrict__ pos, uint64_t* __restrict__ keys,
                                           uint32_t* __restrict__ vals, const Params& P, RunRec* rec, int begin_step,
-                                          uint32_t* __restrict__ hist, int low_bit, int npass)
+                                          uint32_t* hist, unsigned int* ctr, int low_bit, int npass)
 {
 	__shared__ uint32_t h[OS_MAX_PASSES][RS_BINS];
-	if (hist) {
-		for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x) (&h[0][0])[i] = 0;
-		__syncthreads();
+	__shared__ bool s_last;
+	for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x) (&h[0][0])[i] = 0;
+	__syncthreads();
+	if (grd.id() == 0 && threadIdx.x == 0) {
+		rec->n_overflow = 0;
+		rec->n_groups = 0;
+		rec->n_groups_all = 0;
 	}
 	if (begin_step && grd.id() == 0 && threadIdx.x == 0) {
 		const unsigned long long t = rec->t_steps + 1;
@@ -107,6 +111,7 @@ __device__ __forceinline__ void keys_body(G grd, const double4* __restrict__ pos
 		rec->n_collected = 0;
 		rec->n_wall = 0;
 		rec->n_bounced = 0;
+		rec->done_ctr = 0;
 		rec->grain_slot = 0xFFFFFFFFu;
 	}
 	for (uint32_t s = grd.id() * blockDim.x + threadIdx.x; s < P.n; s += grd.n() * blockDim.x) {
@@ -124,34 +129,63 @@ __device__ __forceinline__ void keys_body(G grd, const double4* __restrict__ pos
 		                                                   : morton_key(p.x, p.y, p.z, P.root_w);
 		keys[s] = k;
 		vals[s] = s;
-		if (hist)
-			for (int q = 0; q < npass; q++) atomicAdd(&h[q][(k >> (low_bit + 8 * q)) & 0xFF], 1u);
+		for (int q = 0; q < npass; q++) atomicAdd(&h[q][(k >> (low_bit + 8 * q)) & 0xFF], 1u);
 	}
-	if (hist) {
-		__syncthreads();
-		for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x) {
-			const uint32_t c = (&h[0][0])[i];
-			if (c) atomicAdd(&hist[i], c);
-		}
+	__syncthreads();
+	for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x) {
+		const uint32_t c = (&h[0][0])[i];
+		if (c) atomicAdd(&hist[i], c);
 	}
+	// the last block turns each pass's counts into the digits' starts in the
+	// sorted order (one warp a pass, eight digits a lane)
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0) s_last = atomicAdd(ctr, 1u) + 1u == grd.n();
+	__syncthreads();
+	const int p = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
+	if (!s_last || p >= npass) return;
+	__threadfence();
+	uint4* row = reinterpret_cast<uint4*>(hist + p * RS_BINS) + 2 * lane;
+	uint4 a = __ldcg(row), b = __ldcg(row + 1);
+	const uint32_t sum = a.x + a.y + a.z + a.w + b.x + b.y + b.z + b.w;
+	uint32_t run = sum;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t v = __shfl_up_sync(0xffffffffu, run, o);
+		if (lane >= o) run += v;
+	}
+	run -= sum;
+	uint32_t c;
+	c = a.x; a.x = run; run += c;
+	c = a.y; a.y = run; run += c;
+	c = a.z; a.z = run; run += c;
+	c = a.w; a.w = run; run += c;
+	c = b.x; b.x = run; run += c;
+	c = b.y; b.y = run; run += c;
+	c = b.z; b.z = run; run += c;
+	b.w = run;
+	row[0] = a;
+	row[1] = b;
 }
 
-__global__ void k_keys(const double4* __restrict__ pos, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                       Params P, RunRec* rec, int begin_step, uint32_t* __restrict__ hist, int low_bit, int npass)
+__global__ void __launch_bounds__(256) k_keys(const double4* __restrict__ pos, uint64_t* __restrict__ keys,
+                                              uint32_t* __restrict__ vals, Params P, RunRec* rec, int begin_step,
+                                              uint32_t* words, int low_bit, int npass)
 {
-	keys_body(GridSelf {}, pos, keys, vals, P, rec, begin_step, hist, low_bit, npass);
+	const StepWords W(words, P.n);
+	keys_body(GridSelf {}, pos, keys, vals, P, rec, begin_step, W.hist, W.keys_ctr, low_bit, npass);
 }
 
 // Gather the state into the new Morton order, write the tree sources and
 // mark the particles due this step (electrons every step, ions every
 // tss[ION] steps, the grain every tss[DUST] steps, pot.c:2430-2434).
 // One slot of the reorder; returns whether the particle is due.
-__device__ __forceinline__ bool reorder_one(uint32_t s, const uint32_t* __restrict__ perm,
-                                            const double4* __restrict__ pos_in, const double4* __restrict__ vel_in,
-                                            const uint32_t* __restrict__ pid_in, double4* __restrict__ pos_out,
-                                            double4* __restrict__ vel_out, uint32_t* __restrict__ pid_out,
-                                            double4* __restrict__ src64, float4* __restrict__ src32,
-                                            uint8_t* __restrict__ due, const Params& P, RunRec* rec)
+__device__ __forceinline__ bool reorder_one(uint32_t s, const uint64_t* __restrict__ keys,
+                                            const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+                                            const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in,
+                                            double4* __restrict__ pos_out, double4* __restrict__ vel_out,
+                                            uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
+                                            float4* __restrict__ src32, const Params& P, RunRec* rec)
 {
 	const uint32_t j = perm[s];
 	const double4 p = pos_in[j];
@@ -167,49 +201,148 @@ __device__ __forceinline__ bool reorder_one(uint32_t s, const uint32_t* __restri
 		src32[s] = make_float4((float)((p.x - P.rad) * P.inv_rad), (float)((p.y - P.rad) * P.inv_rad),
 		                       (float)((p.z - P.rad) * P.inv_rad), (float)q);
 	}
-	const bool d = (rec->t_steps % P.tss[sp]) == 0;
-	due[s] = d ? 1 : 0;
 	if (sp == SP_DUST) rec->grain_slot = s;
-	return d;
+	// Two particles at one position: the reference's insertion would split
+	// forever (pot.c:1466-1470) or fail at a reallocation (pot.c:1578-1586).
+	if (s + 1 < P.n_tree && keys[s] == keys[s + 1]) {
+		const double4 o = pos_in[perm[s + 1]];
+		if (p.x == o.x && p.y == o.y && p.z == o.z) set_status(rec, POT_E_COINCIDENT);
+	}
+	return (rec->t_steps % P.tss[sp]) == 0;
 }
 
-
 template <class G>
-__device__ __forceinline__ void reorder_body(G grd, const uint32_t* __restrict__ perm,
-                                             const double4* __restrict__ pos_in, const double4* __restrict__ vel_in,
-                                             const uint32_t* __restrict__ pid_in, double4* __restrict__ pos_out,
-                                             double4* __restrict__ vel_out, uint32_t* __restrict__ pid_out,
-                                             double4* __restrict__ src64, float4* __restrict__ src32,
-                                             uint8_t* __restrict__ due, const Params& P, RunRec* rec,
-                                             uint32_t* __restrict__ due_tiles)
+__device__ __forceinline__ void reorder_body(G grd, const uint64_t* __restrict__ keys,
+                                             const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+                                             const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in,
+                                             double4* __restrict__ pos_out, double4* __restrict__ vel_out,
+                                             uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
+                                             float4* __restrict__ src32, uint8_t* __restrict__ due,
+                                             uint32_t* __restrict__ due_tiles, const Params& P, RunRec* rec)
 {
-	const uint32_t s = grd.id() * blockDim.x + threadIdx.x;
-	// the due flags' count per scan tile of SCAN_TILE slots (the compaction's
-	// first stage; a 256-thread block lies inside one tile)
+	const uint32_t s = grd.id() * REORDER_THREADS + threadIdx.x;
+	// the due slots of each DUE_TILE (a block lies inside one)
 	bool is_due = false;
-	if (s < P.n) is_due = reorder_one(s, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, due,
-	                                  P, rec);
-	if (due_tiles) {
-		__shared__ uint32_t wcnt[32];
-		const uint32_t c = __popc(__ballot_sync(0xffffffffu, is_due));
-		if ((threadIdx.x & 31) == 0) wcnt[threadIdx.x >> 5] = c;
-		__syncthreads();
-		if (threadIdx.x == 0) {
-			uint32_t t = 0;
-			for (uint32_t w = 0; w < (blockDim.x >> 5); w++) t += wcnt[w];
-			if (t) atomicAdd(&due_tiles[(grd.id() * blockDim.x) / SCAN_TILE], t);
+	if (s < P.n) {
+		is_due = reorder_one(s, keys, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, P, rec);
+		due[s] = is_due ? 1 : 0;
+	}
+	__shared__ uint32_t wcnt[REORDER_THREADS / 32];
+	const uint32_t c = __popc(__ballot_sync(0xffffffffu, is_due));
+	if ((threadIdx.x & 31) == 0) wcnt[threadIdx.x >> 5] = c;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		uint32_t t = 0;
+		for (uint32_t w = 0; w < REORDER_THREADS / 32; w++) t += wcnt[w];
+		if (t) atomicAdd(&due_tiles[(grd.id() * REORDER_THREADS) / DUE_TILE], t);
+	}
+}
+
+__global__ void __launch_bounds__(REORDER_THREADS)
+k_reorder(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+          const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in, double4* __restrict__ pos_out,
+          double4* __restrict__ vel_out, uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
+          float4* __restrict__ src32, uint8_t* __restrict__ due, uint32_t* words, Params P, RunRec* rec)
+{
+	reorder_body(GridSelf {}, keys, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, due,
+	             StepWords(words, P.n).due, P, rec);
+}
+
+// Exclusive prefix of tile `tile` over the tiles' counts, by the whole block:
+// each block adds up the counts of the tiles before its own (at most some
+// thousands of words from L2), so a scan needs no launch between the kernel
+// that counts and the one that places.
+__device__ __forceinline__ uint32_t tiles_before(const uint32_t* __restrict__ counts, uint32_t tile)
+{
+	__shared__ uint32_t part[TILE_THREADS / 32];
+	uint32_t s = 0;
+	for (uint32_t i = threadIdx.x; i < tile; i += TILE_THREADS) s += counts[i];
+	s = __reduce_add_sync(0xffffffffu, s);
+	if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+	__syncthreads();
+	uint32_t t = 0;
+#pragma unroll
+	for (int k = 0; k < TILE_THREADS / 32; k++) t += part[k];
+	__syncthreads();
+	return t;
+}
+
+// Exclusive block scan of one value per thread (TILE_THREADS threads);
+// *total = block sum.
+__device__ __forceinline__ uint32_t tile_scan(uint32_t v, uint32_t* total)
+{
+	__shared__ uint32_t wsum[TILE_THREADS / 32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	uint32_t incl = v;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+		if (lane >= o) incl += u;
+	}
+	if (lane == 31) wsum[w] = incl;
+	__syncthreads();
+	uint32_t before = 0, tot = 0;
+#pragma unroll
+	for (int k = 0; k < TILE_THREADS / 32; k++) {
+		const uint32_t c = wsum[k];
+		if (k < w) before += c;
+		tot += c;
+	}
+	__syncthreads();
+	*total = tot;
+	return before + incl - v;
+}
+
+// The due list: due_list[k] is the k-th due slot, due_prefix[s] the number of
+// due slots before s; one DUE_TILE a block, 16 slots a thread.
+template <class G>
+__device__ __forceinline__ void due_list_body(G grd, const uint8_t* __restrict__ due,
+                                              const uint32_t* __restrict__ counts, uint32_t* __restrict__ due_list,
+                                              uint32_t* __restrict__ due_prefix, const Params& P, RunRec* rec)
+{
+	constexpr int ITEMS = DUE_TILE / TILE_THREADS;  // 16: one 16-byte load of flags
+	const uint32_t tile = grd.id(), n = P.n, s0 = tile * DUE_TILE + threadIdx.x * ITEMS;
+	const uint32_t base = tiles_before(counts, tile);
+	uint32_t bits = 0;
+	if (s0 + ITEMS <= n) {
+		const uint4 f = *reinterpret_cast<const uint4*>(due + s0);
+		const uint32_t q[4] = { f.x, f.y, f.z, f.w };
+#pragma unroll
+		for (int k = 0; k < ITEMS; k++) bits |= ((q[k >> 2] >> (8 * (k & 3))) & 1u) << k;
+	} else {
+		for (int k = 0; k < ITEMS; k++)
+			if (s0 + (uint32_t)k < n && due[s0 + k]) bits |= 1u << k;
+	}
+	uint32_t total;
+	uint32_t run = base + tile_scan(__popc(bits), &total);
+	if (threadIdx.x == 0 && (uint64_t)(tile + 1) * DUE_TILE >= n) {
+		rec->n_due = base + total;
+		due_prefix[n] = base + total;
+	}
+#pragma unroll
+	for (int k = 0; k < ITEMS; k += 4) {
+		uint4 o;
+		uint32_t* const op = &o.x;
+#pragma unroll
+		for (int u = 0; u < 4; u++) {
+			const uint32_t s = s0 + (uint32_t)(k + u);
+			op[u] = run;
+			if ((bits >> (k + u)) & 1u) due_list[run++] = s;
+		}
+		if (s0 + (uint32_t)(k + 4) <= n) {
+			*reinterpret_cast<uint4*>(due_prefix + s0 + k) = o;
+		} else {
+			for (int u = 0; u < 4; u++)
+				if (s0 + (uint32_t)(k + u) < n) due_prefix[s0 + k + u] = op[u];
 		}
 	}
 }
 
-__global__ void k_reorder(const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
-                          const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in,
-                          double4* __restrict__ pos_out, double4* __restrict__ vel_out,
-                          uint32_t* __restrict__ pid_out, double4* __restrict__ src64, float4* __restrict__ src32,
-                          uint8_t* __restrict__ due, Params P, RunRec* rec, uint32_t* __restrict__ due_tiles)
+__global__ void __launch_bounds__(TILE_THREADS)
+k_due_list(const uint8_t* __restrict__ due, const uint32_t* __restrict__ words_due, uint32_t* __restrict__ due_list,
+           uint32_t* __restrict__ due_prefix, Params P, RunRec* rec)
 {
-	reorder_body(GridSelf {}, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, due, P, rec,
-	             due_tiles);
+	due_list_body(GridSelf {}, due, words_due, due_list, due_prefix, P, rec);
 }
 
 __device__ __forceinline__ int lcp_levels(uint64_t a, uint64_t b)
@@ -219,65 +352,90 @@ __device__ __forceinline__ int lcp_levels(uint64_t a, uint64_t b)
 	return (__clzll((long long)x) - 1) / 3;
 }
 
-// lvl8[i] = common levels of keys i and i + L (capped at 20: a level-21
-// cell cannot split); cnt[i] = number of cells pair i owns.
-template <class G>
-__device__ __forceinline__ void pairs_body(G grd, const uint64_t* __restrict__ keys,
-                                           const double4* __restrict__ src64, uint32_t n, uint32_t n_pairs,
-                                           uint32_t L, int max_level, int8_t* __restrict__ lvl8,
-                                           uint32_t* __restrict__ cnt, RunRec* rec)
+// Common levels of keys i and i + L, capped at max_level - 1 (a cell of the
+// deepest level cannot split).
+__device__ __forceinline__ int pair_levels(const uint64_t* __restrict__ keys, uint32_t i, uint32_t L, int max_level,
+                                           RunRec* rec)
 {
-	const uint32_t i = grd.id() * blockDim.x + threadIdx.x;
-	// Two particles at one position: the reference's insertion would split
-	// forever (pot.c:1466-1470) or fail at a reallocation (pot.c:1578-1586).
-	if (i + 1 < n && keys[i] == keys[i + 1]) {
-		const double4 a = src64[i], b = src64[i + 1];
-		if (a.x == b.x && a.y == b.y && a.z == b.z) set_status(rec, POT_E_COINCIDENT);
-	}
-	if (i >= n_pairs) return;
-	const int li = lcp_levels(keys[i], keys[i + L]);
-	if (li == MAX_LEVELS && max_level == MAX_LEVELS) atomicOr(&rec->warn, 1u);
-	const int hi = li < max_level - 1 ? li : max_level - 1;
-	int prev = -1;
-	if (i > 0) {
-		const int lp = lcp_levels(keys[i - 1], keys[i - 1 + L]);
-		prev = lp < max_level - 1 ? lp : max_level - 1;
-	}
-	lvl8[i] = (int8_t)hi;
-	cnt[i] = hi > prev ? (uint32_t)(hi - prev) : 0u;
+	const int l = lcp_levels(keys[i], keys[i + L]);
+	if (l == MAX_LEVELS && max_level == MAX_LEVELS && rec) atomicOr(&rec->warn, 1u);
+	return l < max_level - 1 ? l : max_level - 1;
 }
 
-__global__ void k_pairs(const uint64_t* __restrict__ keys, const double4* __restrict__ src64, uint32_t n,
-                        uint32_t n_pairs, uint32_t L, int max_level, int8_t* __restrict__ lvl8,
-                        uint32_t* __restrict__ cnt, RunRec* rec)
-{
-	pairs_body(GridSelf {}, keys, src64, n, n_pairs, L, max_level, lvl8, cnt, rec);
-}
-
-template <class G>
-__device__ __forceinline__ void fill_nodes_body(G grd, const int8_t* __restrict__ lvl8,
-                                                const uint32_t* __restrict__ base, uint32_t n_pairs, const TreeDev& T,
-                                                RunRec* rec)
-{
-	const uint32_t i = grd.id() * blockDim.x + threadIdx.x;
-	if (i >= n_pairs) return;
-	const int hi = lvl8[i];
-	const int lo = i == 0 ? 0 : lvl8[i - 1] + 1;
-	for (int l = lo; l <= hi; l++) {
-		const uint32_t k = base[i] + (uint32_t)(l - lo);
-		if (k >= T.cap) {
-			set_status(rec, POT_E_CAPACITY);
-			return;
+// Cell numbering in two launches over tiles of CELL_TILE key pairs.  Pair i
+// owns the cells of levels (lvl8[i-1], lvl8[i]], lvl8[i] its common levels:
+// the first launch counts the cells each tile owns, the second adds up the
+// counts before its tile, numbers its cells (base[i]: pair i's first) and
+// writes their first slot and level.
+struct PairLevels {
+	int lv[CELL_TILE / TILE_THREADS + 1];  // lv[0]: the pair before this thread's first
+	uint32_t sum;
+	__device__ __forceinline__ PairLevels(const uint64_t* __restrict__ keys, uint32_t i0, uint32_t n_pairs, uint32_t L,
+	                                      int max_level, RunRec* rec)
+	{
+		lv[0] = i0 > 0 && i0 - 1 < n_pairs ? pair_levels(keys, i0 - 1, L, max_level, nullptr) : -1;
+		sum = 0;
+#pragma unroll
+		for (int k = 0; k < CELL_TILE / TILE_THREADS; k++) {
+			const uint32_t i = i0 + (uint32_t)k;
+			lv[k + 1] = i < n_pairs ? pair_levels(keys, i, L, max_level, rec) : -1;
+			if (lv[k + 1] > lv[k]) sum += (uint32_t)(lv[k + 1] - lv[k]);
 		}
-		T.first[k] = i;
-		T.level[k] = (uint8_t)l;
+	}
+};
+
+template <class G>
+__device__ __forceinline__ void cell_count_body(G grd, const uint64_t* __restrict__ keys, uint32_t n_pairs, uint32_t L,
+                                                int max_level, uint32_t* __restrict__ counts, RunRec* rec)
+{
+	const uint32_t i0 = grd.id() * CELL_TILE + threadIdx.x * (CELL_TILE / TILE_THREADS);
+	const PairLevels p(keys, i0, n_pairs, L, max_level, rec);
+	uint32_t total;
+	tile_scan(p.sum, &total);
+	if (threadIdx.x == 0) counts[grd.id()] = total;
+}
+
+template <class G>
+__device__ __forceinline__ void cell_number_body(G grd, const uint64_t* __restrict__ keys, uint32_t n_pairs, uint32_t L,
+                                                 int max_level, const uint32_t* __restrict__ counts, const TreeDev& T,
+                                                 RunRec* rec)
+{
+	const uint32_t tile = grd.id(), i0 = tile * CELL_TILE + threadIdx.x * (CELL_TILE / TILE_THREADS);
+	const PairLevels p(keys, i0, n_pairs, L, max_level, nullptr);
+	const uint32_t base = tiles_before(counts, tile);
+	uint32_t total;
+	uint32_t run = base + tile_scan(p.sum, &total);
+	if (threadIdx.x == 0 && (uint64_t)(tile + 1) * CELL_TILE >= n_pairs) rec->n_nodes = base + total;
+#pragma unroll
+	for (int k = 0; k < CELL_TILE / TILE_THREADS; k++) {
+		const uint32_t i = i0 + (uint32_t)k;
+		if (i >= n_pairs) break;
+		T.lvl8[i] = (int8_t)p.lv[k + 1];
+		T.base[i] = run;
+		for (int l = p.lv[k] + 1; l <= p.lv[k + 1]; l++, run++) {
+			if (run >= T.cap) {
+				set_status(rec, POT_E_CAPACITY);
+				break;
+			}
+			T.first[run] = i;
+			T.level[run] = (uint8_t)l;
+		}
 	}
 }
 
-__global__ void k_fill_nodes(const int8_t* __restrict__ lvl8, const uint32_t* __restrict__ base, uint32_t n_pairs,
-                             TreeDev T, RunRec* rec)
+__global__ void __launch_bounds__(TILE_THREADS) k_cell_count(const uint64_t* __restrict__ keys, uint32_t n_pairs,
+                                                             uint32_t L, int max_level, uint32_t* __restrict__ counts,
+                                                             RunRec* rec)
 {
-	fill_nodes_body(GridSelf {}, lvl8, base, n_pairs, T, rec);
+	cell_count_body(GridSelf {}, keys, n_pairs, L, max_level, counts, rec);
+}
+
+__global__ void __launch_bounds__(TILE_THREADS) k_cell_number(const uint64_t* __restrict__ keys, uint32_t n_pairs,
+                                                              uint32_t L, int max_level,
+                                                              const uint32_t* __restrict__ counts, TreeDev T,
+                                                              RunRec* rec)
+{
+	cell_number_body(GridSelf {}, keys, n_pairs, L, max_level, counts, T, rec);
 }
 
 // The searches below run over a cell's sorted key range, where the tested
@@ -688,28 +846,24 @@ __global__ void __launch_bounds__(MOM_THREADS) k_mom_reduce(const double4* __res
 	mom_reduce_body<K>(GridSelf {}, src64, n, c, bsum);
 }
 
-template <class G>
-__device__ __forceinline__ void mom_top_body(G grd, Mom5* __restrict__ bsum, uint32_t nb)
+// Sum of the block totals before block `id`, added in a fixed order: block
+// scans of MOM_THREADS totals and a running carry.  Every block works its
+// own out, so no launch is needed between the totals and their use.
+__device__ Mom5 mom_before(const Mom5* __restrict__ bsum, uint32_t id)
 {
-	__shared__ Mom5 tot;
-	__shared__ Mom5 carry;
-	if (threadIdx.x == 0) carry = Mom5 { 0, 0, 0, 0, 0 };
-	__syncthreads();
-	for (uint32_t base = 0; base < nb; base += MOM_THREADS) {
+	__shared__ Mom5 tot, mine;
+	Mom5 carry = Mom5 { 0, 0, 0, 0, 0 };
+	for (uint32_t base = 0;; base += MOM_THREADS) {
 		const uint32_t i = base + threadIdx.x;
-		const Mom5 v = i < nb ? bsum[i] : Mom5 { 0, 0, 0, 0, 0 };
+		const Mom5 v = i <= id ? bsum[i] : Mom5 { 0, 0, 0, 0, 0 };  // its own enters the scan it is left out of
 		const Mom5 e = mom_block_excl(v, &tot);
-		const Mom5 c = carry;
-		if (i < nb) bsum[i] = mom_add(c, e);
-		__syncthreads();
-		if (threadIdx.x == 0) carry = mom_add(c, tot);
+		if (i == id) mine = mom_add(carry, e);
+		if (id < base + MOM_THREADS) break;
+		carry = mom_add(carry, tot);
 		__syncthreads();
 	}
-}
-
-__global__ void __launch_bounds__(MOM_THREADS) k_mom_top(Mom5* __restrict__ bsum, uint32_t nb)
-{
-	mom_top_body(GridSelf {}, bsum, nb);
+	__syncthreads();
+	return mine;
 }
 
 template <int K, class G>
@@ -734,7 +888,8 @@ __device__ __forceinline__ void mom_down_body(G grd, const double4* __restrict__
 		                        __shfl_xor_sync(0xffffffffu, wt.z, o) });
 	}
 	const Mom5 mine = lane == 0 ? wt : Mom5 { 0, 0, 0, 0, 0 };
-	Mom5 carry = mom_add(bsum[grd.id()], mom_block_excl(mine, &tot));  // valid on lane 0
+	const Mom5 before = mom_before(bsum, grd.id());
+	Mom5 carry = mom_add(before, mom_block_excl(mine, &tot));  // valid on lane 0
 	carry = mom_shfl(carry, 0);
 	for (int k = 0; k < MOM_ITEMS; k++) {
 		const size_t i = base + (size_t)k * 32 + lane;
@@ -855,65 +1010,75 @@ static inline uint32_t blocks_for(size_t n, int threads) { return (uint32_t)((n 
 uint32_t keys_blocks(size_t n) { return std::min<uint32_t>(blocks_for(n, 256), 148u * 8u); }
 
 void launch_keys(const double4* pos, uint64_t* keys, uint32_t* vals, const Params& P, RunRec* rec,
-                 int begin_step, uint32_t* hist, cudaStream_t s, Timer& tm)
+                 int begin_step, uint32_t* words, cudaStream_t s, Timer& tm)
 {
 	ScopedKernel k(tm, "keys");
-	k_keys<<<keys_blocks(P.n), 256, 0, s>>>(pos, keys, vals, P, rec, begin_step, hist, (int)P.key_bits,
+	k_keys<<<keys_blocks(P.n), 256, 0, s>>>(pos, keys, vals, P, rec, begin_step, words, (int)P.key_bits,
 	                                        radix_passes((int)P.key_bits));
 }
 
-void launch_reorder(const uint32_t* perm, const double4* pos_in, const double4* vel_in, const uint32_t* pid_in,
-                    double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64, float4* src32,
-                    uint8_t* due, const Params& P, RunRec* rec, uint32_t* due_tiles, cudaStream_t s, Timer& tm)
+void launch_reorder(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, const double4* vel_in,
+                    const uint32_t* pid_in, double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64,
+                    float4* src32, uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s,
+                    Timer& tm)
 {
 	ScopedKernel k(tm, "reorder");
-	k_reorder<<<blocks_for(P.n, 256), 256, 0, s>>>(perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out,
-	                                               src64, src32, due, P, rec, due_tiles);
+	k_reorder<<<blocks_for(P.n, REORDER_THREADS), REORDER_THREADS, 0, s>>>(keys, perm, pos_in, vel_in, pid_in, pos_out,
+	                                                                       vel_out, pid_out, src64, src32, due, words,
+	                                                                       P, rec);
 }
 
-void launch_build(const uint64_t* keys, TreeDev& T, const double4* src64, const Params& P, RunRec* rec,
-                  uint32_t* block_sums, cudaStream_t s, Timer& tm)
+void launch_due_list(const uint8_t* due, uint32_t* words, uint32_t* due_list, uint32_t* due_prefix, const Params& P,
+                     RunRec* rec, cudaStream_t s, Timer& tm)
+{
+	ScopedKernel k(tm, "due_list");
+	k_due_list<<<StepWords::due_tiles(P.n), TILE_THREADS, 0, s>>>(due, StepWords(words, P.n).due, due_list, due_prefix,
+	                                                             P, rec);
+}
+
+// Topology from the sorted keys: cell numbering, extents and children.
+void launch_cells(const uint64_t* keys, TreeDev& T, const Params& P, RunRec* rec, uint32_t* words, cudaStream_t s,
+                  Timer& tm)
 {
 	const uint32_t n = P.n_tree, L = P.leaf_size;
 	const uint32_t n_pairs = n - L;  // n_tree > L is checked at creation
-	cudaMemsetAsync(&rec->n_overflow, 0, sizeof(unsigned int), s);
 	{
-		ScopedKernel k(tm, "tree_pairs");
-		k_pairs<<<blocks_for(n - 1, 256), 256, 0, s>>>(keys, src64, n, n_pairs, L, (int)P.max_level, T.lvl8,
-		                                               T.cnt, rec);
+		ScopedKernel k(tm, "tree_cells", 2);
+		uint32_t* counts = StepWords(words, P.n).cell;
+		const uint32_t nb = StepWords::cell_tiles(n_pairs);
+		k_cell_count<<<nb, TILE_THREADS, 0, s>>>(keys, n_pairs, L, (int)P.max_level, counts, rec);
+		k_cell_number<<<nb, TILE_THREADS, 0, s>>>(keys, n_pairs, L, (int)P.max_level, counts, T, rec);
 	}
-	scan_exclusive(T.cnt, T.base, n_pairs, block_sums, &rec->n_nodes, s, tm);
-	{
-		ScopedKernel k(tm, "tree_fill");
-		k_fill_nodes<<<blocks_for(n_pairs, 256), 256, 0, s>>>(T.lvl8, T.base, n_pairs, T, rec);
+	ScopedKernel k(tm, "tree_finish");
+	k_finish_nodes<<<blocks_for(n, 256), 256, 0, s>>>(keys, n, L, T.lvl8, T.base, T, P, rec);
+}
+
+// Fast form: prefix sums of the moments over the reordered particles.
+void launch_mom_sums(TreeDev& T, const double4* src64, const Params& P, cudaStream_t s, Timer& tm)
+{
+	if (P.form != POT_FORM_FAST) return;
+	const uint32_t n = P.n_tree, nb = (uint32_t)((n + MOM_TILE - 1) / MOM_TILE);
+	ScopedKernel k(tm, "moment_sums", T.mom_pre_d ? 4 : 2);
+	Mom5* bs = reinterpret_cast<Mom5*>(T.mom_blk);
+	k_mom_reduce<0><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs);
+	k_mom_down<0><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs, reinterpret_cast<Mom5*>(T.mom_pre));
+	if (T.mom_pre_d) {  // DIPOLES: prefix sums of q x as well
+		Mom5* bs_d = reinterpret_cast<Mom5*>(T.mom_blk_d);
+		k_mom_reduce<1><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs_d);
+		k_mom_down<1><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs_d, reinterpret_cast<Mom5*>(T.mom_pre_d));
 	}
-	{
-		ScopedKernel k(tm, "tree_finish");
-		k_finish_nodes<<<blocks_for(n, 256), 256, 0, s>>>(keys, n, L, T.lvl8, T.base, T, P, rec);
-	}
-	{
-		const bool prefix = P.form == POT_FORM_FAST;
-		const bool dip = prefix && T.mom_pre_d;
-		ScopedKernel k(tm, "tree_moments", prefix ? (dip ? 7 : 4) : 1);
-		if (prefix) {
-			const uint32_t nb = (uint32_t)((n + MOM_TILE - 1) / MOM_TILE);
-			Mom5* pre = reinterpret_cast<Mom5*>(T.mom_pre);
-			Mom5* bs = reinterpret_cast<Mom5*>(T.mom_blk);
-			k_mom_reduce<0><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs);
-			k_mom_top<<<1, MOM_THREADS, 0, s>>>(bs, nb);
-			k_mom_down<0><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs, pre);
-			Mom5* pre_d = nullptr;
-			if (dip) {  // DIPOLES: prefix sums of q x as well
-				pre_d = reinterpret_cast<Mom5*>(T.mom_pre_d);
-				Mom5* bs_d = reinterpret_cast<Mom5*>(T.mom_blk_d);
-				k_mom_reduce<1><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs_d);
-				k_mom_top<<<1, MOM_THREADS, 0, s>>>(bs_d, nb);
-				k_mom_down<1><<<nb, MOM_THREADS, 0, s>>>(src64, n, P.rad, bs_d, pre_d);
-			}
-			k_moments_prefix<<<mom_cell_blocks(n, L), 256, 0, s>>>(T, pre, pre_d, P, rec);
-		} else {
-			k_moments<<<blocks_for(n, 256), 256, 0, s>>>(T, src64, P, rec);
-		}
+}
+
+// The cells' moments, from the prefix sums (fast form) or bottom-up.
+void launch_moments(TreeDev& T, const double4* src64, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm)
+{
+	const uint32_t n = P.n_tree;
+	ScopedKernel k(tm, "tree_moments");
+	if (P.form == POT_FORM_FAST) {
+		k_moments_prefix<<<mom_cell_blocks(n, P.leaf_size), 256, 0, s>>>(
+			T, reinterpret_cast<const Mom5*>(T.mom_pre), reinterpret_cast<const Mom5*>(T.mom_pre_d), P, rec);
+	} else {
+		k_moments<<<blocks_for(n, 256), 256, 0, s>>>(T, src64, P, rec);
 	}
 }
 
@@ -924,37 +1089,45 @@ void launch_build(const uint64_t* keys, TreeDev& T, const double4* src64, const 
 // ---------------------------------------------------------------------------
 namespace pot {
 
-__global__ void kp_keys(PackDev B, int k)
+__global__ void __launch_bounds__(256) kp_keys(PackDev B, int k)
 {
 	const SegBlock sb = seg_block(B.pre[PS_KEYS], B.M);
 	const MemberView& v = B.mv[sb.m];
-	keys_body(GridSeg { sb.id, sb.n }, v.pos[pack_in(v, k)], v.keys[0], v.vals[0], v.P, v.rec, 1,
-	          v.counts + (size_t)OS_MAX_PASSES * v.tiles * RS_BINS, (int)v.P.key_bits, (int)B.npass);
+	const StepWords W(v.words, v.P.n);
+	keys_body(GridSeg { sb.id, sb.n }, v.pos[pack_in(v, k)], v.keys[0], v.vals[0], v.P, v.rec, 1, W.hist, W.keys_ctr,
+	          (int)v.P.key_bits, (int)B.npass);
 }
 
-__global__ void kp_reorder(PackDev B, int k)
+__global__ void __launch_bounds__(REORDER_THREADS) kp_reorder(PackDev B, int k)
 {
 	const SegBlock sb = seg_block(B.pre[PS_N256], B.M);
 	const MemberView& v = B.mv[sb.m];
 	const uint32_t a = pack_in(v, k), b = pack_out(v, k);
-	reorder_body(GridSeg { sb.id, sb.n }, v.vals[v.kb], v.pos[a], v.vel[a], v.pid[a], v.pos[b], v.vel[b], v.pid[b],
-	             v.src64, v.src32, v.due, v.P, v.rec, v.due_tiles);
+	reorder_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.vals[v.kb], v.pos[a], v.vel[a], v.pid[a], v.pos[b], v.vel[b],
+	             v.pid[b], v.src64, v.src32, v.due, StepWords(v.words, v.P.n).due, v.P, v.rec);
 }
 
-__global__ void kp_pairs(PackDev B)
+__global__ void __launch_bounds__(TILE_THREADS) kp_due_list(PackDev B)
 {
-	const SegBlock sb = seg_block(B.pre[PS_PAIRS], B.M);
+	const SegBlock sb = seg_block(B.pre[PS_DUE], B.M);
 	const MemberView& v = B.mv[sb.m];
-	const uint32_t n = v.P.n_tree, L = v.P.leaf_size;
-	pairs_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.src64, n, n - L, L, (int)v.P.max_level, v.T.lvl8, v.T.cnt,
-	           v.rec);
+	due_list_body(GridSeg { sb.id, sb.n }, v.due, StepWords(v.words, v.P.n).due, v.due_list, v.due_prefix, v.P, v.rec);
 }
 
-__global__ void kp_fill_nodes(PackDev B)
+__global__ void __launch_bounds__(TILE_THREADS) kp_cell_count(PackDev B)
 {
-	const SegBlock sb = seg_block(B.pre[PS_FILL], B.M);
+	const SegBlock sb = seg_block(B.pre[PS_CELLS], B.M);
 	const MemberView& v = B.mv[sb.m];
-	fill_nodes_body(GridSeg { sb.id, sb.n }, v.T.lvl8, v.T.base, v.P.n_tree - v.P.leaf_size, v.T, v.rec);
+	cell_count_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.P.n_tree - v.P.leaf_size, v.P.leaf_size,
+	                (int)v.P.max_level, StepWords(v.words, v.P.n).cell, v.rec);
+}
+
+__global__ void __launch_bounds__(TILE_THREADS) kp_cell_number(PackDev B)
+{
+	const SegBlock sb = seg_block(B.pre[PS_CELLS], B.M);
+	const MemberView& v = B.mv[sb.m];
+	cell_number_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.P.n_tree - v.P.leaf_size, v.P.leaf_size,
+	                 (int)v.P.max_level, StepWords(v.words, v.P.n).cell, v.T, v.rec);
 }
 
 __global__ void kp_finish_nodes(PackDev B)
@@ -970,14 +1143,6 @@ __global__ void __launch_bounds__(MOM_THREADS) kp_mom_reduce(PackDev B)
 	const SegBlock sb = seg_block(B.pre[PS_MOM], B.M);
 	const MemberView& v = B.mv[sb.m];
 	mom_reduce_body<0>(GridSeg { sb.id, sb.n }, v.src64, v.P.n_tree, v.P.rad, reinterpret_cast<Mom5*>(v.T.mom_blk));
-}
-
-__global__ void __launch_bounds__(MOM_THREADS) kp_mom_top(PackDev B)
-{
-	const SegBlock sb = seg_block(B.pre[PS_ONE], B.M);
-	const MemberView& v = B.mv[sb.m];
-	const uint32_t nb = (v.P.n_tree + MOM_TILE - 1) / MOM_TILE;
-	mom_top_body(GridSeg { sb.id, sb.n }, reinterpret_cast<Mom5*>(v.T.mom_blk), nb);
 }
 
 __global__ void __launch_bounds__(MOM_THREADS) kp_mom_down(PackDev B)
@@ -1005,19 +1170,29 @@ void pack_keys(const PackDev& B, int k, cudaStream_t s)
 
 void pack_reorder(const PackDev& B, int k, cudaStream_t s)
 {
-	kp_reorder<<<B.blocks[PS_N256], 256, 0, s>>>(B, k);
+	kp_reorder<<<B.blocks[PS_N256], REORDER_THREADS, 0, s>>>(B, k);
 }
 
-// Octree and fast-form moments of every member (launch_build's sequence).
-void pack_build(const PackDev& B, cudaStream_t s)
+void pack_due_list(const PackDev& B, cudaStream_t s)
 {
-	kp_pairs<<<B.blocks[PS_PAIRS], 256, 0, s>>>(B);
-	pack_node_scan(B, s);
-	kp_fill_nodes<<<B.blocks[PS_FILL], 256, 0, s>>>(B);
+	kp_due_list<<<B.blocks[PS_DUE], TILE_THREADS, 0, s>>>(B);
+}
+
+void pack_cells(const PackDev& B, cudaStream_t s)
+{
+	kp_cell_count<<<B.blocks[PS_CELLS], TILE_THREADS, 0, s>>>(B);
+	kp_cell_number<<<B.blocks[PS_CELLS], TILE_THREADS, 0, s>>>(B);
 	kp_finish_nodes<<<B.blocks[PS_FINISH], 256, 0, s>>>(B);
+}
+
+void pack_mom_sums(const PackDev& B, cudaStream_t s)
+{
 	kp_mom_reduce<<<B.blocks[PS_MOM], MOM_THREADS, 0, s>>>(B);
-	kp_mom_top<<<B.blocks[PS_ONE], MOM_THREADS, 0, s>>>(B);
 	kp_mom_down<<<B.blocks[PS_MOM], MOM_THREADS, 0, s>>>(B);
+}
+
+void pack_moments(const PackDev& B, cudaStream_t s)
+{
 	kp_moments_prefix<<<B.blocks[PS_MOMPRE], 256, 0, s>>>(B);
 }
 

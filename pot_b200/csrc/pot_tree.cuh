@@ -25,8 +25,7 @@ struct __align__(32) NodeRec {
 struct TreeDev {
 	uint32_t cap;
 	int8_t* lvl8;      // [n] common levels of pair (i, i + L), capped at 20
-	uint32_t* cnt;     // [n] cells owned by pair i
-	uint32_t* base;    // [n] exclusive scan of cnt: index of pair i's first cell
+	uint32_t* base;    // [n] index of pair i's first cell (prefix of the cells owned)
 	uint32_t* first;   // first particle (Morton slot)
 	uint32_t* last;    // last particle
 	uint8_t* level;    // depth (root 0)
@@ -72,18 +71,14 @@ struct MemberView {
 	float4* src32;
 	uint64_t* keys[2];
 	uint32_t* vals[2];
-	uint32_t* counts;      // radix-sort status words, histograms and tile counters
-	uint32_t* block_sums;  // scan block sums
+	uint32_t* words;       // the step's cleared words (StepWords)
 	uint8_t* due;
-	uint32_t* due_tiles;   // due flags per scan tile, counted by the reorder
 	uint32_t* due_list;
 	uint32_t* due_prefix;
 	uint2* groups;
 	uint32_t* rein_list;
 	uint32_t cur;
 	uint32_t kb;
-	uint32_t tiles;        // radix-sort tiles
-	uint32_t pad;
 };
 
 // A packed batch's step: each kernel of the step is one launch over every
@@ -92,21 +87,18 @@ struct MemberView {
 // entries), blocks[stage] its total.  Stages:
 //   PS_KEYS    keys_blocks(n): keys and the sort's digit counts
 //   PS_N256    blocks_for(n, 256): reorder
-//   PS_TILES   the sort's tiles: clearing the status words, each pass
-//   PS_CMP     scan tiles over n: the due list
-//   PS_PAIRS   blocks_for(n_tree - 1, 256)
-//   PS_NODES   scan tiles over the n_tree - L key pairs: cell numbering
-//   PS_FILL    blocks_for(n_tree - L, 256)
+//   PS_DUE     due_tiles(n): due list
+//   PS_TILES   the sort's tiles: clearing the step's words, each pass
+//   PS_CELLS   cell_tiles(n_tree - L): cell numbering
 //   PS_FINISH  blocks_for(n_tree, 256)
 //   PS_MOM     moment tiles over n_tree: prefix sums
 //   PS_MOMPRE  mom_cell_blocks(n_tree, leaf size): cell moments from the sums
 //   PS_GROUPS  target groups
-//   PS_ONE     one block per member: digit offsets, scan tops, chi_b, grain
-//   PS_SMALL   4-148 blocks per member (one per 8,192 particles): late
-//              absorption, reinjection (one warp per reinjected particle)
+//   PS_ONE     one block per member: chi_b
+//   PS_SMALL   4-148 blocks per member (one per 8,192 particles): the step's
+//              end (one warp per reinjected particle)
 enum PackStage : int {
-	PS_KEYS, PS_N256, PS_TILES, PS_CMP, PS_PAIRS, PS_NODES, PS_FILL, PS_FINISH, PS_MOM, PS_MOMPRE, PS_GROUPS,
-	PS_ONE, PS_SMALL, PS_COUNT
+	PS_KEYS, PS_N256, PS_DUE, PS_TILES, PS_CELLS, PS_FINISH, PS_MOM, PS_MOMPRE, PS_GROUPS, PS_ONE, PS_SMALL, PS_COUNT
 };
 struct PackDev {
 	const MemberView* mv;           // [M], device
@@ -128,29 +120,69 @@ void pack_sort_begin(const PackDev& B, cudaStream_t s);
 void pack_keys(const PackDev& B, int k, cudaStream_t s);
 void pack_sort(const PackDev& B, cudaStream_t s);
 void pack_reorder(const PackDev& B, int k, cudaStream_t s);
-void pack_build(const PackDev& B, cudaStream_t s);
-void pack_compact(const PackDev& B, cudaStream_t s);
-void pack_node_scan(const PackDev& B, cudaStream_t s);
+void pack_due_list(const PackDev& B, cudaStream_t s);
+void pack_cells(const PackDev& B, cudaStream_t s);
+void pack_mom_sums(const PackDev& B, cudaStream_t s);
+void pack_moments(const PackDev& B, cudaStream_t s);
 void pack_groups(const PackDev& B, cudaStream_t s);
 void pack_chi_b(const PackDev& B, cudaStream_t s);
 void pack_push(const PackDev& B, int k, uint32_t tpl, cudaStream_t s);
-void pack_absorb_late(const PackDev& B, int k, cudaStream_t s);
-void pack_reinject(const PackDev& B, int k, cudaStream_t s);
-void pack_grain_end(const PackDev& B, int k, cudaStream_t s);
+void pack_finish_step(const PackDev& B, int k, cudaStream_t s);
 constexpr uint32_t PACK_MOM_TILE = 256 * 16;  // moment prefix-sum tile (tree.cu MOM_TILE)
-uint32_t pack_scan_blocks(uint32_t n);        // scan tiles over n items
 
 uint32_t mom_cell_blocks(size_t n, uint32_t leaf);
 size_t mom_prefix_entries(size_t n);
 size_t mom_block_entries(size_t n);
 void launch_keys(const double4* pos, uint64_t* keys, uint32_t* vals, const Params& P, RunRec* rec,
-                 int begin_step, uint32_t* hist, cudaStream_t s, Timer& tm);
+                 int begin_step, uint32_t* words, cudaStream_t s, Timer& tm);
 uint32_t keys_blocks(size_t n);
-void launch_reorder(const uint32_t* perm, const double4* pos_in, const double4* vel_in, const uint32_t* pid_in,
-                    double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64, float4* src32,
-                    uint8_t* due, const Params& P, RunRec* rec, uint32_t* due_tiles, cudaStream_t s, Timer& tm);
-void launch_build(const uint64_t* keys, TreeDev& T, const double4* src64, const Params& P, RunRec* rec,
-                  uint32_t* block_sums, cudaStream_t s, Timer& tm);
+void launch_reorder(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, const double4* vel_in,
+                    const uint32_t* pid_in, double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64,
+                    float4* src32, uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s,
+                    Timer& tm);
+void launch_due_list(const uint8_t* due, uint32_t* words, uint32_t* due_list, uint32_t* due_prefix, const Params& P,
+                     RunRec* rec, cudaStream_t s, Timer& tm);
+void launch_cells(const uint64_t* keys, TreeDev& T, const Params& P, RunRec* rec, uint32_t* words, cudaStream_t s,
+                  Timer& tm);
+void launch_mom_sums(TreeDev& T, const double4* src64, const Params& P, cudaStream_t s, Timer& tm);
+void launch_moments(TreeDev& T, const double4* src64, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
+
+// ---- branches of a step --------------------------------------------------
+// A captured step runs on three streams: while the main one reorders the
+// state and sums its moments, the second builds the tree's topology from the
+// sorted keys (and later measures chi_b beside the walk) and the third lists
+// the due particles and makes the target groups.  Without side streams the
+// same launches follow each other on the main one.
+struct StepStreams {
+	cudaStream_t main = nullptr, side[2] = { nullptr, nullptr };
+	cudaEvent_t ev[6] = {};
+	bool forked = false;
+	cudaStream_t tree() const { return forked ? side[0] : main; }
+	cudaStream_t list() const { return forked ? side[1] : main; }
+	// what `to` enqueues next waits for what `from` holds now
+	void order(int e, cudaStream_t from, cudaStream_t to) const
+	{
+		if (from == to) return;
+		cudaEventRecord(ev[e], from);
+		cudaStreamWaitEvent(to, ev[e], 0);
+	}
+	bool create()  // side streams and events, once
+	{
+		if (side[0]) return true;
+		for (auto& e : ev)
+			if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
+		if (!side[1] && cudaStreamCreateWithFlags(&side[1], cudaStreamNonBlocking) != cudaSuccess) return false;
+		return cudaStreamCreateWithFlags(&side[0], cudaStreamNonBlocking) == cudaSuccess;
+	}
+	void destroy()
+	{
+		for (auto& e : ev)
+			if (e) cudaEventDestroy(e);
+		for (auto& s : side)
+			if (s) cudaStreamDestroy(s);
+		*this = StepStreams();
+	}
+};
 
 // walk.cu
 size_t macro_scratch_doubles();
@@ -179,10 +211,6 @@ void launch_push(double4* pos, double4* vel, const TreeDev& T, const double4* sr
 uint32_t group_blocks();
 void launch_groups(const TreeDev& T, const uint32_t* dpre, uint2* groups, uint8_t* gcell, uint32_t* gblk,
                    const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
-void launch_absorb_late(double4* pos, double4* vel, const double4* src64, const uint32_t* due_list,
-                        uint32_t* rein_list, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
-void launch_grain_end(double4* pos, double4* vel, StepHist* hist, const Params& P, RunRec* rec, int epe,
-                      cudaStream_t s, Timer& tm);
 void launch_epe(const double4* pos, const TreeDev& T, const double4* src64, const float4* src32, uint2* groups_all,
                 double* partial, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
 void launch_field_query(const TreeDev& T, const double4* src64, const float4* src32, const double* xyz,
@@ -192,8 +220,9 @@ void launch_phi_query(const TreeDev& T, const double4* src64, const double* xyz,
                       const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
 
 // inject.cu
-void launch_reinject(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* rein_list,
-                     const double4* src64, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
+void launch_finish_step(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* due_list, uint32_t* rein_list,
+                        const double4* src64, StepHist* hist, const Params& P, RunRec* rec, int epe, cudaStream_t s,
+                        Timer& tm);
 void launch_init(double4* pos, double4* vel, uint32_t* pid, const Params& P, RunRec* rec, cudaStream_t s,
                  Timer& tm);
 

@@ -1269,7 +1269,6 @@ uint32_t group_blocks() { return (uint32_t)sm_count_fast() * 4u; }
 void launch_groups(const TreeDev& T, const uint32_t* dpre, uint2* groups, uint8_t* gcell, uint32_t* gblk,
                    const Params& P, RunRec* rec, cudaStream_t s, Timer& tm)
 {
-	cudaMemsetAsync(&rec->n_groups, 0, sizeof(unsigned int), s);
 	if (!gcell) {  // one launch, groups in the order their cells finish
 		ScopedKernel k(tm, "groups");
 		k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, dpre, groups, &rec->n_groups, P.group_max, P, rec);
@@ -1354,8 +1353,6 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_epe_fast(const double4* __res
 void launch_epe_fast(const double4* pos, const TreeDev& T, const float4* src32, const double4* src64,
                      uint2* groups_all, double* partial, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm)
 {
-	cudaMemsetAsync(&rec->n_groups_all, 0, sizeof(unsigned int), s);
-	cudaMemsetAsync(&rec->work_ctr2, 0, sizeof(unsigned int), s);
 	ScopedKernel k(tm, "epe_fast", 2);
 	const bool two = P.group_max > 32;
 	k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, nullptr, groups_all, &rec->n_groups_all, two ? 64u : 32u, P,
