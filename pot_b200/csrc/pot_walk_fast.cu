@@ -44,6 +44,16 @@ static_assert(GROUP_MAX == 32 * FW_TPL_MAX, "one group per warp, at most FW_TPL_
 // registers, spilling), 4.51 against 4.65 ms per step on the 4m plasma.  One
 // target per lane fits 96 registers, and five blocks hide more latency.
 constexpr int fw_push_blocks(int tpl) { return tpl == 2 ? 4 : 5; }
+// Pairs of warps take runs of few groups: N at most this many times the
+// largest group (about 20 targets a group of 32, half the particles due, so
+// some 2,400 groups for the 2,960 warps of a launch).  One warp a group then
+// leaves schedulers idle and the step waits for the slowest group; with more
+// groups than warps a pair's barriers only cost.  Walk per step, one warp and
+// a pair: 8,193 particles 104 and 59 us, 16,001 95 and 60, 64,001 149 and 96,
+// 150,001 157 and 166, 1,000,001 712 and 926.  Four blocks per SM: at five
+// (96 registers, 112 bytes of spills) 65, 63, 102 and 171 us.
+constexpr uint32_t PAIR_MAX_N_PER_TARGET = 3200;
+constexpr int PAIR_BLOCKS = 4;
 
 // Per-warp shared memory.  A staged source (accepted cell or gathered
 // particle) takes TPL float4s: with one target per lane it is (x, y, z, q);
@@ -424,331 +434,441 @@ __device__ __forceinline__ void load_rec(const NodeRec* r, float4& c, float& r2,
 // the lanes are split instead: lane l holds member l mod 32/split and
 // evaluates the staged entries with index = sub (mod split), sub = l div
 // 32/split; the split partial fields are added across lanes at the end.
-template <int TPL, bool POT = false, bool DIP = false>
-__device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const float4* __restrict__ src32,
-                                 const Params& P, FastSmem<TPL, DIP>& sm, uint32_t& n_eval, uint32_t& stack_max,
-                                 int& err, int split = 1, uint32_t* n_far_cells = nullptr)
-{
-	const uint32_t lane = lane_f();
-	uint32_t smin = 0xFFFFFFFFu, smax = 0u;
-#pragma unroll
-	for (int k = 0; k < TPL; k++) {
-		if (tg.valid[k] && tg.self[k] != 0xFFFFFFFFu) {
-			smin = min(smin, tg.self[k]);
-			smax = max(smax, tg.self[k]);
-		}
-	}
-#pragma unroll
-	for (int o = 16; o; o >>= 1) {
-		smin = min(smin, __shfl_xor_sync(0xffffffffu, smin, o));
-		smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-	}
-	bool seen[TPL];
-#pragma unroll
-	for (int k = 0; k < TPL; k++) seen[k] = false;
-	int maxlen = 1;
-	// bounding box of the valid targets
-	float3 bmin = make_float3(3.0e38f, 3.0e38f, 3.0e38f), bmax = make_float3(-3.0e38f, -3.0e38f, -3.0e38f);
-#pragma unroll
-	for (int k = 0; k < TPL; k++) {
-		if (tg.valid[k]) {
-			bmin = make_float3(fminf(bmin.x, tg.t[k].x), fminf(bmin.y, tg.t[k].y), fminf(bmin.z, tg.t[k].z));
-			bmax = make_float3(fmaxf(bmax.x, tg.t[k].x), fmaxf(bmax.y, tg.t[k].y), fmaxf(bmax.z, tg.t[k].z));
-		}
-	}
-#pragma unroll
-	for (int o = 16; o; o >>= 1) {
-		bmin.x = fminf(bmin.x, __shfl_xor_sync(0xffffffffu, bmin.x, o));
-		bmin.y = fminf(bmin.y, __shfl_xor_sync(0xffffffffu, bmin.y, o));
-		bmin.z = fminf(bmin.z, __shfl_xor_sync(0xffffffffu, bmin.z, o));
-		bmax.x = fmaxf(bmax.x, __shfl_xor_sync(0xffffffffu, bmax.x, o));
-		bmax.y = fmaxf(bmax.y, __shfl_xor_sync(0xffffffffu, bmax.y, o));
-		bmax.z = fmaxf(bmax.z, __shfl_xor_sync(0xffffffffu, bmax.z, o));
-	}
-	const float eps2 = fmaxf(P.soft2_f, 1e-20f);
-	const float3 bc = make_float3(0.5f * (bmin.x + bmax.x), 0.5f * (bmin.y + bmax.y), 0.5f * (bmin.z + bmax.z));
+// The walk's first half: the tree's traversal for one group.
+template <int TPL, bool POT, bool DIP>
+struct Traversal {
 	// far cells (fields of monopoles only): expanded about bc instead of staged
-	constexpr bool USE_FAR = !POT && !DIP;
-	float far2 = 3.0e38f;
+	static constexpr bool USE_FAR = !POT && !DIP;
+	float3 bmin, bmax, bc;  // the valid targets' box and its centre
+	float far2;
+	uint32_t smin, smax;
 	FarExp far;
-	if constexpr (USE_FAR) {
-		float h2 = 0.f;  // the largest squared distance of a member from bc
+	uint32_t n_far;
+	bool seen[TPL];
+	int len, maxlen, ncell, nleaf;
+
+	__device__ __forceinline__ void start(const Targets<TPL>& tg, const TreeDev& T, uint32_t* stack)
+	{
+		smin = 0xFFFFFFFFu;
+		smax = 0u;
+#pragma unroll
+		for (int k = 0; k < TPL; k++) {
+			if (tg.valid[k] && tg.self[k] != 0xFFFFFFFFu) {
+				smin = min(smin, tg.self[k]);
+				smax = max(smax, tg.self[k]);
+			}
+		}
+#pragma unroll
+		for (int o = 16; o; o >>= 1) {
+			smin = min(smin, __shfl_xor_sync(0xffffffffu, smin, o));
+			smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+		}
+#pragma unroll
+		for (int k = 0; k < TPL; k++) seen[k] = false;
+		bmin = make_float3(3.0e38f, 3.0e38f, 3.0e38f);
+		bmax = make_float3(-3.0e38f, -3.0e38f, -3.0e38f);
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
 			if (tg.valid[k]) {
-				const float dx = tg.t[k].x - bc.x, dy = tg.t[k].y - bc.y, dz = tg.t[k].z - bc.z;
-				h2 = fmaxf(h2, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+				bmin = make_float3(fminf(bmin.x, tg.t[k].x), fminf(bmin.y, tg.t[k].y), fminf(bmin.z, tg.t[k].z));
+				bmax = make_float3(fmaxf(bmax.x, tg.t[k].x), fmaxf(bmax.y, tg.t[k].y), fmaxf(bmax.z, tg.t[k].z));
 			}
 		}
 #pragma unroll
-		for (int o = 16; o; o >>= 1) h2 = fmaxf(h2, __shfl_xor_sync(0xffffffffu, h2, o));
-		far2 = (FAR_RATIO * FAR_RATIO) * h2;
-		far.zero();
+		for (int o = 16; o; o >>= 1) {
+			bmin.x = fminf(bmin.x, __shfl_xor_sync(0xffffffffu, bmin.x, o));
+			bmin.y = fminf(bmin.y, __shfl_xor_sync(0xffffffffu, bmin.y, o));
+			bmin.z = fminf(bmin.z, __shfl_xor_sync(0xffffffffu, bmin.z, o));
+			bmax.x = fmaxf(bmax.x, __shfl_xor_sync(0xffffffffu, bmax.x, o));
+			bmax.y = fmaxf(bmax.y, __shfl_xor_sync(0xffffffffu, bmax.y, o));
+			bmax.z = fmaxf(bmax.z, __shfl_xor_sync(0xffffffffu, bmax.z, o));
+		}
+		bc = make_float3(0.5f * (bmin.x + bmax.x), 0.5f * (bmin.y + bmax.y), 0.5f * (bmin.z + bmax.z));
+		if constexpr (USE_FAR) {
+			float h2 = 0.f;  // the largest squared distance of a member from bc
+#pragma unroll
+			for (int k = 0; k < TPL; k++) {
+				if (tg.valid[k]) {
+					const float dx = tg.t[k].x - bc.x, dy = tg.t[k].y - bc.y, dz = tg.t[k].z - bc.z;
+					h2 = fmaxf(h2, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+				}
+			}
+#pragma unroll
+			for (int o = 16; o; o >>= 1) h2 = fmaxf(h2, __shfl_xor_sync(0xffffffffu, h2, o));
+			far2 = (FAR_RATIO * FAR_RATIO) * h2;
+			far.zero();
+		}
+		n_far = 0;
+		len = maxlen = 1;
+		ncell = nleaf = 0;
+		if (lane_f() == 0) stack[0] = 8u * T.cap;  // the root's record
+		__syncwarp();
 	}
-	const int sub = (int)lane / (32 / split);  // this lane's share of each staged list
-	// Evaluation is FP32x2 in both forms.  Two targets per lane: each pair is
-	// the lane's two targets against one duplicated source.  One target per
-	// lane: each pair is two sources (packed by pair_pack at the flush)
-	// against the duplicated target, and the two halves are added at the end.
+
+	// One round: up to 32 nodes off the stack, tested one a lane; accepted
+	// cells are added to `cells` (dipoles FW_CELLS entries beyond), opened
+	// leaves to `leaves`, opened cells' children to the stack.  Returns whether
+	// the stack had room.
+	__device__ __forceinline__ bool round(const Targets<TPL>& tg, const TreeDev& T, const Params& P, uint32_t* stack,
+	                                      float4* cells, uint2* leaves)
+	{
+		const uint32_t lane = lane_f();
+		Acc<TPL>* tag = nullptr;  // selects the staging layout
+		const int take = len < 32 ? len : 32;
+		const uint32_t node = (int)lane < take ? stack[len - 1 - (int)lane] : NONE;
+		__syncwarp();
+		len -= take;
+		bool acc = false, leafr = false;
+		float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
+		float4 dipole = make_float4(0.f, 0.f, 0.f, 0.f);
+		uint2 range = make_uint2(0u, 0u);
+		uint32_t kids = 0u, base = 0u;  // an opened cell's children: mask, first record
+		if (node != NONE) {
+			uint32_t info;
+			float r2;
+			load_rec(&T.nrec[node], cell, r2, base, info);
+			if (DIP) dipole = T.drec[node];
+			const bool leaf = (info & NR_LEAF) != 0u;
+			if (!(info & NR_UNTESTED) && group_accepts(bmin, bmax, bc, cell, r2, P.oap2_f)) {
+				acc = cell.w != 0.f || (DIP && (dipole.x != 0.f || dipole.y != 0.f || dipole.z != 0.f));
+				if (USE_FAR && acc) {
+					const float fx = bc.x - cell.x, fy = bc.y - cell.y, fz = bc.z - cell.z;
+					if (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) > far2) {
+						far.add(bc, cell);
+						acc = false;
+						n_far++;
+					}
+				}
+			} else if (leaf) {
+				leafr = true;
+				range = make_uint2(base, info & NR_COUNT);
+			} else {
+				kids = info;
+			}
+		}
+		const int nch = __popc(kids);
+		leafr = leafr && range.y > 0u;  // the leaf flush relies on no staged leaf being empty
+		// one warp scan for the three appends: accepted cells in bits 0-9,
+		// leaf ranges in bits 10-19, children in bits 20-31 (totals <= 32,
+		// <= 32 and <= 256 fit)
+		int tot;
+		const int packed = (acc ? 1 : 0) | ((leafr ? 1 : 0) << 10) | (nch << 20);
+		const int off = warp_excl(packed, tot);
+		const int co = off & 0x3FF, lo = (off >> 10) & 0x3FF, po = off >> 20;
+		const int tcell = tot & 0x3FF, tleaf = (tot >> 10) & 0x3FF, tch = tot >> 20;
+		if (acc) stage_src(cells, ncell + co, cell, tag);
+		if (DIP && acc) cells[FW_CELLS + ncell + co] = dipole;
+		ncell += tcell;
+		if (leafr) leaves[nleaf + lo] = range;
+		nleaf += tleaf;
+		// opened leaves that may hold members' own particles
+		unsigned int hits = __ballot_sync(0xffffffffu, leafr && range.x <= smax && range.x + range.y > smin);
+		while (hits) {
+			const int b = __ffs(hits) - 1;
+			hits &= hits - 1;
+			const uint32_t rx = __shfl_sync(0xffffffffu, range.x, b);
+			const uint32_t ry = __shfl_sync(0xffffffffu, range.y, b);
+#pragma unroll
+			for (int k = 0; k < TPL; k++) seen[k] = seen[k] || (tg.self[k] - rx < ry);
+		}
+		if (len + tch > FW_STACK) return false;
+		int w = len + po;
+#pragma unroll
+		for (uint32_t d = 0; d < 8; d++)
+			if (kids & (1u << d)) stack[w++] = base + d;
+		len += tch;
+		maxlen = max(maxlen, len);
+		__syncwarp();
+		return true;
+	}
+};
+
+// The walk's second half: the staged lists' evaluation for the lanes' targets.
+// Evaluation is FP32x2 in both forms.  Two targets per lane: each pair is the
+// lane's two targets against one duplicated source.  One target per lane:
+// each pair is two sources (packed by pair_pack at the flush) against the
+// duplicated target, and the two halves are added at the end.
+template <int TPL, bool POT, bool DIP>
+struct Evaluation {
+	static constexpr int PER_EV = TPL == 1 ? 2 : 1;  // staged sources per evaluation
 	TgtE<2> te;
 	Acc<2> E;
-	if constexpr (TPL == 1) {
-		te.x = make_float2(tg.t[0].x, tg.t[0].x);
-		te.y = make_float2(tg.t[0].y, tg.t[0].y);
-		te.z = make_float2(tg.t[0].z, tg.t[0].z);
-		E.x = E.y = E.z = make_float2(0.f, 0.f);
-	} else {
-		to_eval(tg, te, E);
+	int split, sub;  // the lane's share of each staged list
+
+	// Cells are evaluated in whole units of the unrolled loop: 8 evaluations
+	// per lane, or 4 for a split list of pairs (so that the padded list fits
+	// the cell buffer); at most 32, so that padding is one store per lane.
+	__device__ __forceinline__ static int unit_of(int split)
+	{
+		return ((TPL == 1 && split > 1) ? 4 : 8) * PER_EV * split;
 	}
-	Acc<TPL>* tag = nullptr;  // selects the staging layout
-	// staged sources per evaluation (a pair of sources with one target per lane)
-	constexpr int PER_EV = TPL == 1 ? 2 : 1;
-	// cell evaluations unrolled per lane: 8, or 4 for a split list of pairs
-	// (so that the padded list fits the cell buffer)
-	const int cell_unroll = (TPL == 1 && split > 1) ? 4 : 8;
-	int len = 1, ncell = 0, nleaf = 0;
-	uint32_t n_cells_ev = 0, n_parts_ev = 0, n_far = 0;
-	if (lane == 0) sm.stack[0] = 8u * T.cap;  // the root's record
-	__syncwarp();
-	for (;;) {
-		const bool done = (len == 0);
-		if (!done) {
-			const int take = len < 32 ? len : 32;
-			const uint32_t node = (int)lane < take ? sm.stack[len - 1 - (int)lane] : NONE;
-			__syncwarp();
-			len -= take;
-			bool acc = false, leafr = false;
-			float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
-			float4 dipole = make_float4(0.f, 0.f, 0.f, 0.f);
-			uint2 range = make_uint2(0u, 0u);
-			uint32_t kids = 0u, base = 0u;  // an opened cell's children: mask, first record
-			if (node != NONE) {
-				uint32_t info;
-				float r2;
-				load_rec(&T.nrec[node], cell, r2, base, info);
-				if (DIP) dipole = T.drec[node];
-				const bool leaf = (info & NR_LEAF) != 0u;
-				if (!(info & NR_UNTESTED) && group_accepts(bmin, bmax, bc, cell, r2, P.oap2_f)) {
-					acc = cell.w != 0.f || (DIP && (dipole.x != 0.f || dipole.y != 0.f || dipole.z != 0.f));
-					if (USE_FAR && acc) {
-						const float fx = bc.x - cell.x, fy = bc.y - cell.y, fz = bc.z - cell.z;
-						if (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) > far2) {
-							far.add(bc, cell);
-							acc = false;
-							n_far++;
-						}
-					}
-				} else if (leaf) {
-					leafr = true;
-					range = make_uint2(base, info & NR_COUNT);
-				} else {
-					kids = info;
-				}
+
+	__device__ __forceinline__ void start(const Targets<TPL>& tg, int split_)
+	{
+		split = TPL == 2 ? 1 : split_;
+		sub = (int)lane_f() / (32 / split);
+		if constexpr (TPL == 1) {
+			te.x = make_float2(tg.t[0].x, tg.t[0].x);
+			te.y = make_float2(tg.t[0].y, tg.t[0].y);
+			te.z = make_float2(tg.t[0].z, tg.t[0].z);
+			E.x = E.y = E.z = make_float2(0.f, 0.f);
+		} else {
+			to_eval(tg, te, E);
+		}
+	}
+
+	// the first n staged cells, whole units
+	__device__ __forceinline__ void cells(float4* buf, int n)
+	{
+		if (TPL == 1) {
+			for (int p = (int)lane_f(); p < n / 2; p += 32) {
+				pair_pack(buf, p);
+				if (DIP) pair_pack_dip(buf + FW_CELLS, p);
 			}
-			const int nch = __popc(kids);
-			leafr = leafr && range.y > 0u;  // the leaf flush relies on no staged leaf being empty
-			// one warp scan for the three appends: accepted cells in bits 0-9,
-			// leaf ranges in bits 10-19, children in bits 20-31 (totals <= 32,
-			// <= 32 and <= 256 fit)
-			int tot;
-			const int packed = (acc ? 1 : 0) | ((leafr ? 1 : 0) << 10) | (nch << 20);
-			const int off = warp_excl(packed, tot);
-			const int co = off & 0x3FF, lo = (off >> 10) & 0x3FF, po = off >> 20;
-			const int tcell = tot & 0x3FF, tleaf = (tot >> 10) & 0x3FF, tch = tot >> 20;
-			if (acc) stage_src(sm.cells, ncell + co, cell, tag);
-			if (DIP && acc) sm.cells[FW_CELLS + ncell + co] = dipole;
-			ncell += tcell;
-			if (leafr) sm.leaves[nleaf + lo] = range;
-			nleaf += tleaf;
-			// opened leaves that may hold members' own particles
-			unsigned int hits = __ballot_sync(0xffffffffu, leafr && range.x <= smax && range.x + range.y > smin);
-			while (hits) {
-				const int b = __ffs(hits) - 1;
-				hits &= hits - 1;
-				const uint32_t rx = __shfl_sync(0xffffffffu, range.x, b);
-				const uint32_t ry = __shfl_sync(0xffffffffu, range.y, b);
-#pragma unroll
-				for (int k = 0; k < TPL; k++) seen[k] = seen[k] || (tg.self[k] - rx < ry);
-			}
-			if (len + tch > FW_STACK) {
-				err = POT_E_WALK;
-				break;
-			}
-			int w = len + po;
-#pragma unroll
-			for (uint32_t d = 0; d < 8; d++)
-				if (kids & (1u << d)) sm.stack[w++] = base + d;
-			len += tch;
-			maxlen = max(maxlen, len);
 			__syncwarp();
 		}
-		// flush staged monopoles in whole units of the unrolled loop, so it
-		// needs no remainder: a flush during the walk evaluates the whole units
-		// and carries the rest (fewer than a unit) to the next; the last one
-		// pads to a whole unit with zero-charge cells far outside the domain
-		if (ncell >= FW_CELL_FLUSH || (done && ncell > 0)) {
-			const int unit = cell_unroll * PER_EV * split;  // <= 32: the padding is one store per lane
-			const int padded = done ? (ncell + unit - 1) / unit * unit : ncell / unit * unit;
-			if (done && (int)lane < padded - ncell) {
-				stage_src(sm.cells, ncell + lane, make_float4(64.f, 64.f, 64.f, 0.f), tag);
-				if (DIP) sm.cells[FW_CELLS + ncell + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+		const int nev = n / PER_EV;
+		if (DIP) {  // one target per lane (creation checks the group size)
+			const int stride = split, per = nev / split;
+			for (int j = 0; j < per; j += 4) {
+#pragma unroll
+				for (int u = 0; u < 4; u++) eval_cell_dip<POT>(E, te, buf, buf + FW_CELLS, (j + u) * stride + sub);
 			}
+		} else if (TPL == 2 || split == 1) {
+			for (int j = 0; j < nev; j += 8) {
+#pragma unroll
+				for (int u = 0; u < 8; u++) eval_src<false, POT>(E, te, buf, j + u, 0.f);
+			}
+		} else {
+			const int per = nev / split;
+			for (int j = 0; j < per; j += 4) {
+#pragma unroll
+				for (int u = 0; u < 4; u++) eval_src<false, POT>(E, te, buf, (j + u) * split + sub, 0.f);
+			}
+		}
+	}
+
+	// nleaf staged leaves: their particles are gathered 32 at a time into
+	// shared memory (dense, by a prefix sum over the leaf sizes).  Returns the
+	// number of particles.
+	__device__ __forceinline__ uint32_t leaves(const uint2* lv, int nleaf, uint32_t* lsrc, float4* pbuf,
+	                                           const float4* __restrict__ src32, const Params& P)
+	{
+		const float eps2 = soft_of(P);
+		const uint32_t lane = lane_f();
+		Acc<TPL>* tag = nullptr;
+		const uint2 l0 = (int)lane < nleaf ? lv[lane] : make_uint2(0u, 0u);
+		const uint2 l1 = (int)lane + 32 < nleaf ? lv[lane + 32] : make_uint2(0u, 0u);
+		int t0, t1;
+		const int e0 = warp_excl((int)l0.y, t0);
+		const int e1 = warp_excl((int)l1.y, t1);
+		const uint32_t total = (uint32_t)(t0 + t1);
+		// start offsets of this lane's two staged leaves, ~0 for none, and each
+		// leaf's first slot less its start: the particle at position g of the
+		// list is in slot g + lsrc[leaf]
+		const uint32_t st0 = (int)lane < nleaf ? (uint32_t)e0 : 0xFFFFFFFFu;
+		const uint32_t st1 = (int)lane + 32 < nleaf ? (uint32_t)(t0 + e1) : 0xFFFFFFFFu;
+		lsrc[lane] = l0.x - (uint32_t)e0;
+		lsrc[lane + 32] = l1.x - (uint32_t)(t0 + e1);
+		const uint32_t le_mask = (2u << lane) - 1u;  // lanes 0..lane (all for lane 31)
+		int before = 0;  // staged leaves that start before the chunk gathered next
+		__syncwarp();
+		// the lane's particle of the chunk at `base`
+		const auto gather = [&](uint32_t base) {
+			const uint32_t g = base + lane;
+			// the staged leaves that start inside this chunk, one bit per
+			// start offset (no leaf is empty, so no two share a start)
+			uint32_t bits = 0u;
+			if (st0 - base < 32u) bits |= 1u << (st0 - base);
+			if (st1 - base < 32u) bits |= 1u << (st1 - base);
+			const uint32_t starts = __reduce_or_sync(0xffffffffu, bits);
+			// padding: zero charge far outside the domain
+			float4 p = make_float4(64.f, 64.f, 64.f, 0.f);
+			// the last leaf starting at or before g
+			if (g < total) p = __ldg(&src32[g + lsrc[before + __popc(starts & le_mask) - 1]]);
+			before += __popc(starts);
+			return p;
+		};
+		float4 p = gather(0);
+		for (uint32_t base = 0; base < total; base += 32) {
+			stage_chunk(pbuf, lane, p, tag);
 			__syncwarp();
-			if (TPL == 1) {
-				for (int p = (int)lane; p < padded / 2; p += 32) {
-					pair_pack(sm.cells, p);
-					if (DIP) pair_pack_dip(sm.cells + FW_CELLS, p);
-				}
-				__syncwarp();
-			}
-			const int nev = padded / PER_EV;
-			if (DIP) {  // one target per lane (creation checks the group size)
-				const int stride = split, per = nev / split;
-				for (int j = 0; j < per; j += 4) {
+			// the next chunk's particles are on the way while this one's are
+			// evaluated
+			if (base + 32 < total) p = gather(base + 32);
+			constexpr int nev = 32 / PER_EV;
+			const uint32_t in_chunk = total - base < 32u ? total - base : 32u;
+			if ((TPL == 2 || split == 1) && in_chunk == 32u) {
+#pragma unroll 16
+				for (int m = 0; m < nev; m++) eval_src<true, POT>(E, te, pbuf, m, eps2);
+			} else if (TPL == 2 || split == 1) {
+				// a flush's last, partial chunk: whole quads of evaluations that
+				// cover its particles (the padding beyond has zero charge)
+				const int need = TPL == 1 ? ((int)in_chunk + 1) / 2 : (int)in_chunk;
+				const int nq = (need + 3) & ~3;  // <= nev
+				for (int m = 0; m < nq; m += 4) {
 #pragma unroll
-					for (int u = 0; u < 4; u++)
-						eval_cell_dip<POT>(E, te, sm.cells, sm.cells + FW_CELLS, (j + u) * stride + sub);
-				}
-			} else if (split == 1) {
-				for (int j = 0; j < nev; j += 8) {
-#pragma unroll
-					for (int u = 0; u < 8; u++) eval_src<false, POT>(E, te, sm.cells, j + u, eps2);
+					for (int u = 0; u < 4; u++) eval_src<true, POT>(E, te, pbuf, m + u, eps2);
 				}
 			} else {
 				const int per = nev / split;
-				for (int j = 0; j < per; j += 4) {
-#pragma unroll
-					for (int u = 0; u < 4; u++) eval_src<false, POT>(E, te, sm.cells, (j + u) * split + sub, eps2);
-				}
+#pragma unroll 8
+				for (int m = 0; m < per; m++) eval_src<true, POT>(E, te, pbuf, m * split + sub, eps2);
 			}
-			// carried cells (unpacked, fewer than 32) move to the front; the
-			// ranges [padded, ncell) and [0, ncell - padded) are disjoint
-			const int rem = ncell > padded ? ncell - padded : 0;
-			n_cells_ev += ncell - rem;
-			__syncwarp();
-			if ((int)lane < rem) {
-#pragma unroll
-				for (int k = 0; k < TPL; k++) sm.cells[TPL * (int)lane + k] = sm.cells[TPL * (padded + (int)lane) + k];
-				if (DIP) sm.cells[FW_CELLS + lane] = sm.cells[FW_CELLS + padded + lane];
-			}
-			ncell = rem;
 			__syncwarp();
 		}
-		// flush staged leaves: their particles are gathered 32 at a time into
-		// shared memory (dense, by a prefix sum over the leaf sizes)
-		if (nleaf >= FW_LEAF_FLUSH || (done && nleaf > 0)) {
-			const uint2 l0 = (int)lane < nleaf ? sm.leaves[lane] : make_uint2(0u, 0u);
-			const uint2 l1 = (int)lane + 32 < nleaf ? sm.leaves[lane + 32] : make_uint2(0u, 0u);
-			int t0, t1;
-			const int e0 = warp_excl((int)l0.y, t0);
-			const int e1 = warp_excl((int)l1.y, t1);
-			const uint32_t total = (uint32_t)(t0 + t1);
-			// start offsets of this lane's two staged leaves, ~0 for none, and each
-			// leaf's first slot less its start: the particle at position g of the
-			// list is in slot g + lsrc[leaf]
-			const uint32_t st0 = (int)lane < nleaf ? (uint32_t)e0 : 0xFFFFFFFFu;
-			const uint32_t st1 = (int)lane + 32 < nleaf ? (uint32_t)(t0 + e1) : 0xFFFFFFFFu;
-			sm.lsrc[lane] = l0.x - (uint32_t)e0;
-			sm.lsrc[lane + 32] = l1.x - (uint32_t)(t0 + e1);
-			const uint32_t le_mask = (2u << lane) - 1u;  // lanes 0..lane (all for lane 31)
-			int before = 0;  // staged leaves that start before the chunk gathered next
-			__syncwarp();
-			// the lane's particle of the chunk at `base`
-			const auto gather = [&](uint32_t base) {
-				const uint32_t g = base + lane;
-				// the staged leaves that start inside this chunk, one bit per
-				// start offset (no leaf is empty, so no two share a start)
-				uint32_t bits = 0u;
-				if (st0 - base < 32u) bits |= 1u << (st0 - base);
-				if (st1 - base < 32u) bits |= 1u << (st1 - base);
-				const uint32_t starts = __reduce_or_sync(0xffffffffu, bits);
-				// padding: zero charge far outside the domain
-				float4 p = make_float4(64.f, 64.f, 64.f, 0.f);
-				// the last leaf starting at or before g
-				if (g < total) p = __ldg(&src32[g + sm.lsrc[before + __popc(starts & le_mask) - 1]]);
-				before += __popc(starts);
-				return p;
-			};
-			float4 p = gather(0);
-			for (uint32_t base = 0; base < total; base += 32) {
-				stage_chunk(sm.pbuf, lane, p, tag);
-				__syncwarp();
-				// the next chunk's particles are on the way while this one's are
-				// evaluated
-				if (base + 32 < total) p = gather(base + 32);
-				constexpr int nev = 32 / PER_EV;
-				const uint32_t in_chunk = total - base < 32u ? total - base : 32u;
-				if (split == 1 && in_chunk == 32u) {
-#pragma unroll 16
-					for (int m = 0; m < nev; m++) eval_src<true, POT>(E, te, sm.pbuf, m, eps2);
-				} else if (split == 1) {
-					// a flush's last, partial chunk: whole quads of evaluations that
-					// cover its particles (the padding beyond has zero charge)
-					const int need = TPL == 1 ? ((int)in_chunk + 1) / 2 : (int)in_chunk;
-					const int nq = (need + 3) & ~3;  // <= nev
-					for (int m = 0; m < nq; m += 4) {
-#pragma unroll
-						for (int u = 0; u < 4; u++) eval_src<true, POT>(E, te, sm.pbuf, m + u, eps2);
-					}
-				} else {
-					const int per = nev / split;
-#pragma unroll 8
-					for (int m = 0; m < per; m++) eval_src<true, POT>(E, te, sm.pbuf, m * split + sub, eps2);
-				}
-				__syncwarp();
+		return total;
+	}
+
+	__device__ __forceinline__ Field<TPL> sum()
+	{
+		if constexpr (TPL == 1) {
+			Acc<1> e1;
+			e1.x = E.x.x + E.x.y;
+			e1.y = E.y.x + E.y.y;
+			e1.z = E.z.x + E.z.y;
+			if (split > 1) {  // add the split partial fields (lanes l, l ^ 16, l ^ 8, ... share a member)
+				for (int o = 16; o >= 32 / split; o >>= 1) add_xor(e1, o);
 			}
-			n_parts_ev += total;
-			nleaf = 0;
+			return from_eval(e1);
+		} else {
+			return from_eval(E);
+		}
+	}
+
+	// the softening, floored so that a target's own term is finite
+	__device__ __forceinline__ static float soft_of(const Params& P) { return fmaxf(P.soft2_f, 1e-20f); }
+
+	// take back a member's own term, which was summed
+	__device__ __forceinline__ static void take_back(Field<TPL>& F, int k, const Targets<TPL>& tg,
+	                                                 const float4* __restrict__ src32, const Params& P)
+	{
+		Acc<1> s1;
+		TgtE<1> t1;
+		t1.x = tg.t[k].x;
+		t1.y = tg.t[k].y;
+		t1.z = tg.t[k].z;
+		s1.x = s1.y = s1.z = 0.f;
+		const float4 own = __ldg(&src32[tg.self[k]]);
+		eval_src<true, POT>(s1, t1, &own, 0, soft_of(P));
+		F.x[k] -= s1.x;
+		F.y[k] -= s1.y;
+		F.z[k] -= s1.z;
+	}
+};
+
+// Entry i of a staged cell list as padding: zero charge far outside the domain.
+template <int TPL, bool DIP>
+__device__ __forceinline__ void stage_pad(float4* cells, int i)
+{
+	Acc<TPL>* tag = nullptr;
+	stage_src(cells, i, make_float4(64.f, 64.f, 64.f, 0.f), tag);
+	if (DIP) cells[FW_CELLS + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Entries evaluated per target, deepest stack, far cells of one group.
+struct WalkStats {
+	uint32_t n_eval = 0, depth = 0, n_far = 0;
+};
+
+// The whole walk by one warp: rounds of the traversal, and flushes of the
+// staged lists: cells when 64 or more are staged (the remainder, fewer than a
+// unit, stays for the next flush; the last one is padded), leaves when 32 or
+// more are.
+template <int TPL, bool POT = false, bool DIP = false>
+__device__ Field<TPL> group_walk(const Targets<TPL>& tg, const TreeDev& T, const float4* __restrict__ src32,
+                                 const Params& P, FastSmem<TPL, DIP>& sm, WalkStats& ws, int& err, int split = 1)
+{
+	const int lane = (int)lane_f();
+	Traversal<TPL, POT, DIP> tr;
+	Evaluation<TPL, POT, DIP> ev;
+	tr.start(tg, T, sm.stack);
+	ev.start(tg, split);
+	const int unit = ev.unit_of(split);
+	for (;;) {
+		const bool done = tr.len == 0;
+		if (!done && !tr.round(tg, T, P, sm.stack, sm.cells, sm.leaves)) {
+			err = POT_E_WALK;
+			break;
+		}
+		if (tr.ncell >= FW_CELL_FLUSH || (done && tr.ncell > 0)) {
+			const int n = done ? (tr.ncell + unit - 1) / unit * unit : tr.ncell / unit * unit;
+			if (done && lane < n - tr.ncell) stage_pad<TPL, DIP>(sm.cells, tr.ncell + lane);
+			__syncwarp();
+			ev.cells(sm.cells, n);
+			// carried cells (unpacked, fewer than 32) move to the front; the
+			// ranges [n, ncell) and [0, ncell - n) are disjoint
+			const int rem = tr.ncell > n ? tr.ncell - n : 0;
+			ws.n_eval += (uint32_t)(tr.ncell - rem);
+			__syncwarp();
+			if (lane < rem) {
+#pragma unroll
+				for (int k = 0; k < TPL; k++) sm.cells[TPL * lane + k] = sm.cells[TPL * (n + lane) + k];
+				if (DIP) sm.cells[FW_CELLS + lane] = sm.cells[FW_CELLS + n + lane];
+			}
+			tr.ncell = rem;
+			__syncwarp();
+		}
+		if (tr.nleaf >= FW_LEAF_FLUSH || (done && tr.nleaf > 0)) {
+			ws.n_eval += ev.leaves(sm.leaves, tr.nleaf, sm.lsrc, sm.pbuf, src32, P);
+			tr.nleaf = 0;
 			__syncwarp();
 		}
 		if (done) break;
 	}
-	Field<TPL> F;
-	if constexpr (TPL == 1) {
-		Acc<1> e1;
-		e1.x = E.x.x + E.x.y;
-		e1.y = E.y.x + E.y.y;
-		e1.z = E.z.x + E.z.y;
-		if (split > 1) {  // add the split partial fields (lanes l, l ^ 16, l ^ 8, ... share a member)
-			for (int o = 16; o >= 32 / split; o >>= 1) add_xor(e1, o);
-		}
-		F = from_eval(e1);
-	} else {
-		F = from_eval(E);
-	}
-	if constexpr (USE_FAR) {
-		far.warp_sum();
+	ws.depth = (uint32_t)tr.maxlen;
+	for (int o = 16; o; o >>= 1) tr.n_far += __shfl_xor_sync(0xffffffffu, tr.n_far, o);
+	ws.n_far = tr.n_far;
+	Field<TPL> F = ev.sum();
+	if constexpr (Traversal<TPL, POT, DIP>::USE_FAR) {
+		tr.far.warp_sum();
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
-			const float3 e = far.at(tg.t[k].x - bc.x, tg.t[k].y - bc.y, tg.t[k].z - bc.z);
+			const float3 e = tr.far.at(tg.t[k].x - tr.bc.x, tg.t[k].y - tr.bc.y, tg.t[k].z - tr.bc.z);
 			F.x[k] += e.x;
 			F.y[k] += e.y;
 			F.z[k] += e.z;
 		}
-		// the group's far cells, each expanded once
-		for (int o = 16; o; o >>= 1) n_far += __shfl_xor_sync(0xffffffffu, n_far, o);
-		if (n_far_cells) *n_far_cells = n_far;
 	}
-	// take back the members' own terms
 #pragma unroll
-	for (int k = 0; k < TPL; k++) {
-		if (seen[k]) {
-			Acc<1> s1;
-			TgtE<1> t1;
-			t1.x = tg.t[k].x;
-			t1.y = tg.t[k].y;
-			t1.z = tg.t[k].z;
-			s1.x = s1.y = s1.z = 0.f;
-			const float4 own = __ldg(&src32[tg.self[k]]);
-			eval_src<true, POT>(s1, t1, &own, 0, eps2);
-			F.x[k] -= s1.x;
-			F.y[k] -= s1.y;
-			F.z[k] -= s1.z;
-		}
-	}
-	n_eval = n_cells_ev + n_parts_ev;
-	stack_max = (uint32_t)maxlen;
+	for (int k = 0; k < TPL; k++)
+		if (tr.seen[k]) ev.take_back(F, k, tg, src32, P);
 	return F;
+}
+
+// The push's walk by a pair of warps: one traverses, the other evaluates what
+// it staged, then pushes the group's members while the first is already in
+// the next group.  They meet at a named barrier once a stage, a stage being
+// what one flush of group_walk evaluates: the traversing warp fills stage
+// k + 1 while the other works on stage k.  Buffers are doubled and swapped
+// when a stage takes them, so neither side writes what the other reads.  The
+// stages, and so every sum, are group_walk's.
+template <int TPL, bool DIP>
+struct PairSmem {
+	uint32_t stack[FW_STACK];
+	float4 cells[2][FW_CELLS * TPL * (DIP ? 2 : 1)];
+	uint2 leaves[2][FW_LEAVES];
+	uint32_t lsrc[FW_LEAVES];
+	float4 pbuf[32 * TPL];
+	struct Stage {
+		uint32_t group;  // NONE: no more groups
+		int ncell, cells, nleaf, leaves;  // cells evaluated (padding included), real ones among them
+		int cbuf, lbuf;
+		int flags;       // 1: the group's first stage, 2: its last
+	} stage[2];
+	struct Last {        // with the group's last stage, by group parity
+		float far[15];
+		float3 bc;
+		uint32_t seen[TPL];  // bit per lane
+		uint32_t depth, n_far;
+		int err;
+	} last[2];
+};
+constexpr int ST_FIRST = 1, ST_LAST = 2;
+
+__device__ __forceinline__ void pair_barrier(int pair)
+{
+	asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
 }
 
 // Slot range [a, b) of a child code.
@@ -1053,54 +1173,53 @@ __device__ __forceinline__ PushCtx push_ctx(const double4* __restrict__ pos, con
 	return c;
 }
 
-// One target group grp = (first entry of the due list, count): the warp's
-// walk for the whole group, then each member's push, absorption and boundary
-// test.  Adds to the lane's interaction and push counts and the deepest
-// stack; returns the walk's status (a member that fails leaves the group's
-// pushes undone).
-template <int TPL, int STG, bool DIP>
-__device__ __forceinline__ int push_group(uint2 grp, double4* __restrict__ pos, double4* __restrict__ vel,
-                                          const TreeDev& T, const float4* __restrict__ src32,
-                                          const uint32_t* __restrict__ due_list, uint32_t* __restrict__ rein_list,
-                                          const Params& P, RunRec* rec, const double4* __restrict__ src64,
-                                          const StageBufs& sb, const PushCtx& pc, FastSmem<TPL, DIP>& sm,
-                                          unsigned long long& n_inter, unsigned long long& n_push,
-                                          uint32_t& stack_max, unsigned long long& n_far)
+// The lane's members of a group grp = (first entry of the due list, count).
+// Small groups split the warp (see Evaluation): lanes past the first
+// 32 / split hold copies of members and push nothing.  The FP64 evaluation
+// point (half-drifted for the Boris step) is recomputed for the push from the
+// same state with the same operations, so it is not held in registers through
+// the walk.
+__device__ __forceinline__ int split_of(int tpl, uint32_t count)
 {
-	Targets<TPL> tg;
-	uint32_t slot[TPL];
-	// small groups split the warp (see group_walk): lanes past the
-	// first 32 / split hold copies of members and push nothing
-	const int split = TPL == 1 ? (grp.y <= 8 ? 4 : (grp.y <= 16 ? 2 : 1)) : 1;
+	return tpl == 1 ? (count <= 8 ? 4 : (count <= 16 ? 2 : 1)) : 1;
+}
+
+template <int TPL, int STG>
+__device__ __forceinline__ void load_targets(uint2 grp, int split, const double4* __restrict__ pos,
+                                             const double4* __restrict__ vel, const uint32_t* __restrict__ due_list,
+                                             const Params& P, Targets<TPL>& tg)
+{
 	const uint32_t width = 32u / (uint32_t)split;
-	const bool owner = lane_f() < width;
-	// the FP64 evaluation point (half-drifted for the Boris step) is
-	// recomputed after the walk from the same state with the same
-	// operations, so it is not held in registers through the walk
 #pragma unroll
 	for (int k = 0; k < TPL; k++) {
 		const uint32_t m = (lane_f() & (width - 1u)) + 32u * k;
 		tg.valid[k] = m < grp.y;
-		slot[k] = 0xFFFFFFFFu;
+		tg.self[k] = 0xFFFFFFFFu;
 		double3 h = make_double3(P.rad, P.rad, P.rad);
 		if (tg.valid[k]) {
-			slot[k] = due_list[grp.x + m];
-			h = eval_point<STG>(pos[slot[k]], vel, slot[k], P);
+			const uint32_t s = due_list[grp.x + m];
+			tg.self[k] = s;
+			h = eval_point<STG>(pos[s], vel, s, P);
 		}
-		tg.self[k] = slot[k];
 		tg.t[k] = make_float3((float)((h.x - P.rad) * P.inv_rad), (float)((h.y - P.rad) * P.inv_rad),
 		                      (float)((h.z - P.rad) * P.inv_rad));
 	}
-	uint32_t ne = 0, depth = 0, nf = 0;
-	int err = POT_OK;
-	const Field<TPL> ef = group_walk<TPL, false, DIP>(tg, T, pc.srcf, P, sm, ne, depth, err, split, &nf);
-	stack_max = max(stack_max, depth);
-	if (err != POT_OK) return err;
-	if (lane_f() == 0) n_far += nf;
+}
+
+// Each member's push, absorption and boundary test, from the walk's fields.
+template <int TPL, int STG>
+__device__ __forceinline__ void push_members(const Field<TPL>& ef, const Targets<TPL>& tg, int split, uint32_t n_eval,
+                                             double4* __restrict__ pos, double4* __restrict__ vel,
+                                             const float4* __restrict__ src32, uint32_t* __restrict__ rein_list,
+                                             const Params& P, RunRec* rec, const double4* __restrict__ src64,
+                                             const StageBufs& sb, const PushCtx& pc, unsigned long long& n_inter,
+                                             unsigned long long& n_push)
+{
+	const bool owner = lane_f() < 32u / (uint32_t)split;
 #pragma unroll
 	for (int k = 0; k < TPL; k++) {
 		if (!tg.valid[k] || !owner) continue;
-		const uint32_t s = slot[k];
+		const uint32_t s = tg.self[k];
 		const double4 p = pos[s];
 		double4 v = vel[s];
 		const int sp = (int)p.w;
@@ -1109,7 +1228,7 @@ __device__ __forceinline__ int push_group(uint2 grp, double4* __restrict__ pos, 
 		const double3 hk = STG == 0 ? make_double3(fma(0.5 * dt, v.x, p.x), fma(0.5 * dt, v.y, p.y),
 		                                           fma(0.5 * dt, v.z, p.z))
 		                            : make_double3(p.x, p.y, p.z);
-		n_inter += ne;
+		n_inter += n_eval;
 		if (STG != 1) n_push++;
 		double E[3] = { (double)ef.x[k] * pc.escale, (double)ef.y[k] * pc.escale, (double)ef.z[k] * pc.escale };
 		if (P.shape && sp != SP_DUST) {
@@ -1148,7 +1267,187 @@ __device__ __forceinline__ int push_group(uint2 grp, double4* __restrict__ pos, 
 		vel[s] = v;
 		if (reason) rein_list[atomicAdd(&rec->n_rein, 1u)] = s | (reason << 30);
 	}
+}
+
+// One target group: the warp's walk for the whole group, then its members'
+// push.  Returns the walk's status (a group that fails is not pushed).
+template <int TPL, int STG, bool DIP>
+__device__ __forceinline__ int push_group(uint2 grp, double4* __restrict__ pos, double4* __restrict__ vel,
+                                          const TreeDev& T, const float4* __restrict__ src32,
+                                          const uint32_t* __restrict__ due_list, uint32_t* __restrict__ rein_list,
+                                          const Params& P, RunRec* rec, const double4* __restrict__ src64,
+                                          const StageBufs& sb, const PushCtx& pc, FastSmem<TPL, DIP>& sm,
+                                          unsigned long long& n_inter, unsigned long long& n_push,
+                                          uint32_t& stack_max, unsigned long long& n_far)
+{
+	Targets<TPL> tg;
+	const int split = split_of(TPL, grp.y);
+	load_targets<TPL, STG>(grp, split, pos, vel, due_list, P, tg);
+	WalkStats ws;
+	int err = POT_OK;
+	const Field<TPL> ef = group_walk<TPL, false, DIP>(tg, T, pc.srcf, P, sm, ws, err, split);
+	stack_max = max(stack_max, ws.depth);
+	if (err != POT_OK) return err;
+	if (lane_f() == 0) n_far += ws.n_far;
+	push_members<TPL, STG>(ef, tg, split, ws.n_eval, pos, vel, src32, rein_list, P, rec, src64, sb, pc, n_inter, n_push);
 	return POT_OK;
+}
+
+// The traversing warp's part of one group: its stages, the last with the
+// summed far expansion.  k, cb, lb, par (stage count, buffers, group parity)
+// carry over from group to group.
+template <int TPL, int STG, bool DIP>
+__device__ __forceinline__ int pair_traverse(uint32_t g, uint2 grp, const double4* __restrict__ pos,
+                                             const double4* __restrict__ vel, const TreeDev& T,
+                                             const uint32_t* __restrict__ due_list, const Params& P,
+                                             PairSmem<TPL, DIP>& sm, int pair, int& k, int& cb, int& lb, int& par)
+{
+	const int lane = (int)lane_f();
+	Targets<TPL> tg;
+	const int split = split_of(TPL, grp.y);
+	load_targets<TPL, STG>(grp, split, pos, vel, due_list, P, tg);
+	Traversal<TPL, false, DIP> tr;
+	tr.start(tg, T, sm.stack);
+	const int unit = Evaluation<TPL, false, DIP>::unit_of(split);
+	int first = ST_FIRST;
+	for (;;) {
+		bool done = tr.len == 0;
+		int err = POT_OK;
+		if (!done && !tr.round(tg, T, P, sm.stack, sm.cells[cb], sm.leaves[lb])) {
+			err = POT_E_WALK;
+			done = true;
+			tr.ncell = tr.nleaf = 0;
+		}
+		const bool fc = tr.ncell >= FW_CELL_FLUSH || (done && tr.ncell > 0);
+		const bool fl = tr.nleaf >= FW_LEAF_FLUSH || (done && tr.nleaf > 0);
+		if (!fc && !fl && !done) continue;
+		const int n = !fc ? 0 : (done ? (tr.ncell + unit - 1) / unit * unit : tr.ncell / unit * unit);
+		const int rem = fc && tr.ncell > n ? tr.ncell - n : 0;
+		if (fc && done && lane < n - tr.ncell) stage_pad<TPL, DIP>(sm.cells[cb], tr.ncell + lane);
+		if (done) {
+			auto& l = sm.last[par];
+			if constexpr (Traversal<TPL, false, DIP>::USE_FAR) {
+				tr.far.warp_sum();
+				if (lane == 0) {
+					const float f[15] = { tr.far.ex, tr.far.ey, tr.far.ez, tr.far.jxx, tr.far.jyy,
+					                      tr.far.jxy, tr.far.jxz, tr.far.jyz, tr.far.hxxx, tr.far.hyyy,
+					                      tr.far.hxxy, tr.far.hxxz, tr.far.hxyy, tr.far.hyyz, tr.far.hxyz };
+#pragma unroll
+					for (int i = 0; i < 15; i++) l.far[i] = f[i];
+					l.bc = tr.bc;
+				}
+			}
+			const uint32_t nf = __reduce_add_sync(0xffffffffu, tr.n_far);
+#pragma unroll
+			for (int i = 0; i < TPL; i++) {
+				const uint32_t m = __ballot_sync(0xffffffffu, tr.seen[i]);
+				if (lane == 0) l.seen[i] = m;
+			}
+			if (lane == 0) {
+				l.depth = (uint32_t)tr.maxlen;
+				l.n_far = nf;
+				l.err = err;
+			}
+			par ^= 1;
+		}
+		if (lane == 0) {
+			auto& st = sm.stage[k & 1];
+			st.group = g;
+			st.ncell = n;
+			st.cells = fc ? tr.ncell - rem : 0;
+			st.nleaf = fl ? tr.nleaf : 0;
+			st.cbuf = cb;
+			st.lbuf = lb;
+			st.flags = first | (done ? ST_LAST : 0);
+		}
+		first = 0;
+		__syncwarp();
+		pair_barrier(pair);
+		k++;
+		if (fc) {  // the carried cells (fewer than 32) move to the other buffer
+			if (lane < rem) {
+#pragma unroll
+				for (int i = 0; i < TPL; i++) sm.cells[cb ^ 1][TPL * lane + i] = sm.cells[cb][TPL * (n + lane) + i];
+				if (DIP) sm.cells[cb ^ 1][FW_CELLS + lane] = sm.cells[cb][FW_CELLS + n + lane];
+			}
+			tr.ncell = rem;
+			cb ^= 1;
+			__syncwarp();
+		}
+		if (fl) {
+			tr.nleaf = 0;
+			lb ^= 1;
+		}
+		if (done) return err;
+	}
+}
+
+template <int TPL, int STG, bool DIP>
+__device__ __forceinline__ void pair_end(PairSmem<TPL, DIP>& sm, int pair, int k)
+{
+	if (lane_f() == 0) sm.stage[k & 1].group = NONE;
+	__syncwarp();
+	pair_barrier(pair);
+}
+
+// The evaluating warp's state between the stages of a group.
+template <int TPL, bool DIP>
+struct PairEval {
+	Targets<TPL> tg;
+	Evaluation<TPL, false, DIP> ev;
+	uint32_t n_eval;
+};
+
+// One stage's evaluation, and the push after the group's last.
+template <int TPL, int STG, bool DIP>
+__device__ __forceinline__ void pair_stage(PairEval<TPL, DIP>& c, const typename PairSmem<TPL, DIP>::Stage& st,
+                                           uint2 grp, double4* __restrict__ pos, double4* __restrict__ vel,
+                                           const float4* __restrict__ src32, const uint32_t* __restrict__ due_list,
+                                           uint32_t* __restrict__ rein_list, const Params& P, RunRec* rec,
+                                           const double4* __restrict__ src64, const StageBufs& sb, const PushCtx& pc,
+                                           PairSmem<TPL, DIP>& sm, int& par, unsigned long long& n_inter,
+                                           unsigned long long& n_push, uint32_t& stack_max, unsigned long long& n_far)
+{
+	if (st.flags & ST_FIRST) {
+		const int split = split_of(TPL, grp.y);
+		load_targets<TPL, STG>(grp, split, pos, vel, due_list, P, c.tg);
+		c.ev.start(c.tg, split);
+		c.n_eval = 0;
+	}
+	if (st.ncell) {
+		c.ev.cells(sm.cells[st.cbuf], st.ncell);
+		c.n_eval += (uint32_t)st.cells;
+	}
+	if (st.nleaf) c.n_eval += c.ev.leaves(sm.leaves[st.lbuf], st.nleaf, sm.lsrc, sm.pbuf, pc.srcf, P);
+	if (!(st.flags & ST_LAST)) return;
+	const auto& l = sm.last[par];
+	par ^= 1;
+	stack_max = max(stack_max, l.depth);
+	if (l.err != POT_OK) {  // the group is not pushed
+		if (lane_f() == 0) set_status(rec, l.err);
+		return;
+	}
+	if (lane_f() == 0) n_far += l.n_far;
+	Field<TPL> F = c.ev.sum();
+	if constexpr (Traversal<TPL, false, DIP>::USE_FAR) {
+		FarExp far;
+		far.ex = l.far[0]; far.ey = l.far[1]; far.ez = l.far[2];
+		far.jxx = l.far[3]; far.jyy = l.far[4]; far.jxy = l.far[5]; far.jxz = l.far[6]; far.jyz = l.far[7];
+		far.hxxx = l.far[8]; far.hyyy = l.far[9]; far.hxxy = l.far[10]; far.hxxz = l.far[11];
+		far.hxyy = l.far[12]; far.hyyz = l.far[13]; far.hxyz = l.far[14];
+#pragma unroll
+		for (int i = 0; i < TPL; i++) {
+			const float3 e = far.at(c.tg.t[i].x - l.bc.x, c.tg.t[i].y - l.bc.y, c.tg.t[i].z - l.bc.z);
+			F.x[i] += e.x;
+			F.y[i] += e.y;
+			F.z[i] += e.z;
+		}
+	}
+#pragma unroll
+	for (int i = 0; i < TPL; i++)
+		if ((l.seen[i] >> lane_f()) & 1u) c.ev.take_back(F, i, c.tg, pc.srcf, P);
+	push_members<TPL, STG>(F, c.tg, c.ev.split, c.n_eval, pos, vel, src32, rein_list, P, rec, src64, sb, pc, n_inter,
+	                       n_push);
 }
 
 // The lanes' interaction and push counts, far cells and deepest stack into
@@ -1203,6 +1502,51 @@ k_push_fast(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 	push_stats(rec, n_inter, n_push, stack_max, n_far);
 }
 
+// The same with a pair of warps per group (see PairSmem).  Warps w and w ^ 1
+// of a block are a pair; which of them traverses alternates, so that both
+// kinds run on each of an SM's four schedulers.
+template <int TPL, int STG, bool DIP = false>
+__global__ void __launch_bounds__(FW_WARPS * 32, PAIR_BLOCKS)
+k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, const float4* __restrict__ src32,
+            const uint32_t* __restrict__ due_list, const uint2* __restrict__ groups, uint32_t* __restrict__ rein_list,
+            Params P, RunRec* rec, const double4* __restrict__ src64, StageBufs sb)
+{
+	__shared__ PairSmem<TPL, DIP> smem[FW_WARPS / 2];
+	__shared__ int status;  // one reading for the block: both warps of a pair go on or neither does
+	if (threadIdx.x == 0) status = rec->status;
+	__syncthreads();
+	if (status != POT_OK) return;
+	const int w = (int)(threadIdx.x >> 5), pair = w >> 1;
+	PairSmem<TPL, DIP>& sm = smem[pair];
+	const uint32_t n_groups = rec->n_groups;
+	if (((w ^ (w >> 1) ^ (int)(blockIdx.x / 148u)) & 1) == 0) {
+		int k = 0, cb = 0, lb = 0, par = 0;
+		for (;;) {
+			uint32_t g = 0;
+			if (lane_f() == 0) g = atomicAdd(&rec->work_ctr, 1u);
+			g = __shfl_sync(0xffffffffu, g, 0);
+			if (g >= n_groups) break;
+			if (pair_traverse<TPL, STG, DIP>(g, groups[g], pos, vel, T, due_list, P, sm, pair, k, cb, lb, par) != POT_OK)
+				break;
+		}
+		pair_end<TPL, STG, DIP>(sm, pair, k);
+	} else {
+		const PushCtx pc = push_ctx<STG>(pos, src32, P, rec, sb);
+		PairEval<TPL, DIP> c;
+		unsigned long long n_inter = 0, n_push = 0, n_far = 0;
+		uint32_t stack_max = 0;
+		int par = 0;
+		for (int k = 0;; k++) {
+			pair_barrier(pair);
+			const auto st = sm.stage[k & 1];
+			if (st.group == NONE) break;
+			pair_stage<TPL, STG, DIP>(c, st, groups[st.group], pos, vel, src32, due_list, rein_list, P, rec, src64, sb,
+			                          pc, sm, par, n_inter, n_push, stack_max, n_far);
+		}
+		push_stats(rec, n_inter, n_push, stack_max, n_far);
+	}
+}
+
 template <int TPL, bool DIP = false>
 __global__ void __launch_bounds__(FW_WARPS * 32) k_field_query_fast(TreeDev T, const float4* __restrict__ src32,
                                                                    const double* __restrict__ xyz,
@@ -1232,9 +1576,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_field_query_fast(TreeDev T, c
 				tg.self[k] = self_slot[j];
 			}
 		}
-		uint32_t ne = 0, depth = 0;
+		WalkStats ws;
 		int err = POT_OK;
-		const Field<TPL> ef = group_walk<TPL, false, DIP>(tg, T, src32, P, sm, ne, depth, err);
+		const Field<TPL> ef = group_walk<TPL, false, DIP>(tg, T, src32, P, sm, ws, err);
 		if (err != POT_OK && lane_f() == 0) set_status(rec, err);
 #pragma unroll
 		for (int k = 0; k < TPL; k++) {
@@ -1318,9 +1662,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_epe_fast(const double4* __res
 			tg.t[k] = make_float3(me.x, me.y, me.z);
 			qme[k] = me.w;
 		}
-		uint32_t ne = 0, depth = 0;
+		WalkStats ws;
 		int err = POT_OK;
-		const Field<TPL> f = group_walk<TPL, true, DIP>(tg, T, src32, P, sm, ne, depth, err, split);
+		const Field<TPL> f = group_walk<TPL, true, DIP>(tg, T, src32, P, sm, ws, err, split);
 		if (err != POT_OK) {
 			if (lane_f() == 0) set_status(rec, err);
 			break;
@@ -1375,6 +1719,20 @@ static void push_fast_stage(double4* pos, double4* vel, const TreeDev& T, const 
                             RunRec* rec, const StageBufs& sb, cudaStream_t s)
 {
 	const int nb = sm_count_fast() * 6;
+	if (P.n <= PAIR_MAX_N_PER_TARGET * P.group_max) {
+		const int np = sm_count_fast() * PAIR_BLOCKS;
+		if (P.group_max > 32) {
+			k_push_pair<2, STG><<<np, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P, rec,
+			                                                 src64, sb);
+		} else if (T.drec) {  // DIPOLES
+			k_push_pair<1, STG, true><<<np, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P,
+			                                                       rec, src64, sb);
+		} else {
+			k_push_pair<1, STG><<<np, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P, rec,
+			                                                 src64, sb);
+		}
+		return;
+	}
 	if (P.group_max > 32) {
 		k_push_fast<2, STG><<<nb, FW_WARPS * 32, 0, s>>>(pos, vel, T, src32, due_list, groups, rein_list, P, rec,
 		                                                 src64, sb);
