@@ -299,7 +299,7 @@ static int plan_packs(pot_batch* b, std::vector<int>& chains)
 		const uint32_t M = (uint32_t)views[c].size();
 		// device block: views, then per stage M + 1 prefix words, the group prefix, the counter
 		const size_t views_b = (sizeof(MemberView) * M + 255) / 256 * 256;
-		const size_t words = (size_t)PS_COUNT * (M + 1) + (M + 1) + 1;
+		const size_t words = (size_t)PS_COUNT * (M + 1) + (2 * (size_t)M + 1) + 1;
 		std::vector<uint32_t> h(words, 0u);
 		for (uint32_t m = 0; m < M; m++) {
 			uint32_t nb[PS_COUNT];
@@ -319,7 +319,7 @@ static int plan_packs(pot_batch* b, std::vector<int>& chains)
 			pc.B.blocks[st] = h[(size_t)st * (M + 1) + M];
 		}
 		pc.B.gpre = w + (size_t)PS_COUNT * (M + 1);
-		pc.B.ctr = w + (size_t)PS_COUNT * (M + 1) + (M + 1);
+		pc.B.ctr = w + (size_t)PS_COUNT * (M + 1) + (2 * (size_t)M + 1);
 		BCK(cudaStreamCreateWithFlags(&pc.streams.main, cudaStreamNonBlocking));
 		pc.streams.forked = pc.streams.create();
 		BCK(cudaEventCreateWithFlags(&pc.join, cudaEventDisableTiming));

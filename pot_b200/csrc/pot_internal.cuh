@@ -87,8 +87,8 @@ struct RunRec {
 	unsigned int grain_due;
 	unsigned int warn;       // non-fatal conditions (bit 0: key collision at 21 levels)
 	unsigned int n_overflow; // deepest-level buckets of a leaf-size-1 tree this build
-	unsigned int n_groups;   // fast form: target groups this step
-	unsigned int n_groups_all;  // fast form: groups over every particle (potential energies)
+	unsigned int n_groups[2];      // fast form: target groups this step, large and small (see group_at)
+	unsigned int n_groups_all[2];  // the same over every particle (potential energies)
 	long long dq;
 	unsigned long long de;
 	unsigned long long nabs_ion;

@@ -87,8 +87,7 @@ __device__ __forceinline__ void keys_body(G grd, const double4* __restrict__ pos
 	__syncthreads();
 	if (grd.id() == 0 && threadIdx.x == 0) {
 		rec->n_overflow = 0;
-		rec->n_groups = 0;
-		rec->n_groups_all = 0;
+		for (int k = 0; k < 2; k++) rec->n_groups[k] = rec->n_groups_all[k] = 0;
 	}
 	if (begin_step && grd.id() == 0 && threadIdx.x == 0) {
 		const unsigned long long t = rec->t_steps + 1;

@@ -106,7 +106,7 @@ struct PackDev {
 	uint32_t npass;                 // radix passes, the same for every member
 	const uint32_t* pre[PS_COUNT];
 	uint32_t blocks[PS_COUNT];
-	uint32_t* gpre;                 // [M + 1] prefix of the members' target groups this step (device)
+	uint32_t* gpre;                 // [2 M + 1] prefix of the members' target groups this step (device)
 	unsigned int* ctr;              // the batch walk's work counter (device)
 };
 // The member's state at step k of a graph launch is in buffer cur ^ (k & 1)

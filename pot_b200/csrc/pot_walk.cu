@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_epe_plain(const double4* __re
 __global__ void __launch_bounds__(1024) k_epe_final(const double* __restrict__ partial, const unsigned int* count,
                                                     uint32_t fixed, RunRec* rec)
 {
-	const uint32_t n = count ? *count : fixed;
+	const uint32_t n = count ? count[0] + count[1] : fixed;
 	double v[3] = { 0.0, 0.0, 0.0 };
 	for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
 		for (int k = 0; k < 3; k++) v[k] += partial[3 * i + k];
@@ -764,7 +764,7 @@ void launch_epe(const double4* pos, const TreeDev& T, const double4* src64, cons
 	if (P.form == POT_FORM_FAST) {
 		launch_epe_fast(pos, T, src32, src64, groups_all, partial, P, rec, s, tm);
 		ScopedKernel k(tm, "epe_final");
-		k_epe_final<<<1, 1024, 0, s>>>(partial, &rec->n_groups_all, 0, rec);
+		k_epe_final<<<1, 1024, 0, s>>>(partial, rec->n_groups_all, 0, rec);
 		return;
 	}
 	ScopedKernel k(tm, "epe_plain", 2);

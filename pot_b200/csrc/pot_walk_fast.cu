@@ -896,12 +896,28 @@ __device__ __forceinline__ void child_range(const TreeDev& T, int32_t code, cons
 	}
 }
 
-__device__ __forceinline__ void emit_groups(unsigned int* ctr, uint2* groups, uint32_t start, uint32_t count,
-                                            uint32_t gmax)
+// The groups' array as one launch makes it: large groups (more than half the
+// largest size) from the front, small ones from the back.  The walk takes
+// them in that order, so that the cheap groups -- a small group's warp is
+// split and takes half a large one's time -- fill the launch's end; in the
+// order their cells finish, the last large groups keep a few warps busy
+// alone.  Walk per step 157 -> 143 us at 150,001 particles, 96 -> 91 at
+// 64,001, 718 -> 705 at 1,000,001.
+__device__ __forceinline__ int group_is_small(uint32_t count, uint32_t gmax) { return 2u * count <= gmax ? 1 : 0; }
+// Group g of n_large large and the rest small ones.
+__device__ __forceinline__ uint2 group_at(const uint2* __restrict__ groups, uint32_t cap, uint32_t n_large, uint32_t g)
+{
+	return groups[g < n_large ? g : cap - 1u - (g - n_large)];
+}
+
+__device__ __forceinline__ void emit_groups(unsigned int* ctr, uint2* groups, uint32_t cap, uint32_t start,
+                                            uint32_t count, uint32_t gmax)
 {
 	while (count > 0) {
 		const uint32_t c = count < gmax ? count : gmax;
-		groups[atomicAdd(ctr, 1u)] = make_uint2(start, c);
+		const int sm = group_is_small(c, gmax);
+		const uint32_t i = atomicAdd(&ctr[sm], 1u);
+		groups[sm ? cap - 1u - i : i] = make_uint2(start, c);
 		start += c;
 		count -= c;
 	}
@@ -933,7 +949,7 @@ __device__ __forceinline__ void groups_body(G grd, const TreeDev& T, const uint3
 		const uint32_t d = dpre_at(dpre, b) - dpre_at(dpre, a);
 		if (d == 0) continue;
 		if (d <= gmax) {
-			if (k == 0) emit_groups(ctr, groups, dpre_at(dpre, a), d, gmax);
+			if (k == 0) emit_groups(ctr, groups, P.n, dpre_at(dpre, a), d, gmax);
 			continue;
 		}
 		uint32_t run_start = 0, run = 0;
@@ -945,23 +961,23 @@ __device__ __forceinline__ void groups_body(G grd, const TreeDev& T, const uint3
 			const uint32_t dc = dpre_at(dpre, cb) - dpre_at(dpre, ca);
 			if (dc == 0) continue;
 			if (code >= 0 && dc > gmax) {
-				emit_groups(ctr, groups, run_start, run, gmax);
+				emit_groups(ctr, groups, P.n, run_start, run, gmax);
 				run = 0;
 				continue;
 			}
 			if (run + dc > gmax) {
-				emit_groups(ctr, groups, run_start, run, gmax);
+				emit_groups(ctr, groups, P.n, run_start, run, gmax);
 				run = 0;
 			}
 			if (run == 0) run_start = dpre_at(dpre, ca);
 			run += dc;
 		}
-		emit_groups(ctr, groups, run_start, run, gmax);
+		emit_groups(ctr, groups, P.n, run_start, run, gmax);
 	}
 	// slots after the tree's (a spheroidal grain) are a group of their own
 	if (grd.id() == 0 && threadIdx.x == 0 && P.n_tree < P.n) {
 		const uint32_t a = dpre_at(dpre, P.n_tree), b = dpre_at(dpre, P.n);
-		if (b > a) emit_groups(ctr, groups, a, b - a, gmax);
+		if (b > a) emit_groups(ctr, groups, P.n, a, b - a, gmax);
 	}
 }
 
@@ -1104,7 +1120,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_groups_prefix(uint32_t* __res
 			const uint32_t a = dpre_at(dpre, P.n_tree), b = dpre_at(dpre, P.n);
 			if (b > a) total += put_groups<true>(groups, total, a, b - a, gmax);
 		}
-		rec->n_groups = total;
+		rec->n_groups[0] = total;  // taken in this order, whatever their size
 	}
 }
 
@@ -1483,7 +1499,7 @@ k_push_fast(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 	FastSmem<TPL, DIP>& sm = smem[threadIdx.x >> 5];
 	// warp-uniform: another warp may set the status meanwhile
 	if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) return;
-	const uint32_t n_groups = rec->n_groups;
+	const uint32_t n_large = rec->n_groups[0], n_groups = n_large + rec->n_groups[1];
 	const PushCtx pc = push_ctx<STG>(pos, src32, P, rec, sb);
 	unsigned long long n_inter = 0, n_push = 0, n_far = 0;
 	uint32_t stack_max = 0;
@@ -1492,7 +1508,7 @@ k_push_fast(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 		if (lane_f() == 0) g = atomicAdd(&rec->work_ctr, 1u);
 		g = __shfl_sync(0xffffffffu, g, 0);
 		if (g >= n_groups) break;
-		const int err = push_group<TPL, STG, DIP>(groups[g], pos, vel, T, src32, due_list, rein_list, P, rec, src64,
+		const int err = push_group<TPL, STG, DIP>(group_at(groups, P.n, n_large, g), pos, vel, T, src32, due_list, rein_list, P, rec, src64,
 		                                          sb, pc, sm, n_inter, n_push, stack_max, n_far);
 		if (err != POT_OK) {
 			if (lane_f() == 0) set_status(rec, err);
@@ -1518,7 +1534,7 @@ k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 	if (status != POT_OK) return;
 	const int w = (int)(threadIdx.x >> 5), pair = w >> 1;
 	PairSmem<TPL, DIP>& sm = smem[pair];
-	const uint32_t n_groups = rec->n_groups;
+	const uint32_t n_large = rec->n_groups[0], n_groups = n_large + rec->n_groups[1];
 	if (((w ^ (w >> 1) ^ (int)(blockIdx.x / 148u)) & 1) == 0) {
 		int k = 0, cb = 0, lb = 0, par = 0;
 		for (;;) {
@@ -1526,7 +1542,8 @@ k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 			if (lane_f() == 0) g = atomicAdd(&rec->work_ctr, 1u);
 			g = __shfl_sync(0xffffffffu, g, 0);
 			if (g >= n_groups) break;
-			if (pair_traverse<TPL, STG, DIP>(g, groups[g], pos, vel, T, due_list, P, sm, pair, k, cb, lb, par) != POT_OK)
+			if (pair_traverse<TPL, STG, DIP>(g, group_at(groups, P.n, n_large, g), pos, vel, T, due_list, P, sm, pair, k, cb,
+			                                 lb, par) != POT_OK)
 				break;
 		}
 		pair_end<TPL, STG, DIP>(sm, pair, k);
@@ -1540,7 +1557,7 @@ k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 			pair_barrier(pair);
 			const auto st = sm.stage[k & 1];
 			if (st.group == NONE) break;
-			pair_stage<TPL, STG, DIP>(c, st, groups[st.group], pos, vel, src32, due_list, rein_list, P, rec, src64, sb,
+			pair_stage<TPL, STG, DIP>(c, st, group_at(groups, P.n, n_large, st.group), pos, vel, src32, due_list, rein_list, P, rec, src64, sb,
 			                          pc, sm, par, n_inter, n_push, stack_max, n_far);
 		}
 		push_stats(rec, n_inter, n_push, stack_max, n_far);
@@ -1615,7 +1632,7 @@ void launch_groups(const TreeDev& T, const uint32_t* dpre, uint2* groups, uint8_
 {
 	if (!gcell) {  // one launch, groups in the order their cells finish
 		ScopedKernel k(tm, "groups");
-		k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, dpre, groups, &rec->n_groups, P.group_max, P, rec);
+		k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, dpre, groups, rec->n_groups, P.group_max, P, rec);
 		return;
 	}
 	const uint32_t nb = group_blocks();
@@ -1639,7 +1656,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_epe_fast(const double4* __res
 	FastSmem<TPL, DIP>& sm = smem[threadIdx.x >> 5];
 	// warp-uniform: another warp may set the status meanwhile
 	if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) return;
-	const uint32_t n_groups = rec->n_groups_all;
+	const uint32_t n_large = rec->n_groups_all[0], n_groups = n_large + rec->n_groups_all[1];
 	const uint32_t gs = rec->grain_slot;
 	const double pscale = QE / (P.k4 * P.rad);
 	for (;;) {
@@ -1647,7 +1664,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_epe_fast(const double4* __res
 		if (lane_f() == 0) g = atomicAdd(&rec->work_ctr2, 1u);
 		g = __shfl_sync(0xffffffffu, g, 0);
 		if (g >= n_groups) break;
-		const uint2 grp = groups[g];
+		const uint2 grp = group_at(groups, P.n, n_large, g);
 		Targets<TPL> tg;
 		float qme[TPL];
 		const int split = TPL == 1 ? (grp.y <= 8 ? 4 : (grp.y <= 16 ? 2 : 1)) : 1;
@@ -1699,7 +1716,7 @@ void launch_epe_fast(const double4* pos, const TreeDev& T, const float4* src32, 
 {
 	ScopedKernel k(tm, "epe_fast", 2);
 	const bool two = P.group_max > 32;
-	k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, nullptr, groups_all, &rec->n_groups_all, two ? 64u : 32u, P,
+	k_groups<<<sm_count_fast() * 4, 256, 0, s>>>(T, nullptr, groups_all, rec->n_groups_all, two ? 64u : 32u, P,
 	                                              rec);
 	if (two) {
 		k_epe_fast<2><<<sm_count_fast() * 6, FW_WARPS * 32, 0, s>>>(pos, T, src32, src64, groups_all, partial, P,
@@ -1788,11 +1805,13 @@ __global__ void kp_groups(PackDev B)
 {
 	const SegBlock sb = seg_block(B.pre[PS_GROUPS], B.M);
 	const MemberView& v = B.mv[sb.m];
-	groups_body(GridSeg { sb.id, sb.n }, v.T, v.due_prefix, v.groups, &v.rec->n_groups, v.P.group_max, v.P, v.rec);
+	groups_body(GridSeg { sb.id, sb.n }, v.T, v.due_prefix, v.groups, v.rec->n_groups, v.P.group_max, v.P, v.rec);
 }
 
-// gpre[m] = target groups of members 0..m-1 (a member whose status is set
-// contributes none); the walk's work counter is reset.  One block.
+// The batch's groups, every member's large ones before every member's small
+// ones: gpre[m] = large groups of members 0..m-1, gpre[M + m] = all large ones
+// and the small ones of members 0..m-1 (a member whose status is set has
+// none); the walk's work counter is reset.  One block.
 __global__ void __launch_bounds__(1024) kp_group_prefix(PackDev B)
 {
 	__shared__ uint32_t carry;
@@ -1801,12 +1820,12 @@ __global__ void __launch_bounds__(1024) kp_group_prefix(PackDev B)
 		*B.ctr = 0u;
 	}
 	__syncthreads();
-	for (uint32_t base = 0; base < B.M; base += blockDim.x) {
+	for (uint32_t base = 0; base < 2u * B.M; base += blockDim.x) {
 		const uint32_t m = base + threadIdx.x;
 		uint32_t c = 0;
-		if (m < B.M) {
-			const RunRec* r = B.mv[m].rec;
-			c = r->status == POT_OK ? r->n_groups : 0u;
+		if (m < 2u * B.M) {
+			const RunRec* r = B.mv[m < B.M ? m : m - B.M].rec;
+			c = r->status == POT_OK ? r->n_groups[m < B.M ? 0 : 1] : 0u;
 		}
 		// block-wide inclusive scan of c, warp by warp
 		__shared__ uint32_t wsum[32];
@@ -1829,12 +1848,12 @@ __global__ void __launch_bounds__(1024) kp_group_prefix(PackDev B)
 		}
 		__syncthreads();
 		const uint32_t incl = x + ((threadIdx.x >> 5) ? wsum[(threadIdx.x >> 5) - 1] : 0u) + carry;
-		if (m < B.M) B.gpre[m] = incl - c;
+		if (m < 2u * B.M) B.gpre[m] = incl - c;
 		__syncthreads();
 		if (threadIdx.x == blockDim.x - 1) carry = incl;
 		__syncthreads();
 	}
-	if (threadIdx.x == 0) B.gpre[B.M] = carry;
+	if (threadIdx.x == 0) B.gpre[2u * B.M] = carry;
 }
 
 // The walk and push of every member's groups: each warp takes the next
@@ -1845,19 +1864,21 @@ __global__ void __launch_bounds__(FW_WARPS * 32, fw_push_blocks(TPL)) kp_push_fa
 {
 	__shared__ FastSmem<TPL, false> smem[FW_WARPS];
 	FastSmem<TPL, false>& sm = smem[threadIdx.x >> 5];
-	const uint32_t total = B.gpre[B.M];
+	const uint32_t total = B.gpre[2u * B.M];
 	const StageBufs sb { 0, nullptr, nullptr, nullptr };
 	for (;;) {
 		uint32_t g = 0;
 		if (lane_f() == 0) g = atomicAdd(B.ctr, 1u);
 		g = __shfl_sync(0xffffffffu, g, 0);
 		if (g >= total) break;
-		uint32_t lo = 0, hi = B.M;  // gpre[lo] <= g < gpre[hi]
+		uint32_t lo = 0, hi = 2u * B.M;  // gpre[lo] <= g < gpre[hi]
 		while (hi - lo > 1) {
 			const uint32_t mid = (lo + hi) >> 1;
 			if (B.gpre[mid] <= g) lo = mid; else hi = mid;
 		}
-		const MemberView& v = B.mv[lo];
+		const bool small = lo >= B.M;
+		const MemberView& v = B.mv[small ? lo - B.M : lo];
+		const uint32_t gi = g - B.gpre[lo];
 		RunRec* rec = v.rec;
 		// warp-uniform: another warp may set the status meanwhile
 		if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) continue;
@@ -1865,7 +1886,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32, fw_push_blocks(TPL)) kp_push_fa
 		const PushCtx pc = push_ctx<0>(v.pos[b], v.src32, v.P, rec, sb);
 		unsigned long long n_inter = 0, n_push = 0, n_far = 0;
 		uint32_t stack_max = 0;
-		const int err = push_group<TPL, 0, false>(v.groups[g - B.gpre[lo]], v.pos[b], v.vel[b], v.T, v.src32,
+		const int err = push_group<TPL, 0, false>(v.groups[small ? v.P.n - 1u - gi : gi], v.pos[b], v.vel[b], v.T, v.src32,
 		                                          v.due_list, v.rein_list, v.P, rec, v.src64, sb, pc, sm, n_inter,
 		                                          n_push, stack_max, n_far);
 		if (err != POT_OK && lane_f() == 0) set_status(rec, err);
