@@ -649,89 +649,152 @@ __device__ __forceinline__ void add_moment_dip(int& q, uint32_t& aq, double& cx,
 	aq += caq;
 }
 
-__global__ void k_moments(TreeDev T, const double4* __restrict__ src64, Params P, RunRec* rec)
+// The moments of cell k's children in member order, children with buckets or
+// dipoles among them.
+struct CellMoments {
+	int q;
+	uint32_t aq;
+	double c[3], p[3];
+};
+__device__ __noinline__ CellMoments cell_moments_general(const TreeDev& T, const double4* __restrict__ src64,
+                                                         const Params& P, uint32_t k)
+{
+	const bool dip = T.dip != nullptr;
+	int q = 0;
+	uint32_t aq = 0;
+	double cx = 0.0, cy = 0.0, cz = 0.0;
+	double px = 0.0, py = 0.0, pz = 0.0;
+	for (int s = 0; s < 8; s++) {
+		const int d = slot_digit(s);
+		const int32_t code = T.child[8u * k + (uint32_t)d];
+		if (code == CH_EMPTY) continue;
+		int cq;
+		uint32_t caq;
+		double ccx, ccy, ccz;
+		double cpx = 0.0, cpy = 0.0, cpz = 0.0;
+		if (code >= 0) {
+			cq = __ldcg(&T.q[code]);
+			caq = __ldcg(&T.aq[code]);
+			const double2* cp2 = reinterpret_cast<const double2*>(&T.cq[code]);
+			const double2 c01 = __ldcg(cp2), c23 = __ldcg(cp2 + 1);
+			const double4 c = make_double4(c01.x, c01.y, c23.x, c23.y);
+			ccx = c.x; ccy = c.y; ccz = c.z;
+			if (dip) {
+				const double2* dp2 = reinterpret_cast<const double2*>(&T.dip[code]);
+				const double2 d01 = __ldcg(dp2), d23 = __ldcg(dp2 + 1);
+				cpx = d01.x; cpy = d01.y; cpz = d23.x;
+			}
+		} else if (leaf_payload(code) < P.n_tree) {
+			const double4 sp = src64[leaf_payload(code)];
+			cq = (int)sp.w;
+			caq = (uint32_t)abs(cq);
+			ccx = sp.x; ccy = sp.y; ccz = sp.z;
+		} else {
+			// overflow bucket: its own running moments over its particles
+			const uint32_t e = leaf_payload(code);
+			const uint2 r = T.ovf[e - P.n_tree];
+			cq = 0;
+			caq = 0;
+			ccx = ccy = ccz = 0.0;
+			for (uint32_t j = r.x; j < r.x + r.y; j++) {
+				const double4 sp = src64[j];
+				const int pq = (int)sp.w;
+				const uint32_t paq = (uint32_t)abs(pq);
+				if (!paq) continue;
+				if (dip) {
+					add_moment_dip(cq, caq, ccx, ccy, ccz, cpx, cpy, cpz, pq, paq, sp.x, sp.y, sp.z, 0.0, 0.0,
+					               0.0);
+				} else {
+					add_moment(cq, caq, ccx, ccy, ccz, pq, paq, sp.x, sp.y, sp.z);
+				}
+			}
+		}
+		if (caq) {
+			if (dip) {
+				add_moment_dip(q, aq, cx, cy, cz, px, py, pz, cq, caq, ccx, ccy, ccz, cpx, cpy, cpz);
+			} else {
+				add_moment(q, aq, cx, cy, cz, cq, caq, ccx, ccy, ccz);
+			}
+		}
+	}
+	return CellMoments { q, aq, { cx, cy, cz }, { px, py, pz } };
+}
+
+// Plain form (leaf size 1): the reference's running update bottom-up, a thread
+// a cell, the last child's thread going on to the parent.  The chain of cells
+// from the deepest pair to the root sets the time, so a cell's child codes are
+// loaded at once and its children's moments two ahead of their update: 64 -> 51
+// us at 8,193 particles, 81 -> 65 at 150,001, 268 -> 222 at 1,000,001.
+__global__ void __launch_bounds__(256, 3) k_moments(TreeDev T, const double4* __restrict__ src64, Params P, RunRec* rec)
 {
 	const uint32_t M = rec->n_nodes;
 	if (M > T.cap) return;
-	const uint32_t L = P.leaf_size;
 	const bool dip = T.dip != nullptr;
 	for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < M; k0 += gridDim.x * blockDim.x) {
-	if (T.nint[k0] != 0) continue;
-	uint32_t k = k0;
-	for (;;) {
-		int q = 0;
-		uint32_t aq = 0;
-		double cx = 0.0, cy = 0.0, cz = 0.0;
-		double px = 0.0, py = 0.0, pz = 0.0;
-		for (int s = 0; s < 8; s++) {
-			const int d = slot_digit(s);
-			const int32_t code = T.child[8u * k + (uint32_t)d];
-			if (code == CH_EMPTY) continue;
-			int cq;
-			uint32_t caq;
-			double ccx, ccy, ccz;
-			double cpx = 0.0, cpy = 0.0, cpz = 0.0;
-			if (code >= 0) {
-				cq = __ldcg(&T.q[code]);
-				caq = __ldcg(&T.aq[code]);
-				const double2* cp2 = reinterpret_cast<const double2*>(&T.cq[code]);
-				const double2 c01 = __ldcg(cp2), c23 = __ldcg(cp2 + 1);
-				const double4 c = make_double4(c01.x, c01.y, c23.x, c23.y);
-				ccx = c.x; ccy = c.y; ccz = c.z;
-				if (dip) {
-					const double2* dp2 = reinterpret_cast<const double2*>(&T.dip[code]);
-					const double2 d01 = __ldcg(dp2), d23 = __ldcg(dp2 + 1);
-					cpx = d01.x; cpy = d01.y; cpz = d23.x;
-				}
-			} else if (L == 1 && leaf_payload(code) < P.n_tree) {
-				const double4 sp = src64[leaf_payload(code)];
-				cq = (int)sp.w;
-				caq = (uint32_t)abs(cq);
-				ccx = sp.x; ccy = sp.y; ccz = sp.z;
-			} else {
-				// bucket leaf: its own running moments over its particles
-				const uint32_t e = leaf_payload(code);
-				const uint2 r = L == 1 ? T.ovf[e - P.n_tree] : T.lrange[e];
-				cq = 0;
-				caq = 0;
-				ccx = ccy = ccz = 0.0;
-				for (uint32_t j = r.x; j < r.x + r.y; j++) {
-					const double4 sp = src64[j];
-					const int pq = (int)sp.w;
-					const uint32_t paq = (uint32_t)abs(pq);
-					if (!paq) continue;
-					if (dip) {
-						add_moment_dip(cq, caq, ccx, ccy, ccz, cpx, cpy, cpz, pq, paq, sp.x, sp.y, sp.z, 0.0, 0.0,
-						               0.0);
-					} else {
-						add_moment(cq, caq, ccx, ccy, ccz, pq, paq, sp.x, sp.y, sp.z);
+		if (T.nint[k0] != 0) continue;
+		uint32_t k = k0;
+		for (;;) {
+			const int4* row = reinterpret_cast<const int4*>(&T.child[8u * k]);
+			const int4 r0 = row[0], r1 = row[1];
+			// member order (slot_digit)
+			const int32_t code[8] = { r1.x, r1.y, r0.x, r0.y, r0.z, r0.w, r1.z, r1.w };
+			const int32_t p = T.parent[k] >> 3;
+			const uint32_t nint = k ? T.nint[p < 0 ? 0 : p] : 0u;
+			bool plain = !dip;
+#pragma unroll
+			for (int s = 0; s < 8; s++) plain = plain && (code[s] >= CH_EMPTY || leaf_payload(code[s]) < P.n_tree);
+			int q = 0;
+			uint32_t aq = 0;
+			double cx = 0.0, cy = 0.0, cz = 0.0, px = 0.0, py = 0.0, pz = 0.0;
+			if (plain) {
+				// the next two children's moments are on the way during a child's
+				// update (its divisions)
+				double4 ch[3];
+				uint32_t ca[3];
+				const auto fetch = [&](int32_t cd, double4& m, uint32_t& w) {
+					w = 0;
+					if (cd >= 0) {
+						const double2* cp = reinterpret_cast<const double2*>(&T.cq[cd]);
+						const double2 a = __ldcg(cp), b = __ldcg(cp + 1);
+						m = make_double4(a.x, a.y, b.x, b.y);  // its charge is in .w, exactly
+						w = __ldcg(&T.aq[cd]);
+					} else if (cd != CH_EMPTY) {
+						m = src64[leaf_payload(cd)];
+						w = (uint32_t)abs((int)m.w);
 					}
+				};
+				fetch(code[0], ch[0], ca[0]);
+				fetch(code[1], ch[1], ca[1]);
+#pragma unroll
+				for (int s = 0; s < 8; s++) {
+					if (s < 6) fetch(code[s + 2], ch[(s + 2) % 3], ca[(s + 2) % 3]);
+					asm volatile("" ::: "memory");
+					const double4 m = ch[s % 3];
+					const uint32_t w = ca[s % 3];
+					if (w) add_moment(q, aq, cx, cy, cz, (int)m.w, w, m.x, m.y, m.z);
 				}
+			} else {
+				const CellMoments m = cell_moments_general(T, src64, P, k);
+				q = m.q;
+				aq = m.aq;
+				cx = m.c[0]; cy = m.c[1]; cz = m.c[2];
+				px = m.p[0]; py = m.p[1]; pz = m.p[2];
 			}
-			if (caq) {
-				if (dip) {
-					add_moment_dip(q, aq, cx, cy, cz, px, py, pz, cq, caq, ccx, ccy, ccz, cpx, cpy, cpz);
-				} else {
-					add_moment(q, aq, cx, cy, cz, cq, caq, ccx, ccy, ccz);
-				}
+			T.q[k] = q;
+			T.aq[k] = aq;
+			T.cq[k] = make_double4(cx, cy, cz, (double)q);
+			if (dip) T.dip[k] = make_double4(px, py, pz, 0.0);
+			if (k == 0) break;
+			if (p < 0 || (uint32_t)p >= k) {  // parents precede children in pre-order
+				set_status(rec, POT_E_CAPACITY);
+				break;
 			}
+			__threadfence();
+			const uint32_t arrived = atomicAdd(&T.ctr[p], 1u) + 1u;
+			if (arrived != nint) break;
+			__threadfence();
+			k = (uint32_t)p;
 		}
-		T.q[k] = q;
-		T.aq[k] = aq;
-		T.cq[k] = make_double4(cx, cy, cz, (double)q);
-		if (dip) T.dip[k] = make_double4(px, py, pz, 0.0);
-		if (k == 0) break;
-		const int32_t p = T.parent[k] >> 3;
-		if (p < 0 || (uint32_t)p >= k) {  // parents precede children in pre-order
-			set_status(rec, POT_E_CAPACITY);
-			break;
-		}
-		__threadfence();
-		const uint32_t arrived = atomicAdd(&T.ctr[p], 1u) + 1u;
-		if (arrived != T.nint[p]) break;
-		__threadfence();
-		k = (uint32_t)p;
-	}
 	}
 }
 
