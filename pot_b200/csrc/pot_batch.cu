@@ -258,7 +258,7 @@ static void member_blocks(const MemberView& v, uint32_t out[PS_COUNT])
 	out[PS_KEYS] = keys_blocks(n);
 	out[PS_N256] = div_up(n, REORDER_THREADS);
 	out[PS_DUE] = StepWords::due_tiles(n);
-	out[PS_TILES] = StepWords::radix_tiles(n);
+	out[PS_TILES] = StepWords::radix_tiles(n, OS_ITEMS_MAX);
 	out[PS_CELLS] = StepWords::cell_tiles(nt - L);
 	out[PS_FINISH] = div_up(nt, 256);
 	out[PS_MOM] = div_up(nt, PACK_MOM_TILE);

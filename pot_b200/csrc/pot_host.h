@@ -54,7 +54,15 @@ struct ScopedKernel {
 // ---- sort.cu ------------------------------------------------------------
 constexpr int RS_BINS = 256;
 constexpr int OS_MAX_PASSES = 8;  // radix passes at most (64-bit keys, 8 bits each)
-constexpr int OS_TILE = 2048;     // keys per tile of a radix pass
+constexpr int OS_THREADS = 256;
+// Keys per thread of a radix pass (a tile has OS_THREADS times as many).
+// Small runs take small tiles: the pass is then one tile's latency, which
+// ranking eight keys a thread sets (eight passes of 8,193 keys 97 -> 86 us,
+// of 32,001 102 -> 86; at 128,001 102 and 106, at 1,000,001 245 and 215).  A
+// packed batch's passes, whose launch fills the device, take eight.
+constexpr uint32_t OS_SMALL_N = 100000u;
+constexpr uint32_t OS_ITEMS_MAX = 8;
+__host__ __device__ inline uint32_t os_items(uint32_t n) { return n < OS_SMALL_N ? 4u : OS_ITEMS_MAX; }
 constexpr int TILE_THREADS = 256;  // of the cell numbering and the due list
 constexpr int CELL_TILE = 2048;   // key pairs per tile of the cell numbering
 constexpr int DUE_TILE = 4096;    // slots per tile of the due list (whole blocks of the reorder)
@@ -71,8 +79,13 @@ struct StepWords {
 	unsigned int* keys_ctr;
 	uint32_t* cell;      // [cell_tiles(n)]
 	uint32_t* due;       // [due_tiles(n)]
-	uint32_t* status;    // [passes * radix_tiles(n) * 256]
-	__host__ __device__ static uint32_t radix_tiles(uint32_t n) { return (n + OS_TILE - 1) / OS_TILE; }
+	uint32_t* status;    // [passes * radix_rows(n) * 256]
+	__host__ __device__ static uint32_t radix_tiles(uint32_t n, uint32_t items)
+	{
+		return (n + OS_THREADS * items - 1) / (OS_THREADS * items);
+	}
+	// status rows a pass: the tiles of a single run's, which are the more
+	__host__ __device__ static uint32_t radix_rows(uint32_t n) { return radix_tiles(n, os_items(n)); }
 	__host__ __device__ static uint32_t cell_tiles(uint32_t n) { return (n + CELL_TILE - 1) / CELL_TILE; }
 	__host__ __device__ static uint32_t due_tiles(uint32_t n) { return (n + DUE_TILE - 1) / DUE_TILE; }
 	// words before the status rows, which start on a 256-byte boundary
@@ -91,7 +104,7 @@ struct StepWords {
 	}
 	__host__ __device__ static size_t words(uint32_t n, int passes)
 	{
-		return head(n) + (size_t)passes * radix_tiles(n) * RS_BINS;
+		return head(n) + (size_t)passes * radix_rows(n) * RS_BINS;
 	}
 };
 

@@ -59,23 +59,20 @@ __device__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
 // POT_E_ITER and the pass completes with wrong order but without hanging.
 // The keys are then staged in shared memory in digit order and written out
 // contiguously per digit.
-constexpr int OS_THREADS = 256;
-constexpr int OS_ITEMS = 8;
-static_assert(OS_TILE == OS_THREADS * OS_ITEMS, "radix tile");
 constexpr uint32_t LB_AGG = 1u << 30;
 constexpr uint32_t LB_PRE = 2u << 30;
 constexpr uint32_t LB_COUNT = (1u << 30) - 1u;
 constexpr long LOOKBACK_SPIN_CAP = 1L << 24;
 constexpr int OS_LOOKBACK = 8;      // earlier tiles read per round of the look-back
 
-template <class G>
+template <int OS_ITEMS, class G>
 __device__ __forceinline__ void os_pass_body(G grd, const uint64_t* __restrict__ kin,
                                              const uint32_t* __restrict__ vin, size_t n, int shift,
                                              const uint32_t* __restrict__ goff, uint32_t* __restrict__ status,
                                              unsigned int* __restrict__ tile_ctr, uint64_t* __restrict__ kout,
                                              uint32_t* __restrict__ vout, int* __restrict__ err)
 {
-	constexpr int NW = OS_THREADS / 32;
+	constexpr int NW = OS_THREADS / 32, OS_TILE = OS_THREADS * OS_ITEMS;
 	__shared__ uint32_t s_tile;
 	__shared__ uint32_t s_wcnt[NW][RS_BINS];  // per-warp running count, then per-warp exclusive prefix
 	__shared__ uint32_t s_loc[RS_BINS];       // digit start inside the staged tile
@@ -92,8 +89,7 @@ __device__ __forceinline__ void os_pass_body(G grd, const uint64_t* __restrict__
 		const uint32_t tile = s_tile;
 		const size_t base = (size_t)tile * OS_TILE;
 		if (base >= n) return;
-		// warp w holds the tile's keys [256 w, 256 w + 256), round r the 32 at
-		// 256 w + 32 r, so a key's index in the tile is (warp, round, lane) in order
+		// warp w holds OS_ITEMS rounds of 32 consecutive keys of the tile, so a key's index in the tile is (warp, round, lane) in order
 		uint64_t key[OS_ITEMS];
 		uint32_t val[OS_ITEMS];
 		uint32_t rank[OS_ITEMS];
@@ -197,6 +193,7 @@ __device__ __forceinline__ void os_pass_body(G grd, const uint64_t* __restrict__
 	}
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(OS_THREADS) k_os_pass(const uint64_t* __restrict__ kin,
                                                         const uint32_t* __restrict__ vin, size_t n, int shift,
                                                         const uint32_t* __restrict__ goff,
@@ -205,13 +202,14 @@ __global__ void __launch_bounds__(OS_THREADS) k_os_pass(const uint64_t* __restri
                                                         uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                         int* __restrict__ err)
 {
-	os_pass_body(GridSelf {}, kin, vin, n, shift, goff, status, tile_ctr, kout, vout, err);
+	os_pass_body<ITEMS>(GridSelf {}, kin, vin, n, shift, goff, status, tile_ctr, kout, vout, err);
 }
 
 static inline int os_passes(int low_bit) { return (63 - low_bit + 7) / 8; }
 
 // Blocks of k_os_pass resident on the device at once: the pass's grid, each
 // block taking tiles until none is left (no second wave of blocks).
+template <int ITEMS>
 static uint32_t os_resident()
 {
 	static uint32_t n = 0;
@@ -219,7 +217,7 @@ static uint32_t os_resident()
 		int dev = 0, sms = 0, per = 0;
 		cudaGetDevice(&dev);
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_os_pass, OS_THREADS, 0);
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_os_pass<ITEMS>, OS_THREADS, 0);
 		n = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per);
 	}
 	return n;
@@ -232,23 +230,31 @@ void step_words_clear(uint32_t* words, uint32_t n, int low_bit, cudaStream_t s)
 	cudaMemsetAsync(words, 0, sizeof(uint32_t) * StepWords::words(n, os_passes(low_bit)), s);
 }
 
-int radix_sort_pairs(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t* words, int low_bit, cudaStream_t s,
-                     Timer& tm, int* err)
+template <int ITEMS>
+static int sort_passes(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t* words, int low_bit, cudaStream_t s,
+                       Timer& tm, int* err)
 {
-	if (n == 0) return 0;
 	const StepWords W(words, n);
-	const uint32_t tiles = StepWords::radix_tiles(n);
+	const uint32_t tiles = StepWords::radix_tiles(n, ITEMS);
 	const int npass = os_passes(low_bit);
 	int src = 0;
 	for (int p = 0; p < npass; p++) {
 		ScopedKernel k(tm, "sort_pass");
-		const uint32_t grid = std::min<uint32_t>(tiles, os_resident());
-		k_os_pass<<<grid, OS_THREADS, 0, s>>>(keys[src], vals[src], n, low_bit + 8 * p, W.hist + p * RS_BINS,
-		                                      W.status + (size_t)p * tiles * RS_BINS, W.pass_ctr + p, keys[src ^ 1],
-		                                      vals[src ^ 1], err);
+		const uint32_t grid = std::min<uint32_t>(tiles, os_resident<ITEMS>());
+		k_os_pass<ITEMS><<<grid, OS_THREADS, 0, s>>>(keys[src], vals[src], n, low_bit + 8 * p, W.hist + p * RS_BINS,
+		                                             W.status + (size_t)p * tiles * RS_BINS, W.pass_ctr + p,
+		                                             keys[src ^ 1], vals[src ^ 1], err);
 		src ^= 1;
 	}
 	return src;
+}
+
+int radix_sort_pairs(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t* words, int low_bit, cudaStream_t s,
+                     Timer& tm, int* err)
+{
+	if (n == 0) return 0;
+	return os_items(n) == 4 ? sort_passes<4>(keys, vals, n, words, low_bit, s, tm, err)
+	                        : sort_passes<(int)OS_ITEMS_MAX>(keys, vals, n, words, low_bit, s, tm, err);
 }
 
 }  // namespace pot
@@ -276,9 +282,10 @@ __global__ void __launch_bounds__(OS_THREADS) kp_os_pass(PackDev B, int p)
 	const MemberView& v = B.mv[sb.m];
 	const StepWords W(v.words, v.P.n);
 	const int src = p & 1;
-	os_pass_body(GridSeg { sb.id, sb.n }, v.keys[src], v.vals[src], (size_t)v.P.n, (int)v.P.key_bits + 8 * p,
-	             W.hist + p * RS_BINS, W.status + (size_t)p * StepWords::radix_tiles(v.P.n) * RS_BINS, W.pass_ctr + p,
-	             v.keys[src ^ 1], v.vals[src ^ 1], &v.rec->status);
+	os_pass_body<(int)OS_ITEMS_MAX>(GridSeg { sb.id, sb.n }, v.keys[src], v.vals[src], (size_t)v.P.n,
+	                                (int)v.P.key_bits + 8 * p, W.hist + p * RS_BINS,
+	                                W.status + (size_t)p * StepWords::radix_rows(v.P.n) * RS_BINS, W.pass_ctr + p,
+	                                v.keys[src ^ 1], v.vals[src ^ 1], &v.rec->status);
 }
 
 void pack_sort_begin(const PackDev& B, cudaStream_t s)
