@@ -187,6 +187,46 @@ __device__ __forceinline__ void eval_src(Acc<2>& E, const TgtE<2>& t, const floa
 	}
 }
 
+// N staged evaluations, i, i + stride, ..., stage by stage, so that their
+// chains (a dozen dependent operations each) are in flight together; the sums
+// are added in order, as N calls of eval_src would.
+template <int N, bool SOFT, bool POT>
+__device__ __forceinline__ void eval_batch(Acc<2>& E, const TgtE<2>& t, const float4* buf, int i, int stride, float eps2)
+{
+	float2 dx[N], dy[N], dz[N], q[N], ri[N];
+#pragma unroll
+	for (int u = 0; u < N; u++) {
+		const float4 a = buf[2 * (i + u * stride)], b = buf[2 * (i + u * stride) + 1];
+		dx[u] = __fadd2_rn(t.x, make_float2(a.x, a.y));
+		dy[u] = __fadd2_rn(t.y, make_float2(a.z, a.w));
+		dz[u] = __fadd2_rn(t.z, make_float2(b.x, b.y));
+		q[u] = make_float2(b.z, b.w);
+	}
+#pragma unroll
+	for (int u = 0; u < N; u++) ri[u] = SOFT ? __ffma2_rn(dz[u], dz[u], make_float2(eps2, eps2)) : __fmul2_rn(dz[u], dz[u]);
+#pragma unroll
+	for (int u = 0; u < N; u++) ri[u] = __ffma2_rn(dy[u], dy[u], ri[u]);
+#pragma unroll
+	for (int u = 0; u < N; u++) ri[u] = __ffma2_rn(dx[u], dx[u], ri[u]);
+#pragma unroll
+	for (int u = 0; u < N; u++) ri[u] = make_float2(rsqrt_ftz(ri[u].x), rsqrt_ftz(ri[u].y));
+	if (POT) {
+#pragma unroll
+		for (int u = 0; u < N; u++) E.x = __ffma2_rn(q[u], ri[u], E.x);
+		return;
+	}
+#pragma unroll
+	for (int u = 0; u < N; u++) q[u] = __fmul2_rn(q[u], __fmul2_rn(ri[u], ri[u]));
+#pragma unroll
+	for (int u = 0; u < N; u++) q[u] = __fmul2_rn(q[u], ri[u]);
+#pragma unroll
+	for (int u = 0; u < N; u++) {
+		E.x = __ffma2_rn(q[u], dx[u], E.x);
+		E.y = __ffma2_rn(q[u], dy[u], E.y);
+		E.z = __ffma2_rn(q[u], dz[u], E.z);
+	}
+}
+
 // Two staged sources (x, y, z, q) in float4 slots 2p and 2p + 1 become one
 // FP32x2 operand pair, (-xa, -xb, -ya, -yb) and (-za, -zb, qa, qb), in place:
 // with one target per lane the packed instructions evaluate two sources at
@@ -590,6 +630,7 @@ struct Traversal {
 // duplicated target, and the two halves are added at the end.
 template <int TPL, bool POT, bool DIP>
 struct Evaluation {
+	static constexpr int EB = 4;
 	static constexpr int PER_EV = TPL == 1 ? 2 : 1;  // staged sources per evaluation
 	TgtE<2> te;
 	Acc<2> E;
@@ -637,13 +678,12 @@ struct Evaluation {
 		} else if (TPL == 2 || split == 1) {
 			for (int j = 0; j < nev; j += 8) {
 #pragma unroll
-				for (int u = 0; u < 8; u++) eval_src<false, POT>(E, te, buf, j + u, 0.f);
+				for (int u = 0; u < 8; u += EB) eval_batch<EB, false, POT>(E, te, buf, j + u, 1, 0.f);
 			}
 		} else {
 			const int per = nev / split;
 			for (int j = 0; j < per; j += 4) {
-#pragma unroll
-				for (int u = 0; u < 4; u++) eval_src<false, POT>(E, te, buf, (j + u) * split + sub, 0.f);
+				eval_batch<4, false, POT>(E, te, buf, j * split + sub, split, 0.f);
 			}
 		}
 	}
@@ -699,21 +739,19 @@ struct Evaluation {
 			constexpr int nev = 32 / PER_EV;
 			const uint32_t in_chunk = total - base < 32u ? total - base : 32u;
 			if ((TPL == 2 || split == 1) && in_chunk == 32u) {
-#pragma unroll 16
-				for (int m = 0; m < nev; m++) eval_src<true, POT>(E, te, pbuf, m, eps2);
+#pragma unroll
+				for (int m = 0; m < nev; m += EB) eval_batch<EB, true, POT>(E, te, pbuf, m, 1, eps2);
 			} else if (TPL == 2 || split == 1) {
 				// a flush's last, partial chunk: whole quads of evaluations that
 				// cover its particles (the padding beyond has zero charge)
 				const int need = TPL == 1 ? ((int)in_chunk + 1) / 2 : (int)in_chunk;
 				const int nq = (need + 3) & ~3;  // <= nev
 				for (int m = 0; m < nq; m += 4) {
-#pragma unroll
-					for (int u = 0; u < 4; u++) eval_src<true, POT>(E, te, pbuf, m + u, eps2);
+					eval_batch<4, true, POT>(E, te, pbuf, m, 1, eps2);
 				}
 			} else {
 				const int per = nev / split;
-#pragma unroll 8
-				for (int m = 0; m < per; m++) eval_src<true, POT>(E, te, pbuf, m * split + sub, eps2);
+				for (int m = 0; m < per; m += 4) eval_batch<4, true, POT>(E, te, pbuf, m * split + sub, split, eps2);
 			}
 			__syncwarp();
 		}
