@@ -39,10 +39,10 @@ constexpr int FW_LEAF_FLUSH = 32;
 constexpr uint32_t NONE = 0xFFFFFFFFu;
 static_assert(GROUP_MAX == 32 * FW_TPL_MAX, "one group per warp, at most FW_TPL_MAX targets per lane");
 // Blocks per SM the push kernels are compiled for.  With two targets per
-// lane the walk holds both targets' sums and operands: at four blocks (128
-// registers a thread) it needs no spills and runs faster than at five (96
-// registers, spilling), 4.51 against 4.65 ms per step on the 4m plasma.  One
-// target per lane fits 96 registers, and five blocks hide more latency.
+// lane the walk holds both targets' sums and operands: three, four and five
+// blocks take 3,553, 3,240 and 3,267 us per step on the 4m plasma.  One target
+// per lane fits 96 registers: four, five and six blocks take 702, 679 and
+// 733 us at 1,000,001 particles.
 constexpr int fw_push_blocks(int tpl) { return tpl == 2 ? 4 : 5; }
 // Pairs of warps take runs of few groups: N at most this many times the
 // largest group (about 20 targets a group of 32, half the particles due, so
@@ -189,7 +189,10 @@ __device__ __forceinline__ void eval_src(Acc<2>& E, const TgtE<2>& t, const floa
 
 // N staged evaluations, i, i + stride, ..., stage by stage, so that their
 // chains (a dozen dependent operations each) are in flight together; the sums
-// are added in order, as N calls of eval_src would.
+// are added in order, as N calls of eval_src would.  Four at a time, against
+// one after another: walk per step 704 and 679 us at 1,000,001 particles, 143
+// and 139 us at 150,001, 3,240 us both ways on the 4m plasma (two targets per
+// lane, whose two halves already overlap).
 template <int N, bool SOFT, bool POT>
 __device__ __forceinline__ void eval_batch(Acc<2>& E, const TgtE<2>& t, const float4* buf, int i, int stride, float eps2)
 {
