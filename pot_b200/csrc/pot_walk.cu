@@ -715,11 +715,11 @@ template <int STG, int G, bool DIP>
 static void push_plain(double4* pos, double4* vel, const TreeDev& T, const double4* src64, const uint32_t* due_list,
                        uint32_t* rein_list, const Params& P, RunRec* rec, const StageBufs& sb, cudaStream_t s)
 {
-	static int per = 0;
-	if (!per) {
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_push_plain<STG, G, DIP>, PW_WARPS * 32, 0);
-		if (per <= 0) per = 1;
-	}
+	static const int per = [] {  // set once, also by threads that step their first runs together
+		int n = 0;
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_push_plain<STG, G, DIP>, PW_WARPS * 32, 0);
+		return n > 0 ? n : 1;
+	}();
 	k_push_plain<STG, G, DIP><<<sm_count() * per, PW_WARPS * 32, 0, s>>>(pos, vel, T, src64, due_list, rein_list, P,
 	                                                                    rec, sb);
 }
