@@ -113,12 +113,17 @@ __device__ __forceinline__ void plain_term(PlainAcc& E, bool on, bool dip, const
 constexpr int PW_WARPS = 4;  // warps per block
 constexpr int PW_CAP = 640;
 constexpr int PW_RESERVE = 7 * (MAX_LEVELS + 1);
+// The list: its first 32 entries are evaluated before anything is appended to
+// 32 or more, so an append (of a round's nodes or of 32 of a bucket's
+// particles, at most one entry a lane) starts from 31 or fewer and ends with 63
+// or fewer.
+constexpr int PW_LIST = 64;
 constexpr uint32_t PW_PART = 1u << 31;  // list word: a particle (softened); the low bits the targets' mask
 template <int G, bool DIP> struct PwSmem {
 	int2 stack[PW_CAP];       // node code, targets' mask
-	double4 src[64];          // the list: position and charge
-	double4 dip[DIP ? 64 : 1];
-	uint32_t word[64];
+	double4 src[PW_LIST];     // the list: position and charge
+	double4 dip[DIP ? PW_LIST : 1];
+	uint32_t word[PW_LIST];
 	double2 txy[G];           // the targets
 	double tz[G];
 	uint32_t self[G];
@@ -251,12 +256,15 @@ __device__ PlainAcc plain_walk(uint32_t nt, double x, double y, double z, uint32
 		}
 		__syncwarp();
 		uint32_t om = __ballot_sync(0xffffffffu, over);
-		while (om) {  // every particle of an overflow bucket, a list at a time
+		while (om) {  // every particle of an overflow bucket, 32 at a time
 			const int b = __ffs(om) - 1;
 			om &= om - 1u;
 			const uint2 r = T.ovf[__shfl_sync(0xffffffffu, e, b) - P.n_tree];
 			const uint32_t bm = __shfl_sync(0xffffffffu, mask, b);
 			for (uint32_t j0 = r.x; j0 < r.x + r.y; j0 += 32) {
+				// the nodes before it, or the 32 particles before these, may have left
+				// up to 63 entries
+				if (n >= 32) plain_flush<G, PHI, DIP>(E, n, t, sub, x, y, z, sm, P, n_inter, rc);
 				const uint32_t j = j0 + lane;
 				if (j < r.x + r.y) {
 					uint32_t m = bm;
@@ -268,7 +276,6 @@ __device__ PlainAcc plain_walk(uint32_t nt, double x, double y, double z, uint32
 				}
 				n += (int)min(32u, r.x + r.y - j0);
 				__syncwarp();
-				if (n >= 32) plain_flush<G, PHI, DIP>(E, n, t, sub, x, y, z, sm, P, n_inter, rc);
 			}
 		}
 		// the next round's nodes, whose loads are in flight while the list is
