@@ -59,7 +59,7 @@ struct Rsqrt {
 
 // One term of the sum at offset (dx, dy, dz), squared distance d2 (of a
 // particle, softened; of a cell, not): kq is QE q / (4 pi eps0).  A term
-// whose bit is not set adds zero.
+// whose bit is not set (on) adds zero; dip implies on.
 template <bool PHI, bool DIP>
 __device__ __forceinline__ void plain_term(PlainAcc& E, bool on, bool dip, const double4& pd, double kq, double dx,
                                            double dy, double dz, double d2)
@@ -73,7 +73,7 @@ __device__ __forceinline__ void plain_term(PlainAcc& E, bool on, bool dip, const
 		double es = r.p3(kq);  // pot.c:1737-1749, 1789-1798
 		if (DIP && dip) {  // DIPOLES, pot.c:1739-1745: (q + 3 (p.r) / r^2) r / r^3 - p / r^3
 			es = r.p3(kq + 3.0 * r.p2(fma(dx, pd.x, fma(dy, pd.y, dz * pd.z))));
-			const double n3 = on ? r.p3(-1.0) : 0.0;
+			const double n3 = r.p3(-1.0);
 			E.x = fma(n3, pd.x, E.x);
 			E.y = fma(n3, pd.y, E.y);
 			E.z = fma(n3, pd.z, E.z);
@@ -145,7 +145,9 @@ __device__ __forceinline__ void plain_eval(PlainAcc& E, uint32_t t, uint32_t sub
 		double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
 		if (!PHI && on && part && d2 == 0.0) rc = POT_E_COINCIDENT;
 		if (part) d2 += P.soft2;
-		plain_term<PHI, DIP>(E, on, !part, sm.dip[DIP ? i : 0], c.w, dx, dy, dz, d2);
+		// only a cell's entry has a dipole; what lies in sm.dip of any other is
+		// whatever was there before
+		plain_term<PHI, DIP>(E, on, on && !part, sm.dip[DIP ? i : 0], c.w, dx, dy, dz, d2);
 		n_inter += on ? 1u : 0u;
 	}
 }
