@@ -465,7 +465,7 @@ __device__ __forceinline__ void reinject_body(G grd, double4* __restrict__ pos, 
                                               const uint32_t* __restrict__ pid, const uint32_t* list,
                                               const double4* __restrict__ src64, const Params& P, RunRec* rec)
 {
-	if (rec->status != POT_OK) return;
+	if (warp_status(rec) != POT_OK) return;
 	const uint32_t n = rec->n_rein;
 	const uint32_t t = (uint32_t)rec->t_steps;
 	const double chi_b = rec->chi_b;

@@ -282,6 +282,23 @@ __device__ __forceinline__ void set_status(RunRec* rec, int code)
 	atomicCAS(&rec->status, 0, code);
 }
 
+// The run's status as the whole block, or the calling warp, sees it: one
+// reading, from L2.  A kernel beside this one may set the status at any time, so
+// threads that meet at a barrier or a shuffle must not each read it.
+__device__ __forceinline__ int block_status(const RunRec* rec)
+{
+	__shared__ int status;
+	if (threadIdx.x == 0) status = __ldcg(&rec->status);
+	__syncthreads();
+	return status;
+}
+__device__ __forceinline__ int warp_status(const RunRec* rec)
+{
+	int status = POT_OK;
+	if ((threadIdx.x & 31u) == 0) status = __ldcg(&rec->status);
+	return __shfl_sync(0xffffffffu, status, 0);
+}
+
 __host__ __device__ inline int species_of_id(uint32_t id, uint32_t n_ions)
 {
 	return id == 0 ? SP_DUST : (id <= n_ions ? SP_ION : SP_E);

@@ -347,8 +347,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_epe_plain(const double4* __re
 	__shared__ PwSmem<G, DIP> smem[PW_WARPS];
 	PwSmem<G, DIP>& sm = smem[threadIdx.x >> 5];
 	double acc[3] = { 0.0, 0.0, 0.0 };
-	// warp-uniform: another warp may set the status meanwhile
-	if (__shfl_sync(0xffffffffu, lane_id() == 0 ? rec->status : 0, 0) == POT_OK) {
+	if (warp_status(rec) == POT_OK) {
 		const uint32_t gs = rec->grain_slot;
 		const uint32_t warps = gridDim.x * PW_WARPS;
 		for (uint32_t b = blockIdx.x * PW_WARPS + (threadIdx.x >> 5); b * G < P.n; b += warps) {
@@ -419,8 +418,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_push_plain(double4* __restric
 {
 	__shared__ PwSmem<G, DIP> smem[PW_WARPS];
 	PwSmem<G, DIP>& sm = smem[threadIdx.x >> 5];
-	// warp-uniform: another warp may set the status meanwhile
-	if (__shfl_sync(0xffffffffu, lane_id() == 0 ? rec->status : 0, 0) != POT_OK) return;
+	if (warp_status(rec) != POT_OK) return;
 	const uint32_t n_due = rec->n_due;
 	const unsigned long long t = rec->t_steps;
 	const bool grain_due = rec->grain_due != 0;
@@ -605,8 +603,9 @@ __device__ __forceinline__ void chi_b_body(G grd, const TreeDev& T, const double
 	__shared__ int32_t stack[4][PHI_STACK];
 	__shared__ double sample[64];
 	__shared__ int bad;
-	if (!(P.flags & FLAG_SCEPTIC) || rec->status != POT_OK) return;
+	if (!(P.flags & FLAG_SCEPTIC)) return;
 	if (!force && (rec->t_steps % 20) != 0) return;
+	if (block_status(rec) != POT_OK) return;
 	const uint32_t w = threadIdx.x >> 5;
 	if (threadIdx.x == 0) bad = 0;
 	__syncthreads();

@@ -1120,7 +1120,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_groups_count(TreeDev T, const
                                                                 uint32_t* __restrict__ gblk, uint32_t gmax, Params P,
                                                                 RunRec* rec)
 {
-	if (rec->status != POT_OK) return;
+	if (block_status(rec) != POT_OK) return;
 	uint32_t k0, k1, sum = 0;
 	block_cells(rec->n_nodes, k0, k1);
 	for (uint32_t k = k0 + threadIdx.x; k < k1; k += GROUP_THREADS) {
@@ -1140,7 +1140,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_groups_prefix(uint32_t* __res
                                                                  uint2* __restrict__ groups, uint32_t gmax, Params P,
                                                                  RunRec* rec)
 {
-	if (rec->status != POT_OK) return;
+	if (block_status(rec) != POT_OK) return;
 	__shared__ uint32_t carry;
 	if (threadIdx.x == 0) carry = 0;
 	__syncthreads();
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_groups_emit(TreeDev T, const 
                                                                uint2* __restrict__ groups, uint32_t gmax, Params P,
                                                                RunRec* rec)
 {
-	if (rec->status != POT_OK) return;
+	if (block_status(rec) != POT_OK) return;
 	uint32_t k0, k1;
 	block_cells(rec->n_nodes, k0, k1);
 	uint32_t at = gblk[blockIdx.x];
@@ -1538,8 +1538,7 @@ k_push_fast(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 {
 	__shared__ FastSmem<TPL, DIP> smem[FW_WARPS];
 	FastSmem<TPL, DIP>& sm = smem[threadIdx.x >> 5];
-	// warp-uniform: another warp may set the status meanwhile
-	if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) return;
+	if (warp_status(rec) != POT_OK) return;
 	const uint32_t n_large = rec->n_groups[0], n_groups = n_large + rec->n_groups[1];
 	const PushCtx pc = push_ctx<STG>(pos, src32, P, rec, sb);
 	unsigned long long n_inter = 0, n_push = 0, n_far = 0;
@@ -1569,10 +1568,7 @@ k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
             Params P, RunRec* rec, const double4* __restrict__ src64, StageBufs sb)
 {
 	__shared__ PairSmem<TPL, DIP> smem[FW_WARPS / 2];
-	__shared__ int status;  // one reading for the block: both warps of a pair go on or neither does
-	if (threadIdx.x == 0) status = rec->status;
-	__syncthreads();
-	if (status != POT_OK) return;
+	if (block_status(rec) != POT_OK) return;  // both warps of a pair go on or neither does
 	const int w = (int)(threadIdx.x >> 5), pair = w >> 1;
 	PairSmem<TPL, DIP>& sm = smem[pair];
 	const uint32_t n_large = rec->n_groups[0], n_groups = n_large + rec->n_groups[1];
@@ -1695,8 +1691,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) k_epe_fast(const double4* __res
 {
 	__shared__ FastSmem<TPL, DIP> smem[FW_WARPS];
 	FastSmem<TPL, DIP>& sm = smem[threadIdx.x >> 5];
-	// warp-uniform: another warp may set the status meanwhile
-	if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) return;
+	if (warp_status(rec) != POT_OK) return;
 	const uint32_t n_large = rec->n_groups_all[0], n_groups = n_large + rec->n_groups_all[1];
 	const uint32_t gs = rec->grain_slot;
 	const double pscale = QE / (P.k4 * P.rad);
@@ -1921,8 +1916,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32, fw_push_blocks(TPL)) kp_push_fa
 		const MemberView& v = B.mv[small ? lo - B.M : lo];
 		const uint32_t gi = g - B.gpre[lo];
 		RunRec* rec = v.rec;
-		// warp-uniform: another warp may set the status meanwhile
-		if (__shfl_sync(0xffffffffu, lane_f() == 0 ? rec->status : 0, 0) != POT_OK) continue;
+		if (warp_status(rec) != POT_OK) continue;
 		const uint32_t b = pack_out(v, k);
 		const PushCtx pc = push_ctx<0>(v.pos[b], v.src32, v.P, rec, sb);
 		unsigned long long n_inter = 0, n_push = 0, n_far = 0;
