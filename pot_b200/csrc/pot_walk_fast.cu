@@ -907,8 +907,11 @@ struct PairSmem {
 };
 constexpr int ST_FIRST = 1, ST_LAST = 2;
 
+// bar.sync counts warps, not lanes, and needs the whole warp to arrive as one:
+// the lanes, which part in the members' push, converge first.
 __device__ __forceinline__ void pair_barrier(int pair)
 {
+	__syncwarp();
 	asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
 }
 
@@ -1418,7 +1421,6 @@ __device__ __forceinline__ int pair_traverse(uint32_t g, uint2 grp, const double
 			st.flags = first | (done ? ST_LAST : 0);
 		}
 		first = 0;
-		__syncwarp();
 		pair_barrier(pair);
 		k++;
 		if (fc) {  // the carried cells (fewer than 32) move to the other buffer
@@ -1443,7 +1445,6 @@ template <int TPL, int STG, bool DIP>
 __device__ __forceinline__ void pair_end(PairSmem<TPL, DIP>& sm, int pair, int k)
 {
 	if (lane_f() == 0) sm.stage[k & 1].group = NONE;
-	__syncwarp();
 	pair_barrier(pair);
 }
 
