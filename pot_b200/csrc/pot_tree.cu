@@ -739,7 +739,10 @@ __global__ void __launch_bounds__(256, 3) k_moments(TreeDev T, const double4* __
 			// member order (slot_digit)
 			const int32_t code[8] = { r1.x, r1.y, r0.x, r0.y, r0.z, r0.w, r1.z, r1.w };
 			const int32_t p = T.parent[k] >> 3;
-			const uint32_t nint = k ? T.nint[p < 0 ? 0 : p] : 0u;
+			// parents precede children in pre-order; a cell that none claimed (keys
+			// out of order after a sort that gave up) holds any value
+			const bool orphan = k != 0 && (p < 0 || (uint32_t)p >= k);
+			const uint32_t nint = k != 0 && !orphan ? T.nint[p] : 0u;
 			bool plain = !dip;
 #pragma unroll
 			for (int s = 0; s < 8; s++) plain = plain && (code[s] >= CH_EMPTY || leaf_payload(code[s]) < P.n_tree);
@@ -785,7 +788,7 @@ __global__ void __launch_bounds__(256, 3) k_moments(TreeDev T, const double4* __
 			T.cq[k] = make_double4(cx, cy, cz, (double)q);
 			if (dip) T.dip[k] = make_double4(px, py, pz, 0.0);
 			if (k == 0) break;
-			if (p < 0 || (uint32_t)p >= k) {  // parents precede children in pre-order
+			if (orphan) {
 				set_status(rec, POT_E_CAPACITY);
 				break;
 			}
@@ -1039,6 +1042,12 @@ __device__ __forceinline__ void moments_prefix_body(G grd, const TreeDev& T, con
 		T.aq[k] = (uint32_t)llrint(m.a);
 		T.cq[k] = make_double4(cx + P.rad, cy + P.rad, cz + P.rad, (double)q);
 		const uint32_t o = k == 0 ? 8u * T.cap : (uint32_t)T.parent[k];
+		// parents precede children in pre-order; a cell that none claimed (keys
+		// out of order after a sort that gave up) holds any value
+		if (k != 0 && o >= 8u * k) {
+			set_status(rec, POT_E_CAPACITY);
+			continue;
+		}
 		put_rec(&T.nrec[o], (float)(cx * P.inv_rad), (float)(cy * P.inv_rad), (float)(cz * P.inv_rad), (float)q,
 		        (float)(T.w2[k] * P.inv_rad * P.inv_rad / P.oap2), 8u * k, mask);
 		if (pre_d) {

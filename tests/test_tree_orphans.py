@@ -1,0 +1,83 @@
+"""A tree over keys that are out of order (a radix sort whose look-back gave up
+sets POT_E_ITER and goes on) can hold cells that no parent claims, whose entry
+of T.parent is whatever the memory held.  Restates the claims of k_finish_nodes
+and the uses of the entry in the moments kernels (pot_tree.cu): no index taken
+from it leaves its array."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+import tree_model as tm
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pot_b200", "csrc", "pot_tree.cu")
+
+
+def parents(keys, garbage, L=1):
+    """T.parent after the topology kernels: 8 k + digit, garbage where nobody wrote."""
+    n = len(keys)
+    lvl = np.minimum(tm.lcp_levels(keys[:n - L], keys[L:]), tm.MAX_LEVELS - 1)
+    prev = np.concatenate([[-1], lvl[:-1]])
+    cnt = np.maximum(lvl - prev, 0)
+    base = np.concatenate([[0], np.cumsum(cnt)[:-1]])
+    M = int(cnt.sum())
+    first = np.repeat(np.arange(n - L), cnt)
+    level = np.concatenate([np.arange(p + 1, l + 1) for p, l in zip(prev, lvl)])
+    out = np.array(garbage[:M])
+    claimed = set()
+    for k in range(M):
+        f, l = int(first[k]), int(level[k])
+        shift = 63 - 3 * l
+        e = tm.cell_end(keys, f, n, shift, int(keys[f]) >> shift)
+        s = [f] + tm.child_starts(keys, f, e, shift - 3) + [e]
+        for d in range(8):
+            c = int(s[d + 1]) - int(s[d])
+            if 0 <= c <= L or l + 1 >= tm.MAX_LEVELS:
+                continue
+            sc = int(s[d])
+            lo = 0 if sc == 0 or sc > len(lvl) else int(lvl[sc - 1]) + 1
+            if sc + L >= n:
+                continue
+            kc = int(base[sc]) + l + 1 - lo
+            if kc < 0 or kc >= M or kc <= k:
+                continue
+            out[kc] = 8 * k + d
+            claimed.add(kc)
+    out[0] = -1
+    return out, len(claimed), M
+
+
+def test_unclaimed_cells_are_not_followed():
+    rng = np.random.default_rng(1)
+    x, y, z = rng.uniform(0.0, 1.0, size=(3, 400))
+    keys = np.sort(tm.morton_keys(x, y, z, 1.0))
+    _, claimed, M = parents(keys, np.zeros(4000, np.int64))
+    assert claimed == M - 1  # in order: every cell but the root
+    orphans = wild = 0
+    for seed in range(4):
+        shuffled = np.random.default_rng(seed).permutation(keys)
+        garbage = rng.integers(-2 ** 31, 2 ** 31, size=4000)
+        par, claimed, M = parents(shuffled, garbage)
+        cap = 4 * len(keys) + 4096
+        assert M <= cap
+        orphans += M - 1 - claimed
+        for k in range(1, M):
+            # k_moments: nint[p], cells p < k only
+            p = int(par[k]) >> 3
+            orphan = p < 0 or p >= k
+            assert orphan or p < M
+            # moments_prefix_body: nrec[o], o < 8 k only
+            o = int(par[k]) & 0xFFFFFFFF
+            assert o >= 8 * k or o < 8 * cap
+            wild += o > 8 * cap
+    assert orphans > 0 and wild > 0  # without the checks these were followed
+
+
+@pytest.mark.parametrize("use,check", [(r"T\.nint\[p\]", r"\(uint32_t\)p >= k"), (r"T\.nrec\[o\]", r"o >= 8u \* k")])
+def test_checks_stand_ahead_of_the_uses(use, check):
+    text = re.sub(r"//[^\n]*", "", open(SRC).read())
+    uses = [m.start() for m in re.finditer(use, text)]
+    assert uses
+    for u in uses:
+        assert re.search(check, text[max(0, u - 500):u]), use
