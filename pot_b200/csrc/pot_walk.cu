@@ -172,7 +172,8 @@ __device__ __forceinline__ void plain_flush(PlainAcc& E, int& n, uint32_t t, uin
 
 // Sums of the warp's nt <= G targets: lane l holds target l % G's point and
 // slot (0xFFFFFFFF for none) and its share of the lists; the lanes l < G
-// return the targets' sums.  n_inter counts the lane's terms.
+// return the targets' sums.  n_inter counts the lane's terms; rc is set for a
+// target at a particle's position, whose sum is zero.
 template <int G, bool PHI, bool DIP>
 __device__ PlainAcc plain_walk(uint32_t nt, double x, double y, double z, uint32_t me, const TreeDev& T,
                                const double4* __restrict__ src64, const Params& P, PwSmem<G, DIP>& sm,
@@ -312,6 +313,14 @@ __device__ PlainAcc plain_walk(uint32_t nt, double x, double y, double z, uint32
 		if (!PHI) {
 			E.y += __shfl_xor_sync(0xffffffffu, E.y, o);
 			E.z += __shfl_xor_sync(0xffffffffu, E.z, o);
+		}
+	}
+	if (!PHI) {  // a target at a particle's position has no field, whichever lane met it
+		constexpr uint32_t LANES = G == 2 ? 0x55555555u : (G == 4 ? 0x11111111u : 0x01010101u);  // of target 0
+		static_assert(G == 2 || G == 4 || G == 8, "targets per warp");
+		if (__ballot_sync(0xffffffffu, rc != POT_OK) & (LANES << t)) {
+			rc = POT_E_COINCIDENT;
+			E = PlainAcc { 0.0, 0.0, 0.0 };
 		}
 	}
 	return E;
@@ -461,7 +470,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_push_plain(double4* __restric
 		const int sp = (int)p.w;
 		const double dt = P.dt * (double)P.tss[sp];
 		double E[3] = { r.x, r.y, r.z };
-		if (P.shape && sp != SP_DUST) {
+		if (P.shape && sp != SP_DUST && rc == POT_OK) {
 			// a spheroidal grain's own field first (pot-spheroid.c:1815-1819)
 			spheroid_field(P, qg, dsub(h.x, gx), dsub(h.y, gy), dsub(h.z, gz), E);
 			E[0] += r.x;
@@ -680,7 +689,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32) k_field_query_plain(TreeDev T, 
 	if (rc != POT_OK) set_status(rec, rc);
 	if (!has || lane_id() >= G) return;
 	double e[3] = { 0.0, 0.0, 0.0 };
-	if (P.shape && self != rec->grain_slot) {
+	if (P.shape && self != rec->grain_slot && rc == POT_OK) {
 		spheroid_field(P, (double)rec->grain_q, dsub(h.x, rec->grain_pos[0]), dsub(h.y, rec->grain_pos[1]),
 		               dsub(h.z, rec->grain_pos[2]), e);
 	}
