@@ -916,10 +916,10 @@ static void enqueue_tree(pot_gpu_ctx* c, int begin_step, const StepStreams& S)
 	const int kb = radix_sort_pairs(c->keys, c->vals, c->n, c->words, (int)P.key_bits, s, c->timer, &c->rec->status);
 	c->kb = kb;
 	S.order(0, s, S.tree());
-	launch_cells(c->keys[kb], c->T, P, c->rec, c->words, S.tree(), c->timer);
+	launch_cells(c->keys[kb], c->vals[kb], c->pos[c->cur], c->T, P, c->rec, c->words, S.tree(), c->timer);
 	const int nx = c->cur ^ 1;
-	launch_reorder(c->keys[kb], c->vals[kb], c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->pos[nx], c->vel[nx],
-	               c->pid[nx], c->src64, c->src32, c->due, c->words, P, c->rec, s, c->timer);
+	launch_reorder(c->vals[kb], c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->pos[nx], c->vel[nx], c->pid[nx],
+	               c->src64, c->src32, c->due, c->words, P, c->rec, s, c->timer);
 	c->cur = nx;
 	if (begin_step) {
 		S.order(1, s, S.list());

@@ -339,7 +339,7 @@ static void enqueue_pack(const PackClass& pc, uint32_t spl)
 		pack_keys(B, (int)k, s);
 		pack_sort(B, s);
 		S.order(0, s, S.tree());
-		pack_cells(B, S.tree());
+		pack_cells(B, (int)k, S.tree());
 		pack_reorder(B, (int)k, s);
 		S.order(1, s, S.list());
 		pack_due_list(B, S.list());

@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(256) k_keys(const double4* __restrict__ pos, u
 // mark the particles due this step (electrons every step, ions every
 // tss[ION] steps, the grain every tss[DUST] steps, pot.c:2430-2434).
 // One slot of the reorder; returns whether the particle is due.
-__device__ __forceinline__ bool reorder_one(uint32_t s, const uint64_t* __restrict__ keys,
-                                            const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+__device__ __forceinline__ bool reorder_one(uint32_t s, const uint32_t* __restrict__ perm,
+                                            const double4* __restrict__ pos_in,
                                             const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in,
                                             double4* __restrict__ pos_out, double4* __restrict__ vel_out,
                                             uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
@@ -201,18 +201,12 @@ __device__ __forceinline__ bool reorder_one(uint32_t s, const uint64_t* __restri
 		                       (float)((p.z - P.rad) * P.inv_rad), (float)q);
 	}
 	if (sp == SP_DUST) rec->grain_slot = s;
-	// Two particles at one position: the reference's insertion would split
-	// forever (pot.c:1466-1470) or fail at a reallocation (pot.c:1578-1586).
-	if (s + 1 < P.n_tree && keys[s] == keys[s + 1]) {
-		const double4 o = pos_in[perm[s + 1]];
-		if (p.x == o.x && p.y == o.y && p.z == o.z) set_status(rec, POT_E_COINCIDENT);
-	}
 	return (rec->t_steps % P.tss[sp]) == 0;
 }
 
 template <class G>
-__device__ __forceinline__ void reorder_body(G grd, const uint64_t* __restrict__ keys,
-                                             const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+__device__ __forceinline__ void reorder_body(G grd, const uint32_t* __restrict__ perm,
+                                             const double4* __restrict__ pos_in,
                                              const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in,
                                              double4* __restrict__ pos_out, double4* __restrict__ vel_out,
                                              uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
@@ -223,7 +217,7 @@ __device__ __forceinline__ void reorder_body(G grd, const uint64_t* __restrict__
 	// the due slots of each DUE_TILE (a block lies inside one)
 	bool is_due = false;
 	if (s < P.n) {
-		is_due = reorder_one(s, keys, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, P, rec);
+		is_due = reorder_one(s, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, P, rec);
 		due[s] = is_due ? 1 : 0;
 	}
 	__shared__ uint32_t wcnt[REORDER_THREADS / 32];
@@ -238,12 +232,12 @@ __device__ __forceinline__ void reorder_body(G grd, const uint64_t* __restrict__
 }
 
 __global__ void __launch_bounds__(REORDER_THREADS)
-k_reorder(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
-          const double4* __restrict__ vel_in, const uint32_t* __restrict__ pid_in, double4* __restrict__ pos_out,
+k_reorder(const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in, const double4* __restrict__ vel_in,
+          const uint32_t* __restrict__ pid_in, double4* __restrict__ pos_out,
           double4* __restrict__ vel_out, uint32_t* __restrict__ pid_out, double4* __restrict__ src64,
           float4* __restrict__ src32, uint8_t* __restrict__ due, uint32_t* words, Params P, RunRec* rec)
 {
-	reorder_body(GridSelf {}, keys, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, due,
+	reorder_body(GridSelf {}, perm, pos_in, vel_in, pid_in, pos_out, vel_out, pid_out, src64, src32, due,
 	             StepWords(words, P.n).due, P, rec);
 }
 
@@ -383,12 +377,32 @@ struct PairLevels {
 	}
 };
 
+// Two particles at one position: the reference's insertion would split
+// forever (pot.c:1466-1470) or fail at a reallocation (pot.c:1578-1586).
+__device__ __forceinline__ void check_coincident(uint32_t i, const uint64_t* __restrict__ keys,
+                                                 const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+                                                 RunRec* rec)
+{
+	if (keys[i] != keys[i + 1]) return;
+	const double4 p = pos_in[perm[i]], o = pos_in[perm[i + 1]];
+	if (p.x == o.x && p.y == o.y && p.z == o.z) set_status(rec, POT_E_COINCIDENT);
+}
+
+// The positions of neighbours with one key are compared here, ahead of all that
+// can find the tree too large, so that the status names the cause.
 template <class G>
-__device__ __forceinline__ void cell_count_body(G grd, const uint64_t* __restrict__ keys, uint32_t n_pairs, uint32_t L,
-                                                int max_level, uint32_t* __restrict__ counts, RunRec* rec)
+__device__ __forceinline__ void cell_count_body(G grd, const uint64_t* __restrict__ keys,
+                                                const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
+                                                uint32_t n_pairs, uint32_t L, int max_level,
+                                                uint32_t* __restrict__ counts, RunRec* rec)
 {
 	const uint32_t i0 = grd.id() * CELL_TILE + threadIdx.x * (CELL_TILE / TILE_THREADS);
 	const PairLevels p(keys, i0, n_pairs, L, max_level, rec);
+#pragma unroll
+	for (int k = 0; k < CELL_TILE / TILE_THREADS; k++)
+		if (i0 + (uint32_t)k < n_pairs) check_coincident(i0 + (uint32_t)k, keys, perm, pos_in, rec);
+	// the last L - 1 pairs of neighbours, beyond the pairs (i, i + L)
+	if (grd.id() == 0 && threadIdx.x + 1 < L) check_coincident(n_pairs + threadIdx.x, keys, perm, pos_in, rec);
 	uint32_t total;
 	tile_scan(p.sum, &total);
 	if (threadIdx.x == 0) counts[grd.id()] = total;
@@ -422,11 +436,13 @@ __device__ __forceinline__ void cell_number_body(G grd, const uint64_t* __restri
 	}
 }
 
-__global__ void __launch_bounds__(TILE_THREADS) k_cell_count(const uint64_t* __restrict__ keys, uint32_t n_pairs,
+__global__ void __launch_bounds__(TILE_THREADS) k_cell_count(const uint64_t* __restrict__ keys,
+                                                             const uint32_t* __restrict__ perm,
+                                                             const double4* __restrict__ pos_in, uint32_t n_pairs,
                                                              uint32_t L, int max_level, uint32_t* __restrict__ counts,
                                                              RunRec* rec)
 {
-	cell_count_body(GridSelf {}, keys, n_pairs, L, max_level, counts, rec);
+	cell_count_body(GridSelf {}, keys, perm, pos_in, n_pairs, L, max_level, counts, rec);
 }
 
 __global__ void __launch_bounds__(TILE_THREADS) k_cell_number(const uint64_t* __restrict__ keys, uint32_t n_pairs,
@@ -1088,15 +1104,13 @@ void launch_keys(const double4* pos, uint64_t* keys, uint32_t* vals, const Param
 	                                        radix_passes((int)P.key_bits));
 }
 
-void launch_reorder(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, const double4* vel_in,
-                    const uint32_t* pid_in, double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64,
-                    float4* src32, uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s,
-                    Timer& tm)
+void launch_reorder(const uint32_t* perm, const double4* pos_in, const double4* vel_in, const uint32_t* pid_in,
+                    double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64, float4* src32,
+                    uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm)
 {
 	ScopedKernel k(tm, "reorder");
-	k_reorder<<<blocks_for(P.n, REORDER_THREADS), REORDER_THREADS, 0, s>>>(keys, perm, pos_in, vel_in, pid_in, pos_out,
-	                                                                       vel_out, pid_out, src64, src32, due, words,
-	                                                                       P, rec);
+	k_reorder<<<blocks_for(P.n, REORDER_THREADS), REORDER_THREADS, 0, s>>>(perm, pos_in, vel_in, pid_in, pos_out, vel_out,
+	                                                                       pid_out, src64, src32, due, words, P, rec);
 }
 
 void launch_due_list(const uint8_t* due, uint32_t* words, uint32_t* due_list, uint32_t* due_prefix, const Params& P,
@@ -1108,8 +1122,8 @@ void launch_due_list(const uint8_t* due, uint32_t* words, uint32_t* due_list, ui
 }
 
 // Topology from the sorted keys: cell numbering, extents and children.
-void launch_cells(const uint64_t* keys, TreeDev& T, const Params& P, RunRec* rec, uint32_t* words, cudaStream_t s,
-                  Timer& tm)
+void launch_cells(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, TreeDev& T, const Params& P,
+                  RunRec* rec, uint32_t* words, cudaStream_t s, Timer& tm)
 {
 	const uint32_t n = P.n_tree, L = P.leaf_size;
 	const uint32_t n_pairs = n - L;  // n_tree > L is checked at creation
@@ -1117,7 +1131,7 @@ void launch_cells(const uint64_t* keys, TreeDev& T, const Params& P, RunRec* rec
 		ScopedKernel k(tm, "tree_cells", 2);
 		uint32_t* counts = StepWords(words, P.n).cell;
 		const uint32_t nb = StepWords::cell_tiles(n_pairs);
-		k_cell_count<<<nb, TILE_THREADS, 0, s>>>(keys, n_pairs, L, (int)P.max_level, counts, rec);
+		k_cell_count<<<nb, TILE_THREADS, 0, s>>>(keys, perm, pos_in, n_pairs, L, (int)P.max_level, counts, rec);
 		k_cell_number<<<nb, TILE_THREADS, 0, s>>>(keys, n_pairs, L, (int)P.max_level, counts, T, rec);
 	}
 	ScopedKernel k(tm, "tree_finish");
@@ -1174,7 +1188,7 @@ __global__ void __launch_bounds__(REORDER_THREADS) kp_reorder(PackDev B, int k)
 	const SegBlock sb = seg_block(B.pre[PS_N256], B.M);
 	const MemberView& v = B.mv[sb.m];
 	const uint32_t a = pack_in(v, k), b = pack_out(v, k);
-	reorder_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.vals[v.kb], v.pos[a], v.vel[a], v.pid[a], v.pos[b], v.vel[b],
+	reorder_body(GridSeg { sb.id, sb.n }, v.vals[v.kb], v.pos[a], v.vel[a], v.pid[a], v.pos[b], v.vel[b],
 	             v.pid[b], v.src64, v.src32, v.due, StepWords(v.words, v.P.n).due, v.P, v.rec);
 }
 
@@ -1185,11 +1199,12 @@ __global__ void __launch_bounds__(TILE_THREADS) kp_due_list(PackDev B)
 	due_list_body(GridSeg { sb.id, sb.n }, v.due, StepWords(v.words, v.P.n).due, v.due_list, v.due_prefix, v.P, v.rec);
 }
 
-__global__ void __launch_bounds__(TILE_THREADS) kp_cell_count(PackDev B)
+__global__ void __launch_bounds__(TILE_THREADS) kp_cell_count(PackDev B, int k)
 {
 	const SegBlock sb = seg_block(B.pre[PS_CELLS], B.M);
 	const MemberView& v = B.mv[sb.m];
-	cell_count_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.P.n_tree - v.P.leaf_size, v.P.leaf_size,
+	cell_count_body(GridSeg { sb.id, sb.n }, v.keys[v.kb], v.vals[v.kb], v.pos[pack_in(v, k)],
+	                v.P.n_tree - v.P.leaf_size, v.P.leaf_size,
 	                (int)v.P.max_level, StepWords(v.words, v.P.n).cell, v.rec);
 }
 
@@ -1249,9 +1264,9 @@ void pack_due_list(const PackDev& B, cudaStream_t s)
 	kp_due_list<<<B.blocks[PS_DUE], TILE_THREADS, 0, s>>>(B);
 }
 
-void pack_cells(const PackDev& B, cudaStream_t s)
+void pack_cells(const PackDev& B, int k, cudaStream_t s)
 {
-	kp_cell_count<<<B.blocks[PS_CELLS], TILE_THREADS, 0, s>>>(B);
+	kp_cell_count<<<B.blocks[PS_CELLS], TILE_THREADS, 0, s>>>(B, k);
 	kp_cell_number<<<B.blocks[PS_CELLS], TILE_THREADS, 0, s>>>(B);
 	kp_finish_nodes<<<B.blocks[PS_FINISH], 256, 0, s>>>(B);
 }

@@ -121,7 +121,7 @@ void pack_keys(const PackDev& B, int k, cudaStream_t s);
 void pack_sort(const PackDev& B, cudaStream_t s);
 void pack_reorder(const PackDev& B, int k, cudaStream_t s);
 void pack_due_list(const PackDev& B, cudaStream_t s);
-void pack_cells(const PackDev& B, cudaStream_t s);
+void pack_cells(const PackDev& B, int k, cudaStream_t s);
 void pack_mom_sums(const PackDev& B, cudaStream_t s);
 void pack_moments(const PackDev& B, cudaStream_t s);
 void pack_groups(const PackDev& B, cudaStream_t s);
@@ -136,14 +136,13 @@ size_t mom_block_entries(size_t n);
 void launch_keys(const double4* pos, uint64_t* keys, uint32_t* vals, const Params& P, RunRec* rec,
                  int begin_step, uint32_t* words, cudaStream_t s, Timer& tm);
 uint32_t keys_blocks(size_t n);
-void launch_reorder(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, const double4* vel_in,
-                    const uint32_t* pid_in, double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64,
-                    float4* src32, uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s,
-                    Timer& tm);
+void launch_reorder(const uint32_t* perm, const double4* pos_in, const double4* vel_in, const uint32_t* pid_in,
+                    double4* pos_out, double4* vel_out, uint32_t* pid_out, double4* src64, float4* src32,
+                    uint8_t* due, uint32_t* words, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
 void launch_due_list(const uint8_t* due, uint32_t* words, uint32_t* due_list, uint32_t* due_prefix, const Params& P,
                      RunRec* rec, cudaStream_t s, Timer& tm);
-void launch_cells(const uint64_t* keys, TreeDev& T, const Params& P, RunRec* rec, uint32_t* words, cudaStream_t s,
-                  Timer& tm);
+void launch_cells(const uint64_t* keys, const uint32_t* perm, const double4* pos_in, TreeDev& T, const Params& P,
+                  RunRec* rec, uint32_t* words, cudaStream_t s, Timer& tm);
 void launch_mom_sums(TreeDev& T, const double4* src64, const Params& P, cudaStream_t s, Timer& tm);
 void launch_moments(TreeDev& T, const double4* src64, const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
 
