@@ -149,8 +149,8 @@ void launch_moments(TreeDev& T, const double4* src64, const Params& P, RunRec* r
 // ---- branches of a step --------------------------------------------------
 // A captured step runs on three streams: while the main one reorders the
 // state and sums its moments, the second builds the tree's topology from the
-// sorted keys (and later measures chi_b beside the walk) and the third lists
-// the due particles and makes the target groups.  Without side streams the
+// sorted keys (and later measures chi_b) and the third lists the due particles
+// and makes the target groups; all three meet ahead of the push.  Without side streams the
 // same launches follow each other on the main one.
 struct StepStreams {
 	cudaStream_t main = nullptr, side[2] = { nullptr, nullptr };
