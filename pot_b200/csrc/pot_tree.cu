@@ -345,12 +345,11 @@ __device__ __forceinline__ int lcp_levels(uint64_t a, uint64_t b)
 	return (__clzll((long long)x) - 1) / 3;
 }
 
-// Common levels of keys i and i + L, capped at max_level - 1 (a cell of the
-// deepest level cannot split).
-__device__ __forceinline__ int pair_levels(const uint64_t* __restrict__ keys, uint32_t i, uint32_t L, int max_level,
-                                           RunRec* rec)
+// Common levels of the keys of slots i and i + L, capped at max_level - 1 (a
+// cell of the deepest level cannot split).
+__device__ __forceinline__ int pair_levels(uint64_t a, uint64_t b, int max_level, RunRec* rec)
 {
-	const int l = lcp_levels(keys[i], keys[i + L]);
+	const int l = lcp_levels(a, b);
 	if (l == MAX_LEVELS && max_level == MAX_LEVELS && rec) atomicOr(&rec->warn, 1u);
 	return l < max_level - 1 ? l : max_level - 1;
 }
@@ -363,27 +362,34 @@ __device__ __forceinline__ int pair_levels(const uint64_t* __restrict__ keys, ui
 struct PairLevels {
 	int lv[CELL_TILE / TILE_THREADS + 1];  // lv[0]: the pair before this thread's first
 	uint32_t sum;
+	uint32_t same;  // bit k: slots i0 + k and i0 + k + 1 have one key
 	__device__ __forceinline__ PairLevels(const uint64_t* __restrict__ keys, uint32_t i0, uint32_t n_pairs, uint32_t L,
 	                                      int max_level, RunRec* rec)
 	{
-		lv[0] = i0 > 0 && i0 - 1 < n_pairs ? pair_levels(keys, i0 - 1, L, max_level, nullptr) : -1;
-		sum = 0;
+		lv[0] = i0 > 0 && i0 - 1 < n_pairs ? pair_levels(keys[i0 - 1], keys[i0 - 1 + L], max_level, nullptr) : -1;
+		sum = same = 0;
+		uint64_t next = i0 < n_pairs ? keys[i0] : 0;
 #pragma unroll
 		for (int k = 0; k < CELL_TILE / TILE_THREADS; k++) {
 			const uint32_t i = i0 + (uint32_t)k;
-			lv[k + 1] = i < n_pairs ? pair_levels(keys, i, L, max_level, rec) : -1;
+			const uint64_t key = next;
+			lv[k + 1] = -1;
+			if (i < n_pairs) {
+				next = keys[i + 1];
+				if (next == key) same |= 1u << k;
+				lv[k + 1] = pair_levels(key, L == 1 ? next : keys[i + L], max_level, rec);
+			}
 			if (lv[k + 1] > lv[k]) sum += (uint32_t)(lv[k + 1] - lv[k]);
 		}
 	}
 };
 
-// Two particles at one position: the reference's insertion would split
-// forever (pot.c:1466-1470) or fail at a reallocation (pot.c:1578-1586).
-__device__ __forceinline__ void check_coincident(uint32_t i, const uint64_t* __restrict__ keys,
-                                                 const uint32_t* __restrict__ perm, const double4* __restrict__ pos_in,
-                                                 RunRec* rec)
+// Two particles at one position, slots i and i + 1 with one key: the
+// reference's insertion would split forever (pot.c:1466-1470) or fail at a
+// reallocation (pot.c:1578-1586).
+__device__ __forceinline__ void check_coincident(uint32_t i, const uint32_t* __restrict__ perm,
+                                                 const double4* __restrict__ pos_in, RunRec* rec)
 {
-	if (keys[i] != keys[i + 1]) return;
 	const double4 p = pos_in[perm[i]], o = pos_in[perm[i + 1]];
 	if (p.x == o.x && p.y == o.y && p.z == o.z) set_status(rec, POT_E_COINCIDENT);
 }
@@ -398,11 +404,12 @@ __device__ __forceinline__ void cell_count_body(G grd, const uint64_t* __restric
 {
 	const uint32_t i0 = grd.id() * CELL_TILE + threadIdx.x * (CELL_TILE / TILE_THREADS);
 	const PairLevels p(keys, i0, n_pairs, L, max_level, rec);
-#pragma unroll
-	for (int k = 0; k < CELL_TILE / TILE_THREADS; k++)
-		if (i0 + (uint32_t)k < n_pairs) check_coincident(i0 + (uint32_t)k, keys, perm, pos_in, rec);
-	// the last L - 1 pairs of neighbours, beyond the pairs (i, i + L)
-	if (grd.id() == 0 && threadIdx.x + 1 < L) check_coincident(n_pairs + threadIdx.x, keys, perm, pos_in, rec);
+	for (uint32_t same = p.same; same; same &= same - 1u) check_coincident(i0 + (uint32_t)__ffs(same) - 1u, perm, pos_in, rec);
+	// the last L - 1 neighbours, beyond the pairs (i, i + L)
+	if (grd.id() == 0 && threadIdx.x + 1 < L) {
+		const uint32_t i = n_pairs + threadIdx.x;
+		if (keys[i] == keys[i + 1]) check_coincident(i, perm, pos_in, rec);
+	}
 	uint32_t total;
 	tile_scan(p.sum, &total);
 	if (threadIdx.x == 0) counts[grd.id()] = total;
