@@ -905,8 +905,8 @@ int pot_gpu_init_particles(pot_gpu_ctx* c)
 }
 
 // Keys, sort, reorder (+ due flags) and tree for the current state, on the
-// branches of S.  The target groups of a step (begin_step) go beside the
-// moments; the caller joins the two side branches.
+// branches of S.  The target groups and chi_b of a step (begin_step) go
+// beside the moments and the walk; the caller joins the two side branches.
 static void enqueue_tree(pot_gpu_ctx* c, int begin_step, const StepStreams& S)
 {
 	Params& P = c->P;
@@ -940,12 +940,9 @@ static void enqueue_step(pot_gpu_ctx* c, uint32_t flags, const StepStreams& S)
 	Params& P = c->P;
 	cudaStream_t s = S.main;
 	enqueue_tree(c, 1, S);
-	// the edge potential beside the groups' end, both ahead of the push: a
-	// potential that cannot be had (POT_E_WALK) leaves the particles as they are
 	S.order(4, s, S.tree());
 	launch_chi_b(c->T, c->src64, P, c->rec, 0, S.tree(), c->timer);
 	S.order(5, S.list(), s);
-	S.order(0, S.tree(), s);
 	if (P.integrator == POT_INT_BORIS) {
 		launch_push(c->pos[c->cur], c->vel[c->cur], c->T, c->src64, c->src32, c->due_list, c->groups, c->rein_list,
 		            P, c->rec, StageBufs { 0, nullptr, nullptr, nullptr }, s, c->timer);
@@ -969,8 +966,10 @@ static void enqueue_step(pot_gpu_ctx* c, uint32_t flags, const StepStreams& S)
 		launch_epe(c->pos[c->cur], c->T, two ? c->src64b : c->src64, two ? c->src32b : c->src32, c->groups_all,
 		           c->epe_partial, P, c->rec, s, c->timer);
 	}
-	launch_finish_step(c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->due_list, c->rein_list, c->src64, c->hist, P,
-	                   c->rec, epe, s, c->timer);
+	S.order(0, S.tree(), s);  // chi_b
+	const int from = c->cur ^ 1;
+	launch_finish_step(c->pos[c->cur], c->vel[c->cur], c->pid[c->cur], c->due_list, c->rein_list, c->src64, c->hist,
+	                   StepStart { c->vals[c->kb], c->pos[from], c->vel[from] }, P, c->rec, epe, s, c->timer);
 }
 
 // The context's streams for one enqueued step; forked when the step is being

@@ -351,8 +351,8 @@ static void enqueue_pack(const PackClass& pc, uint32_t spl)
 		S.order(4, s, S.tree());
 		pack_chi_b(B, S.tree());
 		S.order(5, S.list(), s);
-		S.order(0, S.tree(), s);
 		pack_push(B, (int)k, pc.group_max > 32 ? 2u : 1u, s);
+		S.order(0, S.tree(), s);  // chi_b
 		pack_finish_step(B, (int)k, s);
 	}
 }

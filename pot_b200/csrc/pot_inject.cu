@@ -626,6 +626,41 @@ __device__ __forceinline__ void grain_end_body(G grd, double4* __restrict__ pos,
 	hist[rec->t_steps % HIST] = h;
 }
 
+// A step whose edge potential could not be had ends with POT_E_WALK and its
+// particles, which are pushed while chi_b is measured, where they started.
+// Every block gives its share of the due particles back what they had ...
+__device__ __noinline__ void undo_push(GridSeg grd, double4* pos, double4* vel, const uint32_t* due_list, StepStart from,
+                                       RunRec* rec)
+{
+	if (threadIdx.x == 0) atomicExch(&rec->status, POT_E_WALK);
+	__syncthreads();
+	const uint32_t n_due = rec->n_due;
+	for (uint32_t i = grd.id() * blockDim.x + threadIdx.x; i < n_due; i += grd.n() * blockDim.x) {
+		const uint32_t s = due_list[i], j = from.perm[s];
+		pos[s] = from.pos[j];
+		vel[s] = from.vel[j];
+	}
+}
+
+// ... and the last one takes back what the push counted.
+__device__ __noinline__ void undo_counts(RunRec* rec, int epe)
+{
+	rec->n_rein = 0;
+	rec->stack_max = 0;
+	rec->dq = 0;
+	rec->de = 0;
+	rec->nabs_ion = 0;
+	rec->nabs_e = 0;
+	for (int k = 0; k < 3; k++) rec->sumv_ion[k] = rec->sumv_e[k] = 0;
+	rec->interactions = 0;
+	rec->n_pushed = 0;
+	rec->far_cells = 0;
+	rec->n_wall = 0;
+	rec->n_bounced = 0;
+	rec->warn = (rec->warn & ~WARN_WALL) | rec->wall_warn;
+	if (epe) rec->epe[SP_ION] = rec->epe[SP_E] = 0.0;
+}
+
 // The end of a step, one launch: the late absorption of a step on which the
 // grain moves, the reinjections, then -- by the block that finishes last --
 // the grain update and the step's statistics.  On a step on which the grain
@@ -636,12 +671,13 @@ template <class G>
 __device__ __forceinline__ void finish_step_body(G grd, double4* __restrict__ pos, double4* __restrict__ vel,
                                                  const uint32_t* __restrict__ pid,
                                                  const uint32_t* __restrict__ due_list, uint32_t* rein_list,
-                                                 const double4* __restrict__ src64, StepHist* hist, const Params& P,
-                                                 RunRec* rec, int epe)
+                                                 const double4* __restrict__ src64, StepHist* hist,
+                                                 const StepStart& from, const Params& P, RunRec* rec, int epe)
 {
 	__shared__ bool s_last;
-	const bool late = rec->grain_due != 0;
-	if (late) absorb_late_body(grd, pos, vel, src64, due_list, rein_list, P, rec);
+	const bool late = rec->grain_due != 0, undo = rec->chi_failed != 0;
+	if (undo) undo_push(GridSeg { grd.id(), grd.n() }, pos, vel, due_list, from, rec);
+	else if (late) absorb_late_body(grd, pos, vel, src64, due_list, rein_list, P, rec);
 	else reinject_body(grd, pos, vel, pid, rein_list, src64, P, rec);
 	__threadfence();
 	__syncthreads();
@@ -649,7 +685,9 @@ __device__ __forceinline__ void finish_step_body(G grd, double4* __restrict__ po
 	__syncthreads();
 	if (!s_last) return;
 	__threadfence();
-	if (late) {
+	if (undo) {
+		if (threadIdx.x == 0) undo_counts(rec, epe);
+	} else if (late) {
 		reinject_body(GridSeg { 0, 1 }, pos, vel, pid, rein_list, src64, P, rec);
 		__threadfence();
 		__syncthreads();
@@ -660,10 +698,10 @@ __device__ __forceinline__ void finish_step_body(G grd, double4* __restrict__ po
 __global__ void __launch_bounds__(128) k_finish_step(double4* __restrict__ pos, double4* __restrict__ vel,
                                                      const uint32_t* __restrict__ pid,
                                                      const uint32_t* __restrict__ due_list, uint32_t* rein_list,
-                                                     const double4* __restrict__ src64, StepHist* hist, Params P,
-                                                     RunRec* rec, int epe)
+                                                     const double4* __restrict__ src64, StepHist* hist,
+                                                     StepStart from, Params P, RunRec* rec, int epe)
 {
-	finish_step_body(GridSelf {}, pos, vel, pid, due_list, rein_list, src64, hist, P, rec, epe);
+	finish_step_body(GridSelf {}, pos, vel, pid, due_list, rein_list, src64, hist, from, P, rec, epe);
 }
 
 // init_particles for one rank (pot.c:887-935), reference order: slot i holds
@@ -694,11 +732,11 @@ __global__ void k_init(double4* __restrict__ pos, double4* __restrict__ vel, uin
 }
 
 void launch_finish_step(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* due_list, uint32_t* rein_list,
-                        const double4* src64, StepHist* hist, const Params& P, RunRec* rec, int epe, cudaStream_t s,
-                        Timer& tm)
+                        const double4* src64, StepHist* hist, const StepStart& from, const Params& P, RunRec* rec,
+                        int epe, cudaStream_t s, Timer& tm)
 {
 	ScopedKernel k(tm, "finish_step");
-	k_finish_step<<<148, 128, 0, s>>>(pos, vel, pid, due_list, rein_list, src64, hist, P, rec, epe);
+	k_finish_step<<<148, 128, 0, s>>>(pos, vel, pid, due_list, rein_list, src64, hist, from, P, rec, epe);
 }
 
 void launch_init(double4* pos, double4* vel, uint32_t* pid, const Params& P, RunRec* rec, cudaStream_t s,
@@ -719,9 +757,9 @@ __global__ void __launch_bounds__(128) kp_finish_step(PackDev B, int k)
 {
 	const SegBlock sb = seg_block(B.pre[PS_SMALL], B.M);
 	const MemberView& v = B.mv[sb.m];
-	const uint32_t b = pack_out(v, k);
+	const uint32_t a = pack_in(v, k), b = pack_out(v, k);
 	finish_step_body(GridSeg { sb.id, sb.n }, v.pos[b], v.vel[b], v.pid[b], v.due_list, v.rein_list, v.src64, v.hist,
-	                 v.P, v.rec, 0);
+	                 StepStart { v.vals[v.kb], v.pos[a], v.vel[a] }, v.P, v.rec, 0);
 }
 
 void pack_finish_step(const PackDev& B, int k, cudaStream_t s)

@@ -89,6 +89,7 @@ struct RunRec {
 	unsigned int n_overflow; // deepest-level buckets of a leaf-size-1 tree this build
 	unsigned int n_groups[2];      // fast form: target groups this step, large and small (see group_at)
 	unsigned int n_groups_all[2];  // the same over every particle (potential energies)
+	unsigned int wall_warn;  // warn's WARN_WALL at the step's start
 	long long dq;
 	unsigned long long de;
 	unsigned long long nabs_ion;
@@ -101,7 +102,7 @@ struct RunRec {
 	double epe[3];           // potential energies of the last step that computed them (J)
 	double phi_grain;        // potential at the grain from every other particle (V)
 	unsigned int epe_step;   // 1 when this step computes them
-	unsigned int epe_pad;
+	unsigned int chi_failed; // the step's edge potential could not be had (see finish_step_body)
 	long long q_sum;         // sum over completed steps of the grain charge after each step (moving means)
 	unsigned int n_collected;  // Poisson ion collection: charges added this step
 	unsigned int n_wall;       // OUT_BOUNCE: particles outside moving inwards this step

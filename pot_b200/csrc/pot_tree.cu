@@ -99,6 +99,8 @@ __device__ __forceinline__ void keys_body(G grd, const double4* __restrict__ pos
 		rec->work_ctr2 = 0;
 		rec->stack_max = 0;
 		rec->grain_due = (t % P.tss[SP_DUST]) == 0 ? 1u : 0u;
+		rec->chi_failed = 0;
+		rec->wall_warn = rec->warn & WARN_WALL;
 		rec->dq = 0;
 		rec->de = 0;
 		rec->nabs_ion = 0;

@@ -149,8 +149,8 @@ void launch_moments(TreeDev& T, const double4* src64, const Params& P, RunRec* r
 // ---- branches of a step --------------------------------------------------
 // A captured step runs on three streams: while the main one reorders the
 // state and sums its moments, the second builds the tree's topology from the
-// sorted keys (and later measures chi_b) and the third lists the due particles
-// and makes the target groups; all three meet ahead of the push.  Without side streams the
+// sorted keys (and later measures chi_b beside the walk) and the third lists
+// the due particles and makes the target groups.  Without side streams the
 // same launches follow each other on the main one.
 struct StepStreams {
 	cudaStream_t main = nullptr, side[2] = { nullptr, nullptr };
@@ -219,9 +219,15 @@ void launch_phi_query(const TreeDev& T, const double4* src64, const double* xyz,
                       const Params& P, RunRec* rec, cudaStream_t s, Timer& tm);
 
 // inject.cu
+// The state a step started from: slot s of its order was perm[s] of pos and vel.
+struct StepStart {
+	const uint32_t* perm;
+	const double4* pos;
+	const double4* vel;
+};
 void launch_finish_step(double4* pos, double4* vel, const uint32_t* pid, const uint32_t* due_list, uint32_t* rein_list,
-                        const double4* src64, StepHist* hist, const Params& P, RunRec* rec, int epe, cudaStream_t s,
-                        Timer& tm);
+                        const double4* src64, StepHist* hist, const StepStart& from, const Params& P, RunRec* rec,
+                        int epe, cudaStream_t s, Timer& tm);
 void launch_init(double4* pos, double4* vel, uint32_t* pid, const Params& P, RunRec* rec, cudaStream_t s,
                  Timer& tm);
 

@@ -634,7 +634,7 @@ __device__ __forceinline__ void chi_b_body(G grd, const TreeDev& T, const double
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		if (bad) {
-			set_status(rec, POT_E_WALK);
+			rec->chi_failed = 1;  // the step ends with POT_E_WALK (finish_step_body)
 		} else {
 			double sum = 0.0;
 			for (uint32_t k = 0; k < P.chi_ranks; k++) sum += sample[k];
