@@ -799,13 +799,14 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	}
 	AL(T.ovf, OVF_CAP);
 	if (fast) {
-		AL(T.nrec, 8ull * cap + 1);
+		T.spare = 1 + cap + n;
+		AL(T.nrec, (size_t)T.spare + 1);
 		AL(T.mom_pre, 5 * mom_prefix_entries(n));
 		AL(T.mom_blk, 5 * mom_block_entries(n));
 		if (cfg->flags & POT_CFG_DIPOLES) {
 			AL(T.mom_pre_d, 5 * mom_prefix_entries(n));
 			AL(T.mom_blk_d, 5 * mom_block_entries(n));
-			AL(T.drec, 8ull * cap + 1);
+			AL(T.drec, (size_t)T.spare + 1);
 		}
 		if (L > 1) AL(T.lrange, 8ull * cap);
 	}

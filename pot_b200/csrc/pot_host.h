@@ -69,7 +69,8 @@ constexpr int DUE_TILE = 4096;    // slots per tile of the due list (whole block
 constexpr int REORDER_THREADS = 256;
 
 // Words of a step that start at zero: the radix sort's digit counts, the keys
-// kernel's block counter, a tile ticket counter per radix pass, the due
+// kernel's block counter, the count of node records given out, a tile ticket
+// counter per radix pass, the due
 // slots of each DUE_TILE and the passes' look-back status words, 256 a tile.
 // The words of the passes in use come last, so that one memset clears a
 // step's.  The cell counts of each CELL_TILE need no clearing.
@@ -77,6 +78,7 @@ struct StepWords {
 	uint32_t* hist;      // [OS_MAX_PASSES * 256]
 	unsigned int* pass_ctr;  // [OS_MAX_PASSES]
 	unsigned int* keys_ctr;
+	unsigned int* rec_ctr;
 	uint32_t* cell;      // [cell_tiles(n)]
 	uint32_t* due;       // [due_tiles(n)]
 	uint32_t* status;    // [passes * radix_rows(n) * 256]
@@ -98,6 +100,7 @@ struct StepWords {
 		hist = w;
 		pass_ctr = w + OS_MAX_PASSES * RS_BINS;
 		keys_ctr = pass_ctr + OS_MAX_PASSES;
+		rec_ctr = keys_ctr + 1;
 		cell = w + OS_MAX_PASSES * RS_BINS + 16;
 		due = cell + cell_tiles(n);
 		status = w + head(n);

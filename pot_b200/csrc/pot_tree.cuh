@@ -8,9 +8,9 @@ namespace pot {
 // A tree node as the FP32 walk reads it, in units of the domain radius from
 // the domain centre.  A cell: centre of charge and charge, critical radius
 // squared (accepted when d^2 > r2), the index of its first child's record and
-// the mask of its children by octal digit.  A leaf: the same moments, its
-// first slot and, with NR_LEAF, its particle count; a leaf of a leaf-size-1
-// tree has no moments (NR_UNTESTED: always opened).
+// how many children it has.  A leaf: the same moments, its first slot and, with
+// NR_LEAF, its particle count; a leaf of a leaf-size-1 tree has no moments
+// (NR_UNTESTED: always opened).
 constexpr uint32_t NR_LEAF = 1u << 31, NR_UNTESTED = 1u << 30, NR_COUNT = NR_UNTESTED - 1u;
 struct __align__(32) NodeRec {
 	float x, y, z, q;
@@ -30,18 +30,20 @@ struct TreeDev {
 	uint32_t* last;    // last particle
 	uint8_t* level;    // depth (root 0)
 	int32_t* child;    // [8 * cap] child codes by octal digit
-	int32_t* parent;   // 8 parent + octal digit, -1 for the root
+	int32_t* parent;   // the parent cell, -1 for the root; fast form: the cell's own record
 	uint8_t* nint;     // internal children
-	uint32_t* ctr;     // arrivals in the upward pass
+	uint32_t* ctr;     // arrivals in the upward pass; fast form: the first child's record
 	int32_t* q;        // net charge (Tree.q)
 	uint32_t* aq;      // absolute charge (Tree.aq)
 	double4* cq;       // centre of |q| and q
 	double* w2;        // (x2 - x1)^2
 	double4* dip;      // DIPOLES: dipole moment about cq (FP64, both forms); null otherwise
-	// FP32 walk (fast form only; null otherwise): one 32-byte record per child,
-	// record 8 k + d for child d of cell k (the root's is record 8 cap), so that
-	// a walk reads everything it needs of a node with one load
-	NodeRec* nrec;     // [8 * cap + 1]
+	// FP32 walk (fast form only; null otherwise): one 32-byte record per node, so
+	// that a walk reads everything it needs of a node with one load.  The root's
+	// is record 0; a cell's children have consecutive records in digit order
+	// (k_finish_nodes gives them out), at most `cap` of cells and n of leaves.
+	NodeRec* nrec;     // [spare + 1]
+	uint32_t spare;    // a record no node has
 	uint2* lrange;     // [8 * cap] bucket-leaf (first slot, count)
 	uint2* ovf;        // [OVF_CAP] leaf-size-1 overflow buckets (first slot, count)
 	// fast form: exclusive prefix sums of (q, |q|, |q| x, |q| y, |q| z), 5 doubles each
@@ -51,7 +53,7 @@ struct TreeDev {
 	// and the nodes' dipoles in FP32 units of q R
 	double* mom_pre_d;
 	double* mom_blk_d;
-	float4* drec;      // [8 * cap + 1], indexed as nrec
+	float4* drec;      // [spare + 1], indexed as nrec
 };
 
 // One member run of a packed batch as the batched kernels see it: the

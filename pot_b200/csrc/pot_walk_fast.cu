@@ -544,7 +544,7 @@ struct Traversal {
 		n_far = 0;
 		len = maxlen = 1;
 		ncell = nleaf = 0;
-		if (lane_f() == 0) stack[0] = 8u * T.cap;  // the root's record
+		if (lane_f() == 0) stack[0] = 0u;  // the root's record
 		__syncwarp();
 	}
 
@@ -565,7 +565,7 @@ struct Traversal {
 		float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
 		float4 dipole = make_float4(0.f, 0.f, 0.f, 0.f);
 		uint2 range = make_uint2(0u, 0u);
-		uint32_t kids = 0u, base = 0u;  // an opened cell's children: mask, first record
+		uint32_t kids = 0u, base = 0u;  // an opened cell's children: how many, first record
 		if (node != NONE) {
 			uint32_t info;
 			float r2;
@@ -589,7 +589,7 @@ struct Traversal {
 				kids = info;
 			}
 		}
-		const int nch = __popc(kids);
+		const int nch = (int)kids;
 		leafr = leafr && range.y > 0u;  // the leaf flush relies on no staged leaf being empty
 		// one warp scan for the three appends: accepted cells in bits 0-9,
 		// leaf ranges in bits 10-19, children in bits 20-31 (totals <= 32,
@@ -615,10 +615,10 @@ struct Traversal {
 			for (int k = 0; k < TPL; k++) seen[k] = seen[k] || (tg.self[k] - rx < ry);
 		}
 		if (len + tch > FW_STACK) return false;
-		int w = len + po;
+		const int w = len + po;
 #pragma unroll
 		for (uint32_t d = 0; d < 8; d++)
-			if (kids & (1u << d)) stack[w++] = base + d;
+			if (d < kids) stack[w + (int)d] = base + d;
 		len += tch;
 		maxlen = max(maxlen, len);
 		__syncwarp();

@@ -15,7 +15,8 @@ SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), 
 
 
 def parents(keys, garbage, L=1):
-    """T.parent after the topology kernels: 8 k + digit, garbage where nobody wrote."""
+    """T.parent after the topology kernels (plain form: the parent cell; fast
+    form: the cell's record, as many in number), garbage where nobody wrote."""
     n = len(keys)
     lvl = np.minimum(tm.lcp_levels(keys[:n - L], keys[L:]), tm.MAX_LEVELS - 1)
     prev = np.concatenate([[-1], lvl[:-1]])
@@ -42,7 +43,7 @@ def parents(keys, garbage, L=1):
             kc = int(base[sc]) + l + 1 - lo
             if kc < 0 or kc >= M or kc <= k:
                 continue
-            out[kc] = 8 * k + d
+            out[kc] = k
             claimed.add(kc)
     out[0] = -1
     return out, len(claimed), M
@@ -62,22 +63,23 @@ def test_unclaimed_cells_are_not_followed():
         cap = 4 * len(keys) + 4096
         assert M <= cap
         orphans += M - 1 - claimed
+        spare = 1 + cap + len(keys)
         for k in range(1, M):
             # k_moments: nint[p], cells p < k only
-            p = int(par[k]) >> 3
+            p = int(par[k])
             orphan = p < 0 or p >= k
             assert orphan or p < M
-            # moments_prefix_body: nrec[o], o < 8 k only
-            o = int(par[k]) & 0xFFFFFFFF
-            assert o >= 8 * k or o < 8 * cap
-            wild += o > 8 * cap
+            # moments_prefix_body: nrec[o], records up to the spare one
+            o = min(int(par[k]) & 0xFFFFFFFF, spare)
+            assert 0 <= o <= spare
+            wild += int(par[k]) & 0xFFFFFFFF > spare
     assert orphans > 0 and wild > 0  # without the checks these were followed
 
 
-@pytest.mark.parametrize("use,check", [(r"T\.nint\[p\]", r"\(uint32_t\)p >= k"), (r"T\.nrec\[o\]", r"o >= 8u \* k")])
+@pytest.mark.parametrize("use,check", [(r"T\.nint\[p\]", r"\(uint32_t\)p >= k"), (r"T\.nrec\[o\]", r"o = [^;]*min\([^;]*, spare\);")])
 def test_checks_stand_ahead_of_the_uses(use, check):
     text = re.sub(r"//[^\n]*", "", open(SRC).read())
     uses = [m.start() for m in re.finditer(use, text)]
     assert uses
     for u in uses:
-        assert re.search(check, text[max(0, u - 500):u]), use
+        assert re.search(check, text[max(0, u - 1500):u]), use
