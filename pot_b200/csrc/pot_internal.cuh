@@ -284,19 +284,19 @@ __device__ __forceinline__ void set_status(RunRec* rec, int code)
 }
 
 // The run's status as the whole block, or the calling warp, sees it: one
-// reading, from L2.  A kernel beside this one may set the status at any time, so
-// threads that meet at a barrier or a shuffle must not each read it.
+// reading.  A kernel beside this one may set the status at any time, so threads
+// that meet at a barrier or a shuffle must not each read it.
 __device__ __forceinline__ int block_status(const RunRec* rec)
 {
 	__shared__ int status;
-	if (threadIdx.x == 0) status = __ldcg(&rec->status);
+	if (threadIdx.x == 0) status = rec->status;
 	__syncthreads();
 	return status;
 }
 __device__ __forceinline__ int warp_status(const RunRec* rec)
 {
 	int status = POT_OK;
-	if ((threadIdx.x & 31u) == 0) status = __ldcg(&rec->status);
+	if ((threadIdx.x & 31u) == 0) status = rec->status;
 	return __shfl_sync(0xffffffffu, status, 0);
 }
 

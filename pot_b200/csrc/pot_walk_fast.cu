@@ -1573,7 +1573,7 @@ k_push_pair(double4* __restrict__ pos, double4* __restrict__ vel, TreeDev T, con
 	const int w = (int)(threadIdx.x >> 5), pair = w >> 1;
 	PairSmem<TPL, DIP>& sm = smem[pair];
 	const uint32_t n_large = rec->n_groups[0], n_groups = n_large + rec->n_groups[1];
-	if (((w ^ (w >> 1) ^ (int)(blockIdx.x / 148u)) & 1) == 0) {
+	if (((w ^ (w >> 1) ^ (int)(blockIdx.x / (gridDim.x / PAIR_BLOCKS))) & 1) == 0) {  // a grid is PAIR_BLOCKS an SM
 		int k = 0, cb = 0, lb = 0, par = 0;
 		for (;;) {
 			uint32_t g = 0;
