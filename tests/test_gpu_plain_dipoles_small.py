@@ -46,3 +46,29 @@ def test_opened_tree(N):
         assert np.isfinite(F).all()
         # each of fewer than 70 terms within a few roundings, and as many in the sum
         assert (np.sqrt(((F - E[idx]) ** 2).sum(1)) <= 100 * 2.0 ** -53 * mag[idx]).all()
+
+
+@pytest.mark.parametrize("N", [500, 8193, 30001])
+def test_runs_from_their_start(N):
+    """Ordinary runs of the plain form with dipoles: every particle stays a
+    number, and the fields are the oracle's."""
+    d = dict(SMALL, N=N)
+    o = oracle_snapshot(d, seed=N, dipoles=True)
+    o.set_grain(q=-90)
+    p = o.particles()
+    with Run(run_config(d, dipoles=True), form="plain", seed=2, chi_cap=True) as r:
+        r.upload(p, dict(q=-90, pos=(p["x"][0], p["y"][0], p["z"][0])))
+        r.build_tree()
+        idx = np.arange(N, dtype=np.uint32)
+        xyz = np.stack([p[a] for a in "xyz"], 1)
+        F = r.field_at(idx, xyz)
+        assert r.step(6)["status"] == 0
+        q, _ = r.download()
+    assert np.isfinite(F).all()
+    assert all(np.isfinite(q[k]).all() for k in ("x", "y", "z", "vx", "vy", "vz"))
+    o.build_tree()
+    hi, lo = o.field_many(idx, xyz)
+    ref = (np.asarray(hi, np.longdouble) + lo).astype(np.float64)
+    # hundreds of terms of FP64 rounding each against sums whose parts cancel
+    err = np.abs(F - ref).max(1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < 1e-11, err.max()

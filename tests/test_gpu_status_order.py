@@ -5,7 +5,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from pot_b200.gpu import PARTICLE_DTYPE, PotError, Run
+from pot_b200.gpu import PARTICLE_DTYPE, Batch, PotError, Run
 from tests.common import SMALL, run_config
 
 pytestmark = pytest.mark.gpu
@@ -69,11 +69,12 @@ def test_coincident_neighbours_at_the_ends(leaf, where):
         assert e.value.status == E_COINCIDENT
 
 
-@pytest.mark.parametrize("form,N", [("plain", 20001), ("fast", 20001), ("fast", 2000001)])
-def test_a_failed_edge_potential_stops_the_push(form, N):
+@pytest.mark.parametrize("form,N,integrator", [("plain", 20001, 0), ("fast", 20001, 0), ("fast", 2000001, 0),
+                                               ("plain", 5001, 1), ("fast", 5001, 2)])
+def test_a_failed_edge_potential_stops_the_push(form, N, integrator):
     """An edge potential that is no number (the grain's position given as NaN) on
     the 20th step: the step ends with the walk's status and no particle moves."""
-    d = dict(SMALL, N=N)
+    d = dict(SMALL, N=N, integrator=integrator)
     p = _state(N, d["r"] * d["mpp"], 4)
     c = (p["x"][0], p["y"][0], p["z"][0])
     rng = np.random.default_rng(5)
@@ -90,4 +91,40 @@ def test_a_failed_edge_potential_stops_the_push(form, N):
             with pytest.raises(PotError) as e:
                 r.step(1)
             assert e.value.status == E_WALK
-            assert e.value.stats["n_pushed"] == 0
+            st = e.value.stats
+            assert st["n_pushed"] == 0 and st["n_reinjected"] == 0 and st["n_absorbed"] == 0 and st["dq"] == 0
+            assert st["interactions"] == 0 and st["grain_q"] == -7
+        # the drop-in call gives back the records as the step found them
+        r.upload(p, dict(q=-7, pos=c, t_steps=18))
+        r.step(1)
+        out, _ = r.download()
+        kept = out.copy()
+        with pytest.raises(PotError) as e:
+            r.move_particles(out, dict(q=-7, pos=(np.nan, c[1], c[2]), t_steps=19))
+        assert e.value.status == E_WALK
+        for a in ("x", "y", "z", "vx", "vy", "vz", "species"):
+            assert np.array_equal(out[a][1:], kept[a][1:]), a
+
+
+def test_a_failed_edge_potential_in_a_packed_batch():
+    """It undoes the step of its own run only."""
+    N = 6001
+    d = dict(SMALL, N=N)
+    p = _state(N, d["r"] * d["mpp"], 6)
+    c = (p["x"][0], p["y"][0], p["z"][0])
+    cfg = run_config(d)
+    o = dict(leaf_size=8, seed=9, chi_cap=True)
+    with Run(cfg, form="fast", **o) as r, Batch() as b:
+        r.upload(p, dict(q=-7, pos=c, t_steps=18))
+        r.step(2)
+        good = b.admit(cfg, parts=p, grain=dict(q=-7, pos=c, t_steps=18), **o)
+        bad = b.admit(cfg, parts=p, grain=dict(q=-7, pos=(np.nan, c[1], c[2]), t_steps=18), **o)
+        b.step(2)
+        rows = {int(w["slot"]): w for w in b.summary()}
+        want, g = r.download()
+        got, h = b.download(good)
+    assert rows[good]["status"] == 0 and rows[bad]["status"] == E_WALK
+    assert rows[bad]["t_steps"] == rows[good]["t_steps"] == 20
+    for a in ("x", "y", "z", "vx", "vy", "vz", "species"):
+        assert np.array_equal(want[a], got[a]), a
+    assert g["q"] == h["q"] and g["chi_b"] == h["chi_b"]
