@@ -50,7 +50,6 @@ __host__ __device__ inline int slot_digit(int s)
 }
 
 constexpr int MAX_LEVELS = 21;     // 63-bit keys, 3 bits per level
-constexpr int WALK_STACK = 400;    // MAX_PATH_LEN, pot.c:196
 // Leaf size 1 cannot hold two particles that share all 21 key levels (closer
 // than 2R / 2^21 in every axis); such a level-21 cell becomes a bucket in a
 // small overflow table, leaf payload n + j, and sets warn bit 0.

@@ -23,7 +23,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 	return v;
 }
 
-// Exclusive block scan of one value per thread (blockDim.x = SCAN_THREADS);
+// Exclusive block scan of one value per thread (whole warps, at most 32);
 // returns the exclusive prefix, writes the block total to *total.
 __device__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
 {

@@ -1,5 +1,5 @@
 // Barnes-Hut walks fused with the Boris push, grain absorption and the
-// boundary test; edge potential (chi_b); grain update.
+// boundary test; potential energies, point queries, edge potential (chi_b).
 //
 // Plain form (POT_FORM_PLAIN): FP64, leaf size 1.  Every target makes its own
 // accept/open decisions with the reference's unfused opening test
@@ -97,9 +97,13 @@ __device__ __forceinline__ void plain_term(PlainAcc& E, bool on, bool dip, const
 // set in.  So every target's terms are the reference's; only the order of
 // its FP64 sum differs.
 //
-// What bounds it: instruction issue (a walk of one thread per target, the
-// form before, ran 17 of 32 lanes on average through three divergent paths
-// and waited on its stack in local memory).  Sharing a node's load, stack
+// What bounds it: with many targets instruction issue and the FP64 pipe (at
+// 1,000,001 particles 68 % of issue slots, 50 % of the FP64 pipe, 73 % of the
+// shared-memory wavefronts, 26 of 32 lanes active); with few, the latency of
+// each warp's chain of rounds (8,193 particles: 12 warps an SM, 23 % of issue
+// slots over the launch).  A walk of one thread per target, the form before, ran
+// 17 of 32 lanes on average through three divergent paths and waited on its
+// stack in local memory.  Sharing a node's load, stack
 // entry and list entry between G neighbours, and evaluating branch-free
 // lists, took a step's walk from 958 to 54 us on the 8,193-particle plasma,
 // from 2,570 to 291 us at 60,001 particles (theta 0.4) and from 9.18 to
@@ -725,7 +729,11 @@ static int sm_count()
 // node's load, test round and stack entry, fewer make more warps: with 4,096
 // targets (8,193 particles) the walk takes 55, 63, 88 and 138 us with 2, 4, 8
 // and 16 targets a warp, with 15,000 132, 115, 129 and 209, with 30,000 399,
-// 294, 288 and 380, with 500,000 4,990, 3,248, 2,647 and 2,570.
+// 294, 288 and 380, with 500,000 4,990, 3,248, 2,647 and 2,570.  With dipoles
+// (the reference's off-by-default variant) one size is compiled, the one for
+// many targets: 2, 4 and 8 targets take 71, 88 and 126 us with 4,096, 203, 171
+// and 180 with 15,000, 401, 303 and 296 with 30,000, 8,320, 5,450 and 4,363 with
+// 500,000.
 static int plain_group(uint32_t n) { return n < 8192u ? 2 : (n < 32768u ? 4 : 8); }
 
 template <int STG, int G, bool DIP>

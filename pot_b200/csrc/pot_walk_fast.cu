@@ -50,7 +50,11 @@ constexpr int fw_push_blocks(int tpl) { return tpl == 2 ? 4 : 5; }
 // leaves schedulers idle and the step waits for the slowest group; with more
 // groups than warps a pair's barriers only cost.  Walk per step, one warp and
 // a pair: 8,193 particles 104 and 59 us, 16,001 95 and 60, 64,001 149 and 96,
-// 150,001 157 and 166, 1,000,001 712 and 926.  Four blocks per SM: at five
+// 150,001 157 and 166, 1,000,001 712 and 926.  The line's two sides for each
+// group size, one warp and a pair: groups of 8 at 25,601 particles 61 and 58,
+// at 38,401 69 and 80; of 16 at 51,201 97 and 85, at 76,801 95 and 107; of 32 at
+// 102,401 144 and 124, at 128,001 130 and 132; of 64 at 204,801 283 and 270, at
+// 307,201 361 and 381.  Four blocks per SM: at five
 // (96 registers, 112 bytes of spills) 65, 63, 102 and 171 us.
 constexpr uint32_t PAIR_MAX_N_PER_TARGET = 3200;
 constexpr int PAIR_BLOCKS = 4;
