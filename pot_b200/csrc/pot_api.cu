@@ -827,7 +827,11 @@ static int create_impl(const pot_run_cfg* cfg, const pot_gpu_opts* opts, pot_gpu
 	r0.grain_m = MASS_DUST;
 	r0.grain_slot = 0xFFFFFFFFu;
 	r0.ion_temp = cfg->Ti;  // Proc.Ti starts at the injection temperature, pot.c:4252
-	if (cudaMemcpy(c->rec, &r0, sizeof(r0), cudaMemcpyHostToDevice) != cudaSuccess) {
+	// the sort's second order starts as indices too (the keys kernel writes the
+	// first): a sort that gives up leaves slots as they were, and the reorder reads
+	// the state at whatever they hold
+	if (cudaMemcpy(c->rec, &r0, sizeof(r0), cudaMemcpyHostToDevice) != cudaSuccess ||
+	    cudaMemsetAsync(c->vals[1], 0, sizeof(uint32_t) * n, c->stream) != cudaSuccess) {
 		pot_gpu_destroy(c);
 		return POT_E_CUDA;
 	}

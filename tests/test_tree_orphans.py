@@ -76,6 +76,39 @@ def test_unclaimed_cells_are_not_followed():
     assert orphans > 0 and wild > 0  # without the checks these were followed
 
 
+def test_a_sort_that_gave_up_leaves_indices_of_particles():
+    """A tile whose look-back stops early counts too few of the earlier tiles'
+    keys: it writes over theirs, never past its digit, and leaves other slots
+    with what they held.  That is an index too: the keys kernel writes one order
+    every step and a context starts with the other cleared."""
+    rng = np.random.default_rng(2)
+    n, tile = 20000, 2048
+    vals = [np.arange(n), np.zeros(n, np.int64)]
+    unwritten = 0
+    for step in range(3):
+        vals[0] = np.arange(n)
+        for p in range(4):
+            src, dst = vals[p & 1], vals[(p + 1) & 1]
+            digit = rng.integers(0, 256, n)
+            start = np.concatenate([[0], np.cumsum(np.bincount(digit, minlength=256))])
+            written = np.zeros(n, bool)
+            for t0 in range(0, n, tile):
+                seen = int(rng.integers(0, t0 // tile + 1)) * tile  # the tiles the look-back reached
+                before = np.bincount(digit[t0 - seen:t0], minlength=256)
+                count = np.zeros(256, int)
+                for i, d in enumerate(digit[t0:t0 + tile]):
+                    o = start[d] + before[d] + count[d]
+                    assert o < start[d + 1]
+                    dst[o] = src[t0 + i]
+                    written[o] = True
+                    count[d] += 1
+            unwritten += int((~written).sum())
+            assert dst.min() >= 0 and dst.max() < n
+    assert unwritten > 0  # the premise
+    api = open(os.path.join(os.path.dirname(SRC), "pot_api.cu")).read()
+    assert "cudaMemsetAsync(c->vals[1], 0, sizeof(uint32_t) * n, c->stream)" in api
+
+
 @pytest.mark.parametrize("use,check", [(r"T\.nint\[p\]", r"\(uint32_t\)p >= k"), (r"T\.nrec\[o\]", r"o = [^;]*min\([^;]*, spare\);")])
 def test_checks_stand_ahead_of_the_uses(use, check):
     text = re.sub(r"//[^\n]*", "", open(SRC).read())
